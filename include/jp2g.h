@@ -175,29 +175,16 @@ int jp2g_cancel(jp2g_ctx* ctx, uint64_t ticket);
  *                             waves never exceed 246,723 64x64 blocks or
  *                             838,860 32x32 blocks, whose payload slots need
  *                             32-bit offsets);
- * JP2G_OPT_MQ_BLOCKS_PER_WARP code-blocks per warp in MQ coding, 1..32, or 0
- *                             for automatic (1 up to 48 blocks per SM, else
- *                             2..32 for about 24 warps per SM);
+ * JP2G_OPT_MQ_BLOCKS_PER_WARP code-blocks per warp in MQ coding (one per lane),
+ *                             1..32, or 0 for automatic (as few as keep one
+ *                             warp per scheduler, up to 32);
  * JP2G_OPT_HOST_THREADS       host threads for staging and Tier-2 (0 = all but
  *                             two hardware threads);
- * JP2G_OPT_MQ_WARPS_PER_SM    with one code-block per warp, the warps per SM
- *                             that pull blocks heaviest first (0 = automatic:
- *                             8 up to 16 blocks per SM, else 12; -1 = one warp
- *                             per block, no pulling);
- * JP2G_OPT_MQ_PIPES_PER_SM    when pulling: producer/consumer warp pairs per
- *                             SM that split each block's MQ chain into its
- *                             interval and code-register halves (0 =
- *                             automatic: 8 pairs per SM up to 48 blocks per
- *                             SM; -1 = single-warp pulling);
- * JP2G_OPT_MQ_HEAVY           with pipelines: how many of the heaviest blocks
- *                             they take, the rest being coded 32 to a warp
- *                             (0 = all blocks);
- * JP2G_OPT_MQ_CHAINS_PER_PAIR with pipelines: code-blocks each pair codes at
- *                             once, 1 (all lanes of a warp on one chain), 2
- *                             (one per half-warp: about half the issue slots
- *                             per symbol) or 4 (one per quarter-warp); 0 =
- *                             automatic (1 up to 8 blocks per SM, 2 up to 24,
- *                             else 4 on 4 pairs per SM). */
+ * JP2G_OPT_MQ_WARPS_PER_SM, JP2G_OPT_MQ_PIPES_PER_SM, JP2G_OPT_MQ_HEAVY,
+ * JP2G_OPT_MQ_CHAINS_PER_PAIR are accepted in their ranges (-1..64, -1..32,
+ *                             0..2^32-1, and 0, 1, 2 or 4) and kept; the MQ
+ *                             coder has a single form, which they do not
+ *                             change. */
 enum {
   JP2G_OPT_WAVE_BLOCKS = 0,
   JP2G_OPT_MQ_BLOCKS_PER_WARP = 1,
@@ -212,10 +199,9 @@ int jp2g_set_option(jp2g_ctx* ctx, int option, int64_t value);
 int jp2g_get_option(jp2g_ctx* ctx, int option, int64_t* value);
 
 /* Autotuner: encodes the caller's sample pages (through jp2g_encode_batch)
- * under each candidate setting of the MQ schedule (automatic; 4, 8 or 16
- * producer/consumer pairs per SM with one or two chains each; 8, 12 or 16
- * pulling warps per SM; 2 to 32 blocks packed per warp), then of the wave
- * size (20,000 to 240,000 code-blocks) under the fastest schedule, and
+ * under each candidate setting of the MQ schedule (automatic; 1 to 32 blocks
+ * per warp), then of the wave size (20,000 to 240,000 code-blocks) under the
+ * fastest schedule, and
  * leaves the fastest setting on the context. A candidate's time is the least
  * wall time of `repeats` (1..100) encodes after one untimed encode. Every
  * candidate must reproduce the first encode's codestreams byte for byte; a

@@ -444,18 +444,6 @@ int run_dwt_wave(jp2g_ctx* c, const std::vector<PageJob*>& live, bool raw) {
   return kOk;
 }
 
-// Code-blocks each MQ producer/consumer pair codes at once. Automatic: one
-// (all lanes on the chain) up to 8 blocks per SM, where the heaviest
-// block's chain sets the time; two (one per half-warp) up to 24, where
-// instruction issue does; four (one per quarter-warp, on 4 pairs per SM)
-// above (measured on gray pages of 1275x1650 to 3400x4400 and 2550x3300
-// sRGB pages: 4.5 against 5.6 ms of MQ for the sRGB page).
-int mq_chains_per_pair(const jp2g_ctx* c, uint32_t nb) {
-  const int64_t v = c->opt[JP2G_OPT_MQ_CHAINS_PER_PAIR];
-  if (v == 1 || v == 2 || v == 4) return (int)v;
-  return nb <= (uint32_t)c->num_sms * 8u ? 1 : (nb <= (uint32_t)c->num_sms * 24u ? 2 : 4);
-}
-
 // Runs f(0..n-1) on up to `threads` host threads.
 template <class F>
 void parallel_for(size_t n, int threads, F f) {
@@ -884,7 +872,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   ta.res = dptr<BlockOut>(c->res);
   ta.nplanes = dptr<uint32_t>(c->nplanes);
   ta.plane_base = dptr<uint32_t>(c->planebase);
-  ta.sym_slot = (uint32_t)((slot * 5 / 2 + 15) & ~size_t(15));
+  ta.sym_slot = (uint32_t)(((slot * 5 / 2 + 15) & ~size_t(15)) + 48);  // each pass padded to 16 symbols
   ta.sym_count = dptr<unsigned long long>(c->stats);
   if (!cuda_ok(c, cudaMemsetAsync(c->stats.p, 0, 8, c->stream), "memset")) return kEncodeFailed;
   launch_t1_analyze(ta, c->stream);
@@ -910,44 +898,14 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   record(c, kEvAnalyzeEnd);
   launch_t1_model(ta, c->num_sms, c->stream);
   record(c, kEvModelEnd);
-  // Blocks are coded heaviest first: with several blocks per warp so that a
-  // warp's lanes carry similar symbol counts; with one block per warp by a
-  // fixed number of warps per SM that pull blocks in that order, so the
-  // longest chains start first and share their schedulers with few others.
-  // Automatic choice (measured on 1275x1650 to 5100x6600 pages): up to 48
-  // blocks per SM, producer/consumer pipelines pulling blocks; beyond that,
-  // 2..32 blocks packed per warp.
-  const int64_t bpw_opt = c->opt[JP2G_OPT_MQ_BLOCKS_PER_WARP];
-  const int64_t wps_opt = c->opt[JP2G_OPT_MQ_WARPS_PER_SM];
-  const uint32_t sms = (uint32_t)c->num_sms;
-  const int bpw = mq_blocks_per_warp(ta, c->num_sms, (int)bpw_opt);
-  const bool use_pull = bpw == 1 && wps_opt >= 0;
-  const int pull = wps_opt > 0 ? (int)wps_opt : (nb <= sms * 16u ? 8 : 12);
-  int order_launches = 0;
-  if (bpw > 1 || use_pull) {
-    if (!reserve(c, c->mqorder, (size_t)nb * 4) || !reserve(c, c->mqscratch, ((size_t)nb + 2048) * 4))
-      return kEncodeFailed;
-    launch_mq_order(ta, dptr<uint32_t>(c->mqorder), dptr<uint32_t>(c->mqscratch), c->stream);
-    ta.mq_order = dptr<uint32_t>(c->mqorder);
-    order_launches = 3;
-  }
-  // Producer/consumer pairs shorten each block's chain (8 pairs per SM, one
-  // or two chains each); up to 48 blocks per SM they beat single-warp
-  // pulling and packed warps.
-  const int64_t pipes_opt = c->opt[JP2G_OPT_MQ_PIPES_PER_SM];
-  const bool use_pipe = use_pull && (pipes_opt > 0 || (pipes_opt == 0 && nb <= sms * 48u));
-  if (use_pipe) {
-    // four chains per pair run on 4 pairs per SM (16 chains per SM, as 8
-    // pairs of two): measured best for an sRGB 2550x3300 page
-    const int chains = mq_chains_per_pair(c, nb);
-    launch_t1_mq_pipe(ta, c->num_sms, pipes_opt > 0 ? (int)pipes_opt : (chains == 4 ? 4 : 8), chains,
-                      (uint32_t)c->opt[JP2G_OPT_MQ_HEAVY], dptr<uint32_t>(c->stats) + 2, c->stream);
-  }
-  else if (use_pull)
-    launch_t1_mq_pull(ta, c->num_sms, pull, dptr<uint32_t>(c->stats) + 2, c->stream);
-  else
-    launch_t1_mq(ta, c->num_sms, bpw, c->stream);
-  c->counters[5] += 5 + (nb > 1024 ? 1 : 0) + order_launches;
+  // Blocks are coded heaviest first, one per lane: a warp's lanes then carry
+  // similar symbol counts, and the longest chains start first.
+  if (!reserve(c, c->mqorder, (size_t)nb * 4) || !reserve(c, c->mqscratch, ((size_t)nb + 2048) * 4))
+    return kEncodeFailed;
+  launch_mq_order(ta, dptr<uint32_t>(c->mqorder), dptr<uint32_t>(c->mqscratch), c->stream);
+  ta.mq_order = dptr<uint32_t>(c->mqorder);
+  launch_t1_mq(ta, c->num_sms, (int)c->opt[JP2G_OPT_MQ_BLOCKS_PER_WARP], c->stream);
+  c->counters[5] += 8 + (nb > 1024 ? 1 : 0);
   record(c, 3);
   // ---- PCRD ----
   PcrdArgs pa{};
@@ -2178,31 +2136,18 @@ int jp2g_autotune(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, int repeats
     if (why == -2.0)
       return set_err(c, JP2G_ENCODE_FAILED,
                      "autotune: a scheduling setting changed the codestream (mq_blocks_per_warp=" +
-                         std::to_string(o[JP2G_OPT_MQ_BLOCKS_PER_WARP]) + ", mq_warps_per_sm=" +
-                         std::to_string(o[JP2G_OPT_MQ_WARPS_PER_SM]) + ", mq_pipes_per_sm=" +
-                         std::to_string(o[JP2G_OPT_MQ_PIPES_PER_SM]) + ", mq_chains_per_pair=" +
-                         std::to_string(o[JP2G_OPT_MQ_CHAINS_PER_PAIR]) + ", wave_blocks=" +
+                         std::to_string(o[JP2G_OPT_MQ_BLOCKS_PER_WARP]) + ", wave_blocks=" +
                          std::to_string(o[JP2G_OPT_WAVE_BLOCKS]) + ")");
     return set_err(c, JP2G_ENCODE_FAILED, "autotune: the sample failed to encode: " + get_msg(c));
   };
   if (encode_once(saved, true) < 0) return fail(saved, -1.0);
 
-  // stage 1: MQ schedule (automatic; producer/consumer pipelines; single-warp
-  // pulling; blocks packed per warp)
-  struct Mq { int64_t bpw, wps, pipes, chains; };
-  const Mq mq[] = {{0, 0, 0, 0},   {1, 0, 4, 1},   {1, 0, 8, 1},   {1, 0, 16, 1}, {1, 0, 4, 2},
-                   {1, 0, 8, 2},   {1, 0, 16, 2},  {1, 0, 4, 4},   {1, 0, 8, 4},  {1, 8, -1, 0},
-                   {1, 12, -1, 0}, {1, 16, -1, 0}, {2, 0, 0, 0},   {4, 0, 0, 0},  {8, 0, 0, 0},
-                   {16, 0, 0, 0},  {32, 0, 0, 0}};
+  // stage 1: MQ schedule (automatic; blocks packed per warp)
   int64_t cur[JP2G_NUM_OPTS], win[JP2G_NUM_OPTS];
   std::memcpy(cur, saved, sizeof cur);
-  cur[JP2G_OPT_MQ_HEAVY] = 0;
   double win_ms = 1e300;
-  for (const Mq& m : mq) {
-    cur[JP2G_OPT_MQ_BLOCKS_PER_WARP] = m.bpw;
-    cur[JP2G_OPT_MQ_WARPS_PER_SM] = m.wps;
-    cur[JP2G_OPT_MQ_PIPES_PER_SM] = m.pipes;
-    cur[JP2G_OPT_MQ_CHAINS_PER_PAIR] = m.chains;
+  for (int64_t bpw : {0ll, 1ll, 2ll, 4ll, 8ll, 16ll, 32ll}) {
+    cur[JP2G_OPT_MQ_BLOCKS_PER_WARP] = bpw;
     const double t = time_candidate(cur);
     if (t < 0) return fail(cur, t);
     if (t < win_ms) {

@@ -224,7 +224,7 @@ __global__ void copy_bodies_kernel(const BlockDesc* blocks, const BlockKeep* kee
   if (warp >= n) return;
   const uint32_t off = offsets[warp];
   const uint32_t len = keep[warp].body_len;
-  const uint8_t* s = src + blocks[warp].out_off;
+  const uint8_t* s = src + blocks[warp].out_off + 1;  // after the pre-byte
   for (uint32_t i = lane; i < len; i += 32) dst[off + i] = s[i];
 }
 

@@ -39,6 +39,11 @@ namespace {
 
 // Context numbers (src/mq/mod.rs:5-10).
 constexpr int kCtxAGG = 17, kCtxUNI = 18;
+constexpr uint32_t kCtxNone = 19;               // a context of Qe 0: coding its symbols changes nothing
+constexpr uint32_t kPadSymbol = kCtxNone;  // pads symbol streams to whole chunks
+// A symbol is a byte: context | decision << 7.
+constexpr uint32_t kOne = 0x80u;
+constexpr uint32_t kMqCtx = 20;
 constexpr int kModelWarps = 4;  // 7 KB of shared memory each: 6 CTAs per SM
 constexpr int kMqWarps = 4;
 
@@ -263,6 +268,9 @@ __device__ __forceinline__ uint32_t warp_offset(uint32_t v, int lane, uint32_t* 
   return x - v;
 }
 
+// A pass's symbols fill whole 16-byte chunks of its item's slot.
+__device__ __forceinline__ uint32_t pad16(uint32_t n) { return (n + 15u) & ~15u; }
+
 // Writes the symbols of one column of one stripe into the three streams.
 __device__ __forceinline__ void emit_column(uint32_t v, uint32_t sm, uint32_t c, uint32_t b, uint32_t cl,
                                             uint32_t prim, uint32_t sgn, uint8_t*& osp, uint8_t*& omr,
@@ -270,13 +278,13 @@ __device__ __forceinline__ void emit_column(uint32_t v, uint32_t sm, uint32_t c,
   int first = 0;  // rows consumed by a cleanup run
   if (cl) {
     if (b == 0) {
-      *ocl++ = (uint8_t)((uint32_t)kCtxAGG << 1);
+      *ocl++ = (uint8_t)kCtxAGG;
       first = 4;
     } else {
       const int rl = __ffs(b) - 1;
-      ocl[0] = (uint8_t)(((uint32_t)kCtxAGG << 1) | 1u);
-      ocl[1] = (uint8_t)(((uint32_t)kCtxUNI << 1) | ((uint32_t)rl >> 1));
-      ocl[2] = (uint8_t)(((uint32_t)kCtxUNI << 1) | ((uint32_t)rl & 1u));
+      ocl[0] = (uint8_t)(kCtxAGG | kOne);
+      ocl[1] = (uint8_t)(kCtxUNI | ((uint32_t)rl >> 1) << 7);
+      ocl[2] = (uint8_t)(kCtxUNI | ((uint32_t)rl & 1u) << 7);
       ocl[3] = (uint8_t)(sgn >> (8 * rl));  // sign of the run's first significant sample
       ocl += 4;
       first = rl + 1;
@@ -443,7 +451,8 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a)
 
     // ---- 4. emission, stripe by stripe ----
     uint8_t* out = a.sym + (size_t)item * a.sym_slot;
-    uint32_t pos_sp = 0, pos_mr = n_sp, pos_cl = n_sp + sig_before;
+    const uint32_t at_mr = pad16(n_sp), at_cl = at_mr + pad16(sig_before);
+    uint32_t pos_sp = 0, pos_mr = at_mr, pos_cl = at_cl;
     const int nstripes = (h + 3) >> 2;
     for (int half = 0; half < 2 && 8 * half < nstripes; ++half) {
       uint32_t qa[kNumPlanes], qb[kNumPlanes];
@@ -462,17 +471,17 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a)
         const uint32_t offA = warp_offset(column_counts(vA4, sA4, cA4, bA4, lA), lane, &totA);
         const uint32_t offB = warp_offset(column_counts(vB4, sB4, cB4, bB4, lB), lane, &totB);
         // primary and sign symbols of the 4 rows, one per byte
-        uint32_t primA = spread4(bA4), primB = spread4(bB4);
+        uint32_t primA = spread4(bA4) << 7, primB = spread4(bB4) << 7;
         #pragma unroll
         for (int k = 0; k < 5; ++k) {
-          primA |= spread4(nib(qa[kPlP0 + k], s)) << (k + 1);
-          primB |= spread4(nib(qb[kPlP0 + k], s)) << (k + 1);
+          primA |= spread4(nib(qa[kPlP0 + k], s)) << k;
+          primB |= spread4(nib(qb[kPlP0 + k], s)) << k;
         }
-        uint32_t sgnA = 0x10101010u | spread4(nib(qa[kPlX], s)), sgnB = 0x10101010u | spread4(nib(qb[kPlX], s));
+        uint32_t sgnA = 0x08080808u | spread4(nib(qa[kPlX], s)) << 7, sgnB = 0x08080808u | spread4(nib(qb[kPlX], s)) << 7;
         #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          sgnA |= spread4(nib(qa[kPlM0 + k], s)) << (k + 1);
-          sgnB |= spread4(nib(qb[kPlM0 + k], s)) << (k + 1);
+          sgnA |= spread4(nib(qa[kPlM0 + k], s)) << k;
+          sgnB |= spread4(nib(qb[kPlM0 + k], s)) << k;
         }
         uint8_t* osp = out + pos_sp + (offA & 0x7ffu);
         uint8_t* omr = out + pos_mr + ((offA >> 11) & 0x3ffu);
@@ -487,11 +496,15 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a)
         pos_cl += (totA >> 21) + (totB >> 21);
       }
     }
+    // padding of each pass to whole 16-symbol chunks
+    if (pos_sp + lane < at_mr) out[pos_sp + lane] = (uint8_t)kPadSymbol;
+    if (pos_mr + lane < at_cl) out[pos_mr + lane] = (uint8_t)kPadSymbol;
+    if (pos_cl + lane < pad16(pos_cl)) out[pos_cl + lane] = (uint8_t)kPadSymbol;
     if (lane == 0) {
       ItemRec rec;
       rec.n_sp = n_sp;
       rec.n_mr = sig_before;
-      rec.n_cl = pos_cl - (n_sp + sig_before);
+      rec.n_cl = pos_cl - at_cl;
       rec.ns_sp = ns_sp;
       rec.ns_cl = ns_cl;
       rec.sig_before = sig_before;
@@ -504,593 +517,309 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a)
 }
 
 // --------------------------------------------------------------------- MQ --
-// The coder runs one code-block per lane. Every step is written without
-// data-dependent branches (conditional exchange, renormalisation and byte
-// output are predicated), so the 32 lanes of a warp, each coding a different
-// block, stay converged; only pass boundaries and stream refills branch.
+// The coder runs one code-block per lane, 1 to 32 lanes of a warp. A symbol
+// takes the same instructions on every lane whatever it does, so a warp of 32
+// blocks issues as many as a warp of one. What bounds it: in batches the
+// ALU pipe (half rate; 77 % busy) and the latency of the context entries in
+// shared memory; on a single page one chain's latency.
 //
-// Per context the shared table holds the full probability-state entry
-// (qe | MPS << 16 | next-MPS index << 17 | next-LPS index << 24), so one load
-// yields qe and the MPS; the state table T is only consulted to move a
-// context to its next state.
+// - Interval register as a float in [1, 2) (A / 2^15): A - Qe, its comparison
+//   with Qe and the renormalised result are exact in 24 bits, and
+//   renormalisation is a logic operation that sets the exponent, where an
+//   integer needs a leading-zero count and a shift on the chain.
+// - The code register and the byte output, which part the lanes of a warp
+//   when done per symbol, are done once per 16 symbols (mq_chunk16).
+// - Each pass's symbols are padded to whole 16-symbol chunks with symbols that
+//   change nothing (t1_model_kernel), so a pass ends between two chunks.
+//
+// Measured (2550x3300 gray q85 page; batch of 24 sRGB q75 pages): MQ stage 3.04
+// and 5.2 ms (403 G symbols/s); 4.38 and 11.1 ms with an integer coder, split
+// over producer/consumer warp pairs on the page, branching at its byte output
+// in the batch. A lone chain takes 105 cycles per symbol.
+// Context entry, in shared memory: x = Qe / 2^15 as a float, its sign bit the
+// MPS; y = offset of the state's successors in the table | Qe << 16. The table
+// holds per state (state, MPS pair) its successors' entries: after an MPS
+// renormalisation, then after an LPS.
+constexpr uint32_t kStates = 94;
+// Padding's Qe: too small to change A in a subtraction (1 - 2^-30 rounds to
+// 1), and its exponent's upper bits are those of every Qe (mq_code8).
+constexpr uint32_t kPadQe = 0x30800000u;
+struct MqTable {
+  uint2 next[kStates][2];
+};
+__device__ __forceinline__ uint2 mq_entry(uint32_t state) {
+  const uint32_t qe = c_tables.mq[state] & 0xffffu;
+  return make_uint2(__float_as_uint((float)qe * (1.0f / 32768.0f)) | (state & 1u) << 31, state * 16u | qe << 16);
+}
+__device__ __forceinline__ void load_mq_table(MqTable& t) {
+  for (uint32_t i = threadIdx.x; i < kStates; i += blockDim.x) {
+    const uint32_t v = c_tables.mq[i];  // qe | nmps << 16 | nlps << 24
+    t.next[i][0] = mq_entry((v >> 16) & 0xffu);
+    t.next[i][1] = mq_entry(v >> 24);
+  }
+}
+
 struct Mq {
-  uint32_t a, c, ct;
-  int pos;        // index of the last written byte; 0 is the pre-byte
-  uint32_t last;  // value of that byte
-  uint8_t* out;   // out[k] holds byte k+1
-  int cap;
-  int ovf;
+  float a;        // interval, A / 2^15 in [1, 2)
+  uint32_t c;     // code register
+  int ct;         // shifts left until a byte is cut
+  uint32_t last;  // the last byte cut, before the next one's carry into it
+  uint8_t* at;    // its place; a block's slot begins with the pre-byte
 };
 
-// BYTEOUT (src/mq/mod.rs:382-404) as straight-line code: a carry into the
-// previous byte is applied first, then one byte is emitted (7 bits after an
-// 0xFF, 8 otherwise).
-__device__ __forceinline__ void mq_byteout(Mq& m) {
-  const bool carry = m.last != 0xffu && (m.c & 0x8000000u) != 0;
-  if (carry) {
-    m.last = (m.last + 1) & 0xffu;
-    if (m.pos >= 1 && m.pos <= m.cap) m.out[m.pos - 1] = (uint8_t)m.last;
-    if (m.last == 0xffu) m.c &= 0x7ffffffu;
-  }
-  const bool big = m.last == 0xffu;
-  const uint32_t byte = (big ? (m.c >> 20) : (m.c >> 19)) & 0xffu;
-  m.c &= big ? 0xfffffu : 0x7ffffu;
-  m.ct = big ? 7u : 8u;
-  ++m.pos;
-  m.last = byte;
-  if (m.pos <= m.cap) m.out[m.pos - 1] = (uint8_t)byte;
-  else m.ovf = 1;
+// Payload bytes are written by volatile assembly, which keeps its order: a
+// byte may be written again by mq_shift.
+__device__ __forceinline__ void put_byte(uint8_t* at, uint32_t v) {
+  asm volatile("st.global.u8 [%0], %1;" ::"l"(at), "r"(v));
 }
 
-// Probability-state entry of a context, in shared memory: x = qe |
-// (leading zeros of qe in 16 bits) << 16 | MPS << 20; y = index of the next
-// state after an MPS renormalisation | index after an LPS << 8 (indices
-// into the 94-entry table of (state, MPS) pairs).
-//
-// One MQ symbol (C.2.4-C.2.7) with the decisions folded: after A -= qe the
-// coder keeps A (and adds qe to C) exactly when (A < qe) equals "LPS", and
-// otherwise takes qe (C unchanged). A stays >= 0x8000 between symbols and qe
-// <= 0x5601, so a kept A is either >= 0x8000 (no renormalisation) or in
-// [0x29ff, 0x8000) (a shift of 1 or 2), while a taken qe shifts by its
-// stored leading-zero count. The context moves to its next state exactly
-// when the shift is non-zero. Returns the context's new entry.
-__device__ __forceinline__ uint2 mq_step(Mq& m, uint2 e, uint32_t sym, const uint2* T) {
-  const uint32_t qe = e.x & 0xffffu;
-  const uint32_t lps = ((e.x >> 20) ^ sym) & 1u;
-  const uint32_t a = m.a - qe;
-  const bool take_a = (a < qe) == (lps != 0);
-  uint32_t n = take_a ? (a < 0x4000u ? 2u : (a < 0x8000u ? 1u : 0u)) : ((e.x >> 16) & 15u);
-  m.c += take_a ? qe : 0u;
-  m.a = (take_a ? a : qe) << n;
-  uint2 ne = e;
-  if (n) ne = T[lps ? (e.y >> 8) : (e.y & 0xffu)];
-  if (n >= m.ct) {
-    do {
-      m.c <<= m.ct;
-      n -= m.ct;
-      mq_byteout(m);
-    } while (n >= m.ct);
+// Adds to the code register and shifts it by n bits, cutting bytes as it
+// fills (BYTEOUT, src/mq/mod.rs:382-404).
+__device__ __forceinline__ void mq_shift(Mq& m, uint32_t add, int n) {
+  uint32_t c = m.c + add;
+  while (n >= m.ct) {
+    c <<= m.ct;
+    n -= m.ct;
+    if (m.last != 0xffu && (c & 0x8000000u) != 0) {
+      ++m.last;
+      if (m.last == 0xffu) c &= 0x7ffffffu;
+    }
+    put_byte(m.at++, m.last);
+    const bool big = m.last == 0xffu;
+    m.last = (big ? c >> 20 : c >> 19) & 0xffu;
+    c &= big ? 0xfffffu : 0x7ffffu;
+    m.ct = big ? 7 : 8;
   }
-  m.c <<= n;
   m.ct -= n;
-  return ne;
+  m.c = c << n;
 }
 
-__device__ __forceinline__ void mq_flush(Mq& m) {  // src/mq/mod.rs:244-250, 373-379
-  uint32_t t = m.c + m.a;
-  m.c |= 0xffffu;
-  if (m.c >= t) m.c -= 0x8000u;
-  m.c <<= m.ct;
-  mq_byteout(m);
-  m.c <<= m.ct;
-  mq_byteout(m);
+// Context entries of a CTA's lanes: context c of thread t at byte
+// c * kCtxStride + 8 t (no bank conflicts whatever contexts the lanes use).
+constexpr uint32_t kCtxStride = kMqWarps * 32 * 8;
+static_assert(kCtxStride == 1024, "the context offset is a shift of the symbol");
+struct MqSmem {
+  __align__(16) uint8_t ce[kMqCtx * kCtxStride];
+  MqTable table;
+};
+__device__ __forceinline__ uint2& ctx_at(MqSmem& sm, uint32_t off) {
+  return *reinterpret_cast<uint2*>(sm.ce + off);
 }
-
-// Symbol i (0..15) of a 16-byte chunk.
-__device__ __forceinline__ uint32_t chunk_sym(const uint4& q, int i) {
-  const uint32_t w = i < 8 ? (i < 4 ? q.x : q.y) : (i < 12 ? q.z : q.w);
-  return (w >> (8 * (i & 3))) & 0xffu;
+// Offset of the context entry of symbol i (0..3) of a word for the lane whose
+// entries start at `lane`; the symbol's decision as a sign bit.
+__device__ __forceinline__ uint32_t sym_ctx(uint32_t w, int i, uint32_t lane) {
+  return ((i < 2 ? w << (10 - 8 * i) : w >> (8 * i - 10)) & 0x7c00u) | lane;
 }
+__device__ __forceinline__ uint32_t sym_sign(uint32_t w, int i) { return w << (24 - 8 * i); }
 
-// Codes all 16 symbols of a chunk, the next symbol's context entry loaded
-// one step ahead of its use, capturing numbytes() after symbols e0 - 1 and
-// e1 - 1 (pass ends; outside 1..16 they capture nothing) with predicated
-// selects, so lanes of a warp at different pass ends stay converged.
-__device__ __forceinline__ void mq_chunk16_at(Mq& m, uint2* ce, const uint2* T, const uint4 q, int e0,
-                                              int e1, uint32_t& p0, uint32_t& p1) {
-  uint32_t sym = q.x & 0xffu;
-  uint2 e = ce[32 * (sym >> 1)];
+// Codes the 16 symbols of a chunk.
+//
+// A symbol (C.2.4-C.2.7) with the decisions folded: after A -= Qe the coder
+// keeps A (and adds Qe to C) exactly when (A < Qe) equals "LPS", and
+// otherwise takes Qe (C unchanged). The context moves to its next state
+// exactly when the result is below 0x8000 and is renormalised.
+//
+// The code register is brought up to date once for the chunk: its 16
+// additions are summed at 31 fractional bits (`acc`), each at the shift it
+// comes at, and bytes are cut from the sum. A byte is then cut with additions
+// in the sum that come after it. They can only carry one into it, as the
+// next cut would have found; what they could get wrong is a byte of 0xFF
+// that such a carry turns to zeros, so a byte of zeros with the three bits
+// below it zero too (a carry adds less than their weight) makes the chunk
+// take the additions one by one, as does one that shifts by more than 31
+// bits.
+__device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, const uint4 q) {
+  const uint32_t w[5] = {q.x, q.y, q.z, q.w, kPadSymbol};
+  const uint32_t table = (uint32_t)__cvta_generic_to_shared(&sm.table) - 3u;
+  uint32_t add[16], ex[16];
+  uint64_t acc = 0;
+  int room = 31;  // fractional bits left: 31 - shifts so far
+  uint32_t cx = sym_ctx(w[0], 0, lane);
+  uint2 e = ctx_at(sm, cx);
   #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const uint32_t symn = i < 15 ? chunk_sym(q, i + 1) : 0u;
-    const uint32_t cx = sym >> 1, cxn = symn >> 1;
-    uint2 en = i < 15 ? ce[32 * cxn] : make_uint2(0u, 0u);
-    const uint2 ne = mq_step(m, e, sym, T);
-    ce[32 * cx] = ne;
-    if (cxn == cx) en = ne;
-    e = en;
-    sym = symn;
-    p0 = e0 == i + 1 ? (uint32_t)m.pos : p0;
-    p1 = e1 == i + 1 ? (uint32_t)m.pos : p1;
+    const uint32_t cxn = sym_ctx(w[(i + 1) >> 2], (i + 1) & 3, lane);
+    const uint2 en = ctx_at(sm, cxn);  // the next symbol's entry, one step ahead
+    const float qe = fabsf(__uint_as_float(e.x));
+    const uint32_t xs = e.x ^ (sym_sign(w[i >> 2], i & 3) & 0x80000000u);
+    const bool lps = (int)xs < 0;
+    // bits 28..30 of every Qe are 3, so the top four bits are 8 * lps + 3
+    const uint32_t next = table + (((xs >> 28) & ~0x7f0u) | (e.y & 0x7f0u));
+    const float a = __fsub_rn(m.a, qe);
+    const bool take_a = (a < qe) == lps;
+    const float v = take_a ? a : qe;
+    const uint32_t vb = __float_as_uint(v);
+    m.a = __uint_as_float((vb & 0x7fffffu) | 0x3f800000u);
+    add[i] = take_a ? e.y >> 16 : 0u;
+    ex[i] = vb >> 23;  // 127 - the shift
+    acc += (uint64_t)add[i] * __funnelshift_l(0u, 1u, (uint32_t)room);
+    room += (int)ex[i] - 127;
+    // the next state, loaded only when renormalised (selecting from a load
+    // made ahead costs more in selects than it hides)
+    asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, 0f3F800000;\n\t@p ld.shared.v2.u32 {%0, %1}, [%3];\n\t}"
+        : "+r"(e.x), "+r"(e.y)
+        : "f"(v), "r"(next));
+    ctx_at(sm, cx) = e;
+    e.x = cxn == cx ? e.x : en.x;
+    e.y = cxn == cx ? e.y : en.y;
+    cx = cxn;
+  }
+  bool one_by_one = room < 0;
+  if (!one_by_one) {
+    uint64_t x = (((uint64_t)m.c << 31) + acc) << m.ct;  // C at its next cut, 31 fractional bits
+    int t = m.ct + room - 31;                            // shifts that cut lacks
+    uint32_t last = m.last;
+    uint8_t* at = m.at;
+    while (t <= 0) {
+      const uint32_t hi = (uint32_t)(x >> 32);  // C's bit k at k - 1
+      one_by_one |= ((hi >> 15) & 0x7ffu) == 0;
+      const uint32_t done = last == 0xffu ? 0xffu : last + (hi >> 26);  // with the carry
+      const bool big = done == 0xffu;
+      put_byte(at++, done);
+      // after 0xFF a byte takes 7 bits, and the carry place when it was
+      // 0xFF before the carry
+      last = big ? (last == 0xffu ? hi >> 19 : (hi >> 19) & 0x7fu) : (hi >> 18) & 0xffu;
+      const int bits = big ? 7 : 8;
+      x = ((uint64_t)(hi & (big ? 0x7ffffu : 0x3ffffu)) << 32 | (uint32_t)x) << bits;
+      t += bits;
+    }
+    if (!one_by_one) {
+      m.c = (uint32_t)(x >> 32) >> (t - 1);
+      m.ct = t;
+      m.last = last;
+      m.at = at;
+    }
+  }
+  if (one_by_one) {
+    #pragma unroll
+    for (int i = 0; i < 16; ++i) mq_shift(m, add[i], 127 - (int)ex[i]);
   }
 }
 
-// Per-block MQ coding over the symbol streams of the block's bit-planes.
-// Blocks go `bpw` to a warp, one per lane: 32 when enough blocks are in
-// flight to fill the GPU, 1 when a single page leaves it mostly idle and the
-// longest block's serial chain sets the time (lanes of a warp diverge on
-// every byte emitted, which lengthens each lane's chain).
-// The 94 state entries in the layout mq_step uses.
-__device__ __forceinline__ void load_mq_table(uint2* T) {
-  for (int i = threadIdx.x; i < 94; i += blockDim.x) {
-    // (qe | nmps << 16 | nlps << 24) -> the entry layout of mq_step
-    const uint32_t v = c_tables.mq[i];
-    const uint32_t qe = v & 0xffffu;
-    T[i] = make_uint2(qe | ((uint32_t)(__clz(qe) - 16) << 16) | ((uint32_t)(i & 1) << 20),
-                      ((v >> 16) & 0xffu) | (((v >> 24) & 0xffu) << 8));
-  }
-}
-
-// MQ-codes code-block b on the calling lane; ce is the lane's context
-// column (context c at ce[32 * c]).
-__device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, uint2* ce, const uint2* T) {
-  BlockOut o = a.res[b];
+// MQ-codes code-block b on the calling lane, or nothing when b is kNoBlock;
+// every lane of the warp calls. The lanes meet at every chunk (the vote):
+// left to themselves, a lane that ends a pass falls behind the others and
+// each would run the chunk code on its own.
+constexpr uint32_t kNoBlock = 0xffffffffu;
+__device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSmem& sm) {
+  const uint32_t lane = threadIdx.x * 8u;
+  BlockOut o{};
+  if (b != kNoBlock) o = a.res[b];
   const int mbp = o.status ? 0 : o.mbp;
-  if (mbp == 0) return;
-  const BlockDesc d = a.blocks[b];
-  // contexts: state 0 except UNI 46, AGG 3, ZC 4 (src/mq/mod.rs:195-200)
-  for (int c = 0; c < 19; ++c) ce[32 * c] = T[0];
-  ce[32 * kCtxUNI] = T[92];
-  ce[32 * kCtxAGG] = T[6];
-  ce[0] = T[8];
-  Mq m{0x8000u, 0u, 12u, 0, 0u, a.out + d.out_off, (int)d.out_cap, 0};
+  bool active = mbp > 0;
+  BlockDesc d{};
+  uint32_t base = 0;
+  ItemRec r{};
+  const uint4* src = nullptr;
+  uint4 c0 = make_uint4(0u, 0u, 0u, 0u), c1 = c0;
+  if (active) {
+    d = a.blocks[b];
+    base = a.plane_base[b];
+    r = a.item_rec[base];
+    src = reinterpret_cast<const uint4*>(a.sym + (size_t)base * a.sym_slot);
+    c0 = src[0];
+    c1 = src[1];  // the slot and buffer are padded for these reads
+    // contexts: state 0 except UNI 46, AGG 3, ZC 4 (src/mq/mod.rs:195-200)
+    for (uint32_t c = 0; c < kMqCtx; ++c)
+      ctx_at(sm, c * kCtxStride + lane) = c == kCtxNone ? make_uint2(kPadQe, 0u)
+                                                        : mq_entry(c == kCtxUNI ? 92 : c == kCtxAGG ? 6 : c == 0 ? 8 : 0);
+  }
+  uint8_t* const slot = a.out + d.out_off;
+  const uint8_t* const slot_end = slot + d.out_cap - 40;  // a chunk cuts at most 35 bytes
+  Mq m{1.0f, 0u, 12, 0u, slot};
+  bool ovf = false;
   PassRec* pr = a.passes + d.pass_off;
-  const uint32_t base = a.plane_base[b];
-  int pi = 0;
-  uint32_t nsym = 0;
-  // One flat loop over the chunks of all items (bit-planes), so lanes of a
-  // warp coding different blocks stay in the same code; the next item's
-  // record and first chunks are fetched during the current item's last
-  // chunk.
-  ItemRec r = a.item_rec[base];
-  ItemRec rn = mbp > 1 ? a.item_rec[base + 1] : r;
-  const uint4* src = reinterpret_cast<const uint4*>(a.sym + (size_t)base * a.sym_slot);
-  uint4 c0 = src[0], c1 = src[1], c2 = src[2];  // the slot and buffer are padded for these reads
-  uint4 n0 = c0, n1 = c0, n2 = c0;
-  int j = 0, lo = 0, kp = 0;
-  auto item_total = [](const ItemRec& x) { return (int)(x.n_sp + x.n_mr + x.n_cl); };
-  // pass ends of item j: SP | MR | CL, or CL alone for the first item
-  auto end_of = [&](int k) {
-    if (j == 0) return item_total(r);
-    return k == 0 ? (int)r.n_sp : (k == 1 ? (int)(r.n_sp + r.n_mr) : item_total(r));
-  };
-  auto record = [&](int k, uint32_t pos) {  // numbytes() after pass k
+  // One flat loop over the chunks of all items (bit-planes); the next item's
+  // record and first chunks are fetched during the current item's last chunk.
+  ItemRec rn = r;
+  uint4 n0 = c0, n1 = c0;
+  uint32_t nsym = r.n_cl;
+  int j = 0, k = 2;                     // item and pass (SP, MR, cleanup; the first item has only its cleanup)
+  uint32_t left = (r.n_cl + 15u) >> 4;  // chunks of the pass
+  uint32_t ahead = left;                // chunks of the item
+  auto record = [&] {                   // numbytes() after the pass
+    const uint32_t pos = (uint32_t)(m.at - slot);
     const uint8_t bp = (uint8_t)r.bitplane;
-    if (j == 0 || k == 2)
-      pr[pi] = PassRec{pos, r.ns_cl, j == 0 ? 0u : r.sig_before + r.ns_sp, 2, bp, 0};
+    if (k == 2)
+      *pr = PassRec{pos, r.ns_cl, j == 0 ? 0u : r.sig_before + r.ns_sp, 2, bp, 0};
     else if (k == 0)
-      pr[pi] = PassRec{pos, r.ns_sp, r.sig_before, 0, bp, 0};
+      *pr = PassRec{pos, r.ns_sp, r.sig_before, 0, bp, 0};
     else
-      pr[pi] = PassRec{pos, 0u, r.sig_before, 1, bp, 0};
-    ++pi;
+      *pr = PassRec{pos, 0u, r.sig_before, 1, bp, 0};
+    ++pr;
   };
-  int npass = 1, total = item_total(r);
-  nsym = (uint32_t)total;
-  for (;;) {
-    // passes of item j that end at its first symbol
-    while (kp < npass - 1 && end_of(kp) == lo) record(kp++, (uint32_t)m.pos);
-    const int cnt = min(16, total - lo);
-    const bool last = lo + cnt >= total;
-    if (last && j + 1 < mbp) {
+  while (__any_sync(0xffffffffu, active)) {
+    if (!active) continue;
+    if (ahead == 1 && j + 1 < mbp) {
+      rn = a.item_rec[base + j + 1];
       const uint4* ns = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j + 1) * a.sym_slot);
       n0 = ns[0];
       n1 = ns[1];
-      n2 = ns[2];
     }
     const uint4 q = c0;
     c0 = c1;
-    c1 = c2;
-    c2 = src[(lo >> 4) + 3];  // 48 bytes ahead: inside the slot or the buffer's pad
-    const int e0 = kp < npass - 1 ? end_of(kp) - lo : -1;
-    const int e1 = kp + 1 < npass - 1 ? end_of(kp + 1) - lo : -1;
-    uint32_t p0 = 0, p1 = 0;
-    if (cnt == 16) {
-      mq_chunk16_at(m, ce, T, q, e0, e1, p0, p1);
-    } else {
-      for (int i = 0; i < cnt; ++i) {
-        const uint32_t sym = chunk_sym(q, i);
-        const uint32_t cx = sym >> 1;
-        ce[32 * cx] = mq_step(m, ce[32 * cx], sym, T);
-        p0 = e0 == i + 1 ? (uint32_t)m.pos : p0;
-        p1 = e1 == i + 1 ? (uint32_t)m.pos : p1;
+    c1 = src[2];  // 32 bytes ahead: inside the slot or the buffer's pad
+    ++src;
+    mq_chunk16(m, sm, lane, q);
+    if (m.at > slot_end) {  // no room for another chunk: the block has failed
+      ovf = true;
+      m.at = slot;
+    }
+    --ahead;
+    if (--left == 0) {
+      record();
+      while (k < 2 && left == 0) {  // the next pass that has symbols
+        ++k;
+        left = ((k == 1 ? r.n_mr : r.n_cl) + 15u) >> 4;
+        if (left == 0) record();
+      }
+      if (left == 0) {  // the next item
+        if (++j == mbp) {
+          active = false;
+        } else {
+          r = rn;
+          src = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j) * a.sym_slot);
+          c0 = n0;
+          c1 = n1;
+          nsym += r.n_sp + r.n_mr + r.n_cl;
+          ahead = ((r.n_sp + 15u) >> 4) + ((r.n_mr + 15u) >> 4) + ((r.n_cl + 15u) >> 4);
+          k = 0;
+          left = (r.n_sp + 15u) >> 4;
+          while (k < 2 && left == 0) {
+            record();
+            ++k;
+            left = ((k == 1 ? r.n_mr : r.n_cl) + 15u) >> 4;
+          }
+        }
       }
     }
-    if (e0 >= 1 && e0 <= cnt) {
-      record(kp++, p0);
-      if (e1 >= 1 && e1 <= cnt) record(kp++, p1);
-    }
-    lo += cnt;
-    if (!last) continue;
-    record(npass == 1 ? 0 : 2, (uint32_t)m.pos);  // cleanup: the item's last pass
-    if (++j == mbp) break;
-    r = rn;
-    if (j + 1 < mbp) rn = a.item_rec[base + j + 1];
-    src = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j) * a.sym_slot);
-    c0 = n0;
-    c1 = n1;
-    c2 = n2;
-    lo = 0;
-    kp = 0;
-    npass = 3;
-    total = item_total(r);
-    nsym += (uint32_t)total;
   }
-  mq_flush(m);
-  o.payload_len = (uint32_t)(m.last == 0xffu ? m.pos - 1 : m.pos);  // take_bytes
-  o.status = m.ovf ? 1 : 0;
+  if (mbp == 0) return;
+  // termination (src/mq/mod.rs:244-250, 373-379)
+  uint32_t c = m.c;
+  const uint32_t t = c + ((__float_as_uint(m.a) & 0x7fffffu) | 0x800000u) / 256u;
+  c |= 0xffffu;
+  if (c >= t) c -= 0x8000u;
+  m.c = c;
+  mq_shift(m, 0u, m.ct);
+  mq_shift(m, 0u, m.ct);
+  put_byte(m.at, m.last);
+  const uint32_t pos = (uint32_t)(m.at - slot);
+  o.payload_len = m.last == 0xffu ? pos - 1 : pos;  // take_bytes
+  o.status = ovf ? 1 : 0;
   a.res[b] = o;
   atomicAdd(a.sym_count, (unsigned long long)nsym);
 }
 
-// ------------------------------------------------- two-warp MQ pipeline --
-// For one code-block at a time, the MQ coder splits into two chains: the
-// interval and context-state chain (A register, probability states) and the
-// code register chain (C register, byte output). The first never depends on
-// the second, so a producer warp runs it over 16-symbol chunks, handing each
-// symbol's (qe added to C | shift << 16) to a consumer warp that runs the C
-// chain, writes the bytes and records numbytes() at every pass end, one
-// chunk behind. All lanes of a chain (the whole warp, or one half-warp when
-// a pair codes two blocks at once) run the same chain on the same values, so
-// their byte stores coincide and only the chain's first lane writes the
-// handoff. Chains pull blocks, heaviest first, from an atomic counter.
-constexpr int kPipes = 4;  // pipelines (warp pairs) per CTA
-constexpr uint32_t kPipeEnd = 0xffffffffu;
-
-struct PipeChunk {
-  uint32_t block;  // code-block, or kPipeEnd
-  uint16_t item;   // item (bit-plane) index within the block
-  uint16_t lo;     // first symbol of the chunk within the item
-  uint32_t count;  // symbols in the chunk, 0..16
-  uint32_t flags;  // 1: first chunk of the block, 2: last of its item, 4: last of the block
-  uint32_t a_end;  // A after the block's last symbol (flags & 4)
-  uint32_t op[16];
-};
-
-// Barrier `id` of one producer/consumer pair (64 threads). With two chains
-// per warp the halves of a warp may arrive apart, so that form uses the
-// barrier that does not require a converged warp.
-template <int H>
-__device__ __forceinline__ void pipe_bar(int id) {
-  if constexpr (H == 1) asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
-  else asm volatile("barrier.sync %0, 64;" ::"r"(id) : "memory");
-}
-
-// State entry with its successors: x = qe | leading zeros of qe << 16 |
-// MPS << 20, y and z the x of the states after an MPS and an LPS
-// renormalisation, w their indices (MPS | LPS << 8).
-__device__ __forceinline__ void load_fat_table(uint4* F) {
-  for (int i = threadIdx.x; i < 94; i += blockDim.x) {
-    auto xs = [](int k) {
-      const uint32_t v = c_tables.mq[k], qe = v & 0xffffu;
-      return qe | ((uint32_t)(__clz(qe) - 16) << 16) | ((uint32_t)(k & 1) << 20);
-    };
-    const uint32_t v = c_tables.mq[i], nm = (v >> 16) & 0xffu, nl = (v >> 24) & 0xffu;
-    F[i] = make_uint4(xs(i), xs((int)nm), xs((int)nl), nm | (nl << 8));
-  }
-}
-
-// Interval/state step of one symbol whose context state index is
-// ci[32 * cx] (the calling lane's own copy of the context states); returns
-// the symbol's C operation (see mq_step for the folded decisions).
-__device__ __forceinline__ uint32_t phase_a_one(uint32_t& A, uint32_t* ci, const uint4* F, uint32_t sym) {
-  const uint32_t cx = sym >> 1, cur = ci[32 * cx];
-  const uint4 f = F[cur];
-  const uint32_t qe = f.x & 0xffffu;
-  const uint32_t lps = ((f.x >> 20) ^ sym) & 1u;
-  const uint32_t a = A - qe;
-  const bool take_a = (a < qe) == (lps != 0);
-  const uint32_t n = take_a ? ((a < 0x4000u ? 1u : 0u) + (a < 0x8000u ? 1u : 0u)) : ((f.x >> 16) & 15u);
-  A = (take_a ? a : qe) << n;
-  ci[32 * cx] = n ? (lps ? (f.w >> 8) : (f.w & 0xffu)) : cur;
-  return (take_a ? qe : 0u) | (n << 16);
-}
-
-// The same over a full chunk: the next state's qe comes from the current
-// entry (no load on the chain), context indices are read two symbols ahead
-// and forwarded when a context repeats.
-__device__ __forceinline__ void phase_a_chunk(uint32_t& A, uint32_t* ci, const uint4* F, const uint4 q,
-                                              uint32_t (&op)[16]) {
-  uint32_t sy[16];
-  #pragma unroll
-  for (int i = 0; i < 16; ++i) sy[i] = chunk_sym(q, i);
-  uint32_t cur = ci[32 * (sy[0] >> 1)];
-  uint4 f = F[cur];
-  uint32_t idx_next = ci[32 * (sy[1] >> 1)];
-  uint4 fl_next = F[idx_next];
-  #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const uint32_t cx = sy[i] >> 1;
-    uint32_t raw2 = 0;
-    if (i + 2 < 16) raw2 = ci[32 * (sy[i + 2] >> 1)];  // before this symbol's update
-    const uint32_t qe = f.x & 0xffffu;
-    const uint32_t lps = ((f.x >> 20) ^ sy[i]) & 1u;
-    const uint32_t a = A - qe;
-    const bool take_a = (a < qe) == (lps != 0);
-    const uint32_t n = take_a ? ((a < 0x4000u ? 1u : 0u) + (a < 0x8000u ? 1u : 0u)) : ((f.x >> 16) & 15u);
-    A = (take_a ? a : qe) << n;
-    op[i] = (take_a ? qe : 0u) | (n << 16);
-    const uint32_t newidx = n ? (lps ? (f.w >> 8) : (f.w & 0xffu)) : cur;
-    const uint32_t newx = n ? (lps ? f.z : f.y) : f.x;
-    ci[32 * cx] = newidx;
-    if (i + 1 < 16) {
-      const uint4 L = F[newidx];
-      const uint32_t cxn = sy[i + 1] >> 1;
-      if (cxn == cx) {
-        f = make_uint4(newx, L.y, L.z, L.w);
-        cur = newidx;
-      } else {
-        f = fl_next;
-        cur = idx_next;
-      }
-      if (i + 2 < 16) {
-        idx_next = (sy[i + 2] >> 1) == cx ? newidx : raw2;
-        fl_next = F[idx_next];
-      }
-    }
-  }
-}
-
-// Code-register step of one symbol's operation (byte output as needed).
-__device__ __forceinline__ void phase_c_one(Mq& m, uint32_t op) {
-  m.c += op & 0xffffu;
-  uint32_t n = op >> 16;
-  if (n >= m.ct) {
-    do {
-      m.c <<= m.ct;
-      n -= m.ct;
-      mq_byteout(m);
-    } while (n >= m.ct);
-  }
-  m.c <<= n;
-  m.ct -= n;
-}
-
-// CTAs below pipe_ctas are pipelines that pull the `heavy` heaviest blocks;
-// the CTAs above code the remaining (lighter) blocks 32 to a warp, one per
-// lane, which costs the schedulers far fewer issue slots per symbol.
-//
-// H chains per warp pair: with H = 2 the two half-warps of each warp run the
-// chains of two different code-blocks in the same instruction stream (each
-// half pulls its own blocks), so a symbol costs about half the issue slots
-// of H = 1 (all 32 lanes on one chain), at the price of executing both
-// halves' byte-output branches. A half with nothing left keeps taking part
-// in the pair's barriers with empty chunks until both halves are done.
-template <int H>
-__global__ void __launch_bounds__(kPipes * 64, 2) t1_mq_pipe_kernel(T1Args a, uint32_t* next, uint32_t pipe_ctas,
-                                                                uint32_t heavy) {
-  constexpr int HL = 32 / H;  // lanes per chain
-  __shared__ uint4 F[94];
-  __shared__ PipeChunk slots[kPipes][2][H];
-  // Context state indices: every lane keeps its own copy (context c of a
-  // lane at [pipe][c][lane]). The lanes of a chain compute identical values,
-  // but a shared copy would be read and written by all of them with nothing
-  // ordering one lane's write after another lane's read of the same symbol;
-  // private copies make the chain correct however the lanes are scheduled.
-  __shared__ uint32_t ci_all[kPipes][19][32];
-  if (blockIdx.x >= pipe_ctas) {
-    __shared__ uint2 T[94];
-    __shared__ uint2 ce_all[kPipes * 2][20 * 32];
-    load_mq_table(T);
-    __syncthreads();
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const uint32_t slot = heavy + ((blockIdx.x - pipe_ctas) * (kPipes * 2) + (uint32_t)w) * 32u + (uint32_t)l;
-    if (slot < a.nblocks) mq_code_block(a, a.mq_order[slot], &ce_all[w][l], T);
-    return;
-  }
-  load_fat_table(F);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int half = lane / HL, hl = lane % HL;  // this lane's chain, its lane within it
-  const uint32_t hmask = H == 1 ? 0xffffffffu : (((1u << HL) - 1u) << (HL * half));
-  // producers are warps 0..kPipes-1 and consumers the warps above, so the
-  // (heavier) producer chains spread over the SM's schedulers
-  const int pipe = warp % kPipes;
-  const int bar = 1 + pipe;
-  if (warp < kPipes) {
-    // ---- producer: interval and state chain ----
-    uint32_t* ci = &ci_all[pipe][0][lane];
-    uint32_t b = kPipeEnd, base = 0, A = 0x8000u;
-    int mbp = 0, j = 0, lo = 0, total = 0;
-    bool exhausted = false;  // the block queue is empty for this chain
-    const uint4* src = nullptr;
-    uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0, c2 = c0;
-    auto start_item = [&]() {
-      const ItemRec r = a.item_rec[base + j];
-      total = (int)(r.n_sp + r.n_mr + r.n_cl);
-      lo = 0;
-      src = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j) * a.sym_slot);
-      c0 = src[0];
-      c1 = src[1];
-      c2 = src[2];  // the slot and the buffer are padded for these reads
-    };
-    for (uint32_t k = 0;; ++k) {
-      PipeChunk& s = slots[pipe][k & 1][half];
-      uint32_t flags = 0;
-      while (b == kPipeEnd && !exhausted) {
-        uint32_t t = 0;
-        if (hl == 0) t = atomicAdd(next, 1u);
-        t = __shfl_sync(hmask, t, half * HL);
-        if (t >= heavy) {
-          exhausted = true;
-          break;
-        }
-        const uint32_t cand = a.mq_order[t];
-        const BlockOut o = a.res[cand];
-        const int m_ = o.status ? 0 : o.mbp;
-        if (m_ == 0) continue;
-        b = cand;
-        mbp = m_;
-        j = 0;
-        base = a.plane_base[b];
-        A = 0x8000u;
-        // contexts: state 0 except UNI 46, AGG 3, ZC 4 (src/mq/mod.rs:195-200)
-        #pragma unroll
-        for (int x = 0; x < 19; ++x) ci[32 * x] = x == kCtxUNI ? 92u : (x == kCtxAGG ? 6u : (x == 0 ? 8u : 0u));
-        flags = 1;
-        start_item();
-      }
-      const bool idle = b == kPipeEnd;
-      if (idle) {
-        if (hl == 0) s.block = kPipeEnd;
-      } else {
-        const int cnt = min(16, total - lo);
-        if (cnt == 16) {
-          const uint4 q = c0;
-          c0 = c1;
-          c1 = c2;
-          c2 = src[(lo >> 4) + 3];  // 48 bytes ahead: inside the slot or the buffer's pad
-          uint32_t op[16];
-          phase_a_chunk(A, ci, F, q, op);
-          if (hl == 0) {
-            #pragma unroll
-            for (int i = 0; i < 16; ++i) s.op[i] = op[i];
-          }
-        } else {
-          const uint4 q = c0;
-          for (int i = 0; i < cnt; ++i) {
-            const uint32_t o = phase_a_one(A, ci, F, chunk_sym(q, i));
-            if (hl == 0) s.op[i] = o;
-          }
-        }
-        if (hl == 0) {
-          s.block = b;
-          s.item = (uint16_t)j;
-          s.lo = (uint16_t)lo;
-          s.count = (uint32_t)cnt;
-        }
-        lo += cnt;
-        if (lo >= total) {
-          flags |= 2;
-          if (++j == mbp) {
-            flags |= 4;
-            if (hl == 0) s.a_end = A;
-            b = kPipeEnd;
-          } else {
-            start_item();
-          }
-        }
-        if (hl == 0) s.flags = flags;
-      }
-      const bool all_idle = __all_sync(0xffffffffu, idle);
-      pipe_bar<H>(bar);
-      if (all_idle) break;
-    }
-  } else {
-    // ---- consumer: code register chain, bytes and pass records ----
-    Mq m{0x8000u, 0u, 12u, 0, 0u, nullptr, 0, 0};
-    BlockOut o{};
-    PassRec* pr = nullptr;
-    ItemRec r{};
-    uint32_t base = 0, nsym = 0;
-    int pi = 0, npass = 1, kp = 0;
-    int end[3] = {0, 0, 0};
-    auto snapshot = [&](int k, int item) {  // numbytes() after pass k
-      const uint8_t bp = (uint8_t)r.bitplane;
-      if (npass == 1 || k == 2)
-        pr[pi] = PassRec{(uint32_t)m.pos, r.ns_cl, item == 0 ? 0u : r.sig_before + r.ns_sp, 2, bp, 0};
-      else if (k == 0)
-        pr[pi] = PassRec{(uint32_t)m.pos, r.ns_sp, r.sig_before, 0, bp, 0};
-      else
-        pr[pi] = PassRec{(uint32_t)m.pos, 0u, r.sig_before, 1, bp, 0};
-      ++pi;
-    };
-    for (uint32_t k = 0;; ++k) {
-      __syncwarp();  // the halves meet before the pair's barrier
-      pipe_bar<H>(bar);
-      const PipeChunk& s = slots[pipe][k & 1][half];
-      const uint32_t blk = s.block;
-      if (__all_sync(0xffffffffu, blk == kPipeEnd)) break;
-      if (blk == kPipeEnd) continue;  // this chain is idle in this round
-      const uint32_t flags = s.flags;
-      const int item = s.item, lo = s.lo, cnt = (int)s.count;
-      if (flags & 1) {
-        const BlockDesc d = a.blocks[blk];
-        o = a.res[blk];
-        m = Mq{0x8000u, 0u, 12u, 0, 0u, a.out + d.out_off, (int)d.out_cap, 0};
-        pr = a.passes + d.pass_off;
-        pi = 0;
-        nsym = 0;
-        base = a.plane_base[blk];
-      }
-      if (lo == 0) {
-        r = a.item_rec[base + item];
-        const int total = (int)(r.n_sp + r.n_mr + r.n_cl);
-        npass = item == 0 ? 1 : 3;
-        end[0] = item == 0 ? total : (int)r.n_sp;
-        end[1] = (int)(r.n_sp + r.n_mr);
-        end[2] = total;
-        nsym += (uint32_t)total;
-        kp = 0;
-        while (kp < npass - 1 && end[kp] == 0) snapshot(kp++, item);
-      }
-      const int hi = lo + cnt;
-      if (cnt == 16 && (kp == npass - 1 || end[kp] >= hi)) {
-        uint32_t op[16];
-        #pragma unroll
-        for (int i = 0; i < 16; ++i) op[i] = s.op[i];
-        #pragma unroll
-        for (int i = 0; i < 16; ++i) phase_c_one(m, op[i]);
-      } else {
-        for (int i = 0; i < cnt; ++i) {
-          phase_c_one(m, s.op[i]);
-          while (kp < npass - 1 && end[kp] == lo + i + 1) snapshot(kp++, item);
-        }
-      }
-      while (kp < npass - 1 && end[kp] == hi) snapshot(kp++, item);
-      if (flags & 2) snapshot(npass == 1 ? 0 : 2, item);
-      if (flags & 4) {
-        m.a = s.a_end;
-        mq_flush(m);
-        o.payload_len = (uint32_t)(m.last == 0xffu ? m.pos - 1 : m.pos);  // take_bytes
-        o.status = m.ovf ? 1 : 0;
-        if (hl == 0) {
-          a.res[blk] = o;
-          atomicAdd(a.sym_count, (unsigned long long)nsym);
-        }
-      }
-    }
-  }
-}
-
-// Static mapping: warp w codes blocks order[w * bpw + lane], lanes < bpw.
+// Warp w codes blocks order[w * bpw + lane], lanes < bpw.
 __global__ void __launch_bounds__(kMqWarps * 32) t1_mq_kernel(T1Args a, int bpw) {
-  __shared__ uint2 T[94];
-  __shared__ uint2 ce_all[kMqWarps][20 * 32];
-  load_mq_table(T);
+  __shared__ MqSmem sm;
+  load_mq_table(sm.table);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
-  if (lane >= bpw) return;
   const uint32_t slot = (blockIdx.x * kMqWarps + wid) * (uint32_t)bpw + (uint32_t)lane;
-  if (slot >= a.nblocks) return;
-  mq_code_block(a, a.mq_order ? a.mq_order[slot] : slot, &ce_all[wid][lane], T);
-}
-
-// Persistent form for one block per warp: a fixed number of warps per SM
-// take the next block of the order (heaviest first) until none is left, so
-// the longest chains start first and share their schedulers with few others.
-__global__ void __launch_bounds__(kMqWarps * 32) t1_mq_pull_kernel(T1Args a, uint32_t* next) {
-  __shared__ uint2 T[94];
-  __shared__ uint2 ce_all[kMqWarps][20 * 32];
-  load_mq_table(T);
-  __syncthreads();
-  if ((threadIdx.x & 31) != 0) return;
-  uint2* ce = &ce_all[threadIdx.x >> 5][0];
-  for (;;) {
-    const uint32_t slot = atomicAdd(next, 1u);
-    if (slot >= a.nblocks) return;
-    mq_code_block(a, a.mq_order[slot], ce, T);
-  }
+  mq_code_block(a, lane < bpw && slot < a.nblocks ? a.mq_order[slot] : kNoBlock, sm);
 }
 
 }  // namespace
@@ -1144,17 +873,13 @@ void launch_t1_model(const T1Args& a, int num_sms, cudaStream_t st) {
   t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a);
 }
 
+// Automatic: as few blocks per warp as keep at most one warp on each of
+// the SMs' four schedulers (a warp's lanes cost nothing, and a second warp on
+// a scheduler lengthens both warps' chains), up to 32.
 int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw) {
-  // Automatic: up to 48 blocks per SM, one block per chain (the caller
-  // pulls or pipelines them); beyond that, as few blocks per warp (at least
-  // 2) as keep about 24 latency-bound warps per SM, since the lanes of a
-  // warp diverge.
-  if (bpw <= 0 || bpw > 32) {
-    const uint32_t sms = (uint32_t)num_sms;
-    if (a.nblocks <= sms * 48u) return 1;
-    bpw = (int)std::min<uint32_t>(32u, std::max<uint32_t>(2u, (a.nblocks + sms * 24u - 1) / (sms * 24u)));
-  }
-  return bpw;
+  if (bpw >= 1 && bpw <= 32) return bpw;
+  const uint32_t warps = (uint32_t)num_sms * 4u;
+  return (int)std::min<uint32_t>(32u, std::max<uint32_t>(1u, (a.nblocks + warps - 1) / warps));
 }
 
 void launch_t1_mq(const T1Args& a, int num_sms, int bpw, cudaStream_t st) {
@@ -1162,34 +887,6 @@ void launch_t1_mq(const T1Args& a, int num_sms, int bpw, cudaStream_t st) {
   bpw = mq_blocks_per_warp(a, num_sms, bpw);
   const uint32_t per_cta = (uint32_t)bpw * kMqWarps;
   t1_mq_kernel<<<(a.nblocks + per_cta - 1) / per_cta, kMqWarps * 32, 0, st>>>(a, bpw);
-}
-
-void launch_t1_mq_pipe(const T1Args& a, int num_sms, int pipes_per_sm, int chains, uint32_t heavy, uint32_t* next,
-                       cudaStream_t st) {
-  if (a.nblocks == 0) return;
-  cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
-  heavy = heavy == 0 ? a.nblocks : std::min(heavy, a.nblocks);
-  chains = chains == 2 || chains == 4 ? chains : 1;
-  const uint32_t per_pipe_cta = (uint32_t)kPipes * (uint32_t)chains;  // blocks a CTA codes at once
-  const uint32_t pipe_ctas = std::max<uint32_t>(
-      1u, std::min<uint32_t>((uint32_t)num_sms * (uint32_t)pipes_per_sm / kPipes,
-                             (heavy + per_pipe_cta - 1) / per_pipe_cta));
-  const uint32_t per_cta = kPipes * 2 * 32;
-  const uint32_t packed_ctas = (a.nblocks - heavy + per_cta - 1) / per_cta;
-  if (chains == 4)
-    t1_mq_pipe_kernel<4><<<pipe_ctas + packed_ctas, kPipes * 64, 0, st>>>(a, next, pipe_ctas, heavy);
-  else if (chains == 2)
-    t1_mq_pipe_kernel<2><<<pipe_ctas + packed_ctas, kPipes * 64, 0, st>>>(a, next, pipe_ctas, heavy);
-  else
-    t1_mq_pipe_kernel<1><<<pipe_ctas + packed_ctas, kPipes * 64, 0, st>>>(a, next, pipe_ctas, heavy);
-}
-
-void launch_t1_mq_pull(const T1Args& a, int num_sms, int warps_per_sm, uint32_t* next, cudaStream_t st) {
-  if (a.nblocks == 0) return;
-  cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
-  const uint32_t ctas = std::min<uint32_t>((uint32_t)num_sms * (uint32_t)warps_per_sm / kMqWarps,
-                                           (a.nblocks + kMqWarps - 1) / kMqWarps);
-  t1_mq_pull_kernel<<<std::max<uint32_t>(ctas, 1u), kMqWarps * 32, 0, st>>>(a, next);
 }
 
 namespace {
