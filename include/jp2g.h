@@ -235,7 +235,8 @@ int jp2g_set_timing(jp2g_ctx* ctx, int enabled);
 int jp2g_stage_times(jp2g_ctx* ctx, float* ms, int n);
 
 /* Work counters of the last encode (or batch): [0] code-blocks,
- * [1] non-empty blocks, [2] coding passes, [3] payload bytes before rate
+ * [1] non-empty blocks, [2] passes coded, [3] payload bytes coded (a block is
+ * coded as far as rate control can choose its passes) before rate
  * control, [4] bytes retained, [5] kernel launches, [6] coefficient
  * bit-planes (sum over blocks of coefficients x magnitude bit-planes),
  * [7] MQ symbols coded. */

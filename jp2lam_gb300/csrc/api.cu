@@ -269,6 +269,7 @@ void build_tables(const PagePlan& p, uint32_t block_base, uint32_t band_base, ui
       bp.band_bias = q.orient == LL ? 1.20 : (q.orient == HH ? 0.82 : 1.00);
     }
     bp.is_ll = q.orient == LL;
+    bp.unit = (float)(bp.subband_weight * bp.band_bias * bp.quant_step * bp.quant_step);
     bands->push_back(bp);
   }
   for (int c = 0; c < p.ncomp; ++c) {
@@ -278,6 +279,9 @@ void build_tables(const PagePlan& p, uint32_t block_base, uint32_t band_base, ui
     cp.comp_weight = p.comp_weight[c];
     cp.lossless = p.quality >= 100;
     cp.quality = p.quality;
+    cp.lambda = (float)std::min(p.lambda_raw, 1e30);
+    cp.weight = (float)p.comp_weight[c];
+    cp.settled = (float)(p.lambda_floor / 1.2 * (1.0 + 1e-5));
     comps->push_back(cp);
   }
 }
@@ -803,7 +807,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
       !reserve(c, c->blocks, std::max<size_t>(nb, 1) * sizeof(BlockDesc)) ||
       !reserve(c, c->bands, bands.size() * sizeof(BandParam)) ||
       !reserve(c, c->comps, comps.size() * sizeof(CompParam)) ||
-      !reserve(c, c->maxslope, std::max<size_t>(comps.size(), 8) * sizeof(unsigned long long)) ||
+      !reserve(c, c->maxslope, std::max<size_t>(comps.size(), 8) * (sizeof(unsigned long long) + sizeof(uint32_t))) ||
       !reserve(c, c->hullp, std::max<size_t>(nb, 1) * pcap * sizeof(uint16_t)) ||
       !reserve(c, c->hulls, std::max<size_t>(nb, 1) * pcap * sizeof(double)) ||
       !reserve(c, c->hulln, std::max<size_t>(nb, 1)) ||
@@ -874,7 +878,13 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   ta.plane_base = dptr<uint32_t>(c->planebase);
   ta.sym_slot = (uint32_t)(((slot * 5 / 2 + 15) & ~size_t(15)) + 48);  // each pass padded to 16 symbols
   ta.sym_count = dptr<unsigned long long>(c->stats);
-  if (!cuda_ok(c, cudaMemsetAsync(c->stats.p, 0, 8, c->stream), "memset")) return kEncodeFailed;
+  ta.bands = dptr<BandParam>(c->bands);
+  ta.comps = dptr<CompParam>(c->comps);
+  // the inspection entry points see every pass of every block
+  ta.settled = dbg ? nullptr : reinterpret_cast<uint32_t*>(dptr<unsigned long long>(c->maxslope) + comps.size());
+  if (!cuda_ok(c, cudaMemsetAsync(c->stats.p, 0, 8, c->stream), "memset") ||
+      (ta.settled && !cuda_ok(c, cudaMemsetAsync(ta.settled, 0, comps.size() * 4, c->stream), "memset")))
+    return kEncodeFailed;
   launch_t1_analyze(ta, c->stream);
   launch_scan_u32(ta.nplanes, 1, nb, ta.plane_base, dptr<uint32_t>(c->scratch), c->stream);
   // the number of (block, bit-plane) items sizes the symbol buffer

@@ -110,7 +110,7 @@ struct ItemRec {
   uint32_t ns_sp, ns_cl;
   uint32_t sig_before;
   uint32_t bitplane;
-  uint32_t pad;
+  float remain;  // upper bound of the distortion removed by the block's bit-planes below this one
 };
 
 // Tier-1 per-block result.
@@ -140,7 +140,7 @@ struct BandParam {
   double subband_weight;  // norm97^2
   double band_bias;
   uint32_t is_ll;
-  uint32_t pad;
+  float unit;  // distortion of one significant sample at bit-plane 0, without block and component weights
 };
 
 // PCRD constants per (page, component).
@@ -150,6 +150,10 @@ struct CompParam {
   double comp_weight;
   uint32_t lossless;  // PCRD skipped when quality >= 100
   int32_t quality;
+  // for stopping a block's coding early (t1_mq_kernel)
+  float lambda, weight;  // lambda_raw and comp_weight
+  float settled;         // a block slope that makes lambda_raw the component's lambda
+  uint32_t pad;
 };
 
 }  // namespace jp2g

@@ -68,7 +68,12 @@ struct T1Args {
   uint8_t* sym;          // per item: a slot of sym_slot symbol bytes
   uint32_t sym_slot;
   unsigned long long* sym_count;  // total MQ symbols coded (statistics)
-  const uint32_t* mq_order;       // MQ processing order of the blocks, or null (work-list order)
+  const uint32_t* mq_order;       // MQ processing order of the blocks
+  const BandParam* bands;
+  const CompParam* comps;
+  // per component key, zeroed: 1 once a block has shown a slope that settles
+  // the component's lambda; null: code every pass of every block
+  uint32_t* settled;
 };
 
 void launch_t1_analyze(const T1Args& a, cudaStream_t st);

@@ -52,3 +52,42 @@ def test_lanes_of_a_warp_do_not_disturb_each_other(eng, orc, bpw):
             assert eng.encode(px, w, h, 1, q, 1) == orc.encode(px, w, h, 1, q, 1)
     finally:
         eng.set_option(_native.OPT_MQ_BLOCKS_PER_WARP, 0)
+
+
+def _stop_content(kind, w, h, c):
+    rng = np.random.default_rng(w + 7 * h + 31 * c)
+    y, x = np.mgrid[0:h, 0:w]
+    if kind == "faint":  # slopes too small to settle lambda: every pass is coded
+        px = 128 + rng.integers(0, 2, (h, w, c))
+    elif kind == "outlier":  # one huge coefficient above much small detail
+        px = 120 + rng.integers(-6, 7, (h, w, c))
+        px[h // 2, w // 2] = 255
+        px[h // 3:h // 3 + 2, w // 5] = 0
+    elif kind == "texture":
+        px = 128 + 60 * np.sin(x / 3.1)[..., None] * np.cos(y / 4.7)[..., None] + rng.normal(0, 12, (h, w, c))
+    else:  # chroma much fainter than luma
+        g = np.where((x // 9 + y // 7) % 2, 230, 20)[..., None]
+        px = g + rng.integers(0, 3, (h, w, c))
+    return np.ascontiguousarray(np.clip(px, 0, 255).astype(np.uint8))
+
+
+@pytest.mark.parametrize("kind", ["faint", "outlier", "texture", "checks"])
+@pytest.mark.parametrize("w,h,c", [(64, 64, 1), (200, 150, 3), (321, 257, 1)])
+def test_blocks_stopped_early_lose_nothing(eng, orc, kind, w, h, c):
+    # lossy codestreams of blocks whose coding stops at some bit-plane, over
+    # the whole range of lambda, byte for byte
+    px = _stop_content(kind, w, h, c)
+    for q in (0, 1, 5, 15, 29, 30, 45, 50, 70, 85, 92, 98, 99):
+        assert eng.encode(px, w, h, c, q, 0) == orc.encode(px, w, h, c, q, 0), q
+
+
+def test_block_inspection_shows_every_pass(eng, orc):
+    # jp2g_debug_blocks reports complete coding, an encode only what it needed
+    w, h = 256, 256
+    px = _stop_content("texture", w, h, 1)
+    rows = eng.debug_blocks(px, w, h, 1, 60)
+    coded = rows[:, 0] > 0
+    assert np.array_equal(rows[coded, 2], 1 + 3 * (rows[coded, 0] - 1))
+    full = eng.counters()[2]
+    eng.encode(px, w, h, 1, 60, 0)
+    assert 0 < eng.counters()[2] < full
