@@ -1391,8 +1391,11 @@ struct DecodePage {
 };
 
 uint64_t decode_device_bytes(const DecodePage& p, size_t nbytes) {
-  // bytes, planes, tmp planes, samples, code-blocks, jobs
-  return nbytes + p.npx * p.L.ncomp * 9 + p.L.blocks.size() * sizeof(DecBlock) +
+  // bytes, planes, tmp planes or masks, samples, code-blocks, jobs
+  uint64_t masks = 0;
+  for (const DecBlock& b : p.L.blocks) masks += 8ull * dec_mask_words(b.npasses);
+  return nbytes + p.npx * p.L.ncomp * 5 + std::max<uint64_t>(p.npx * p.L.ncomp * 4, masks) +
+         p.L.blocks.size() * sizeof(DecBlock) +
          (uint64_t)(p.L.levels * p.L.ncomp + 1) * sizeof(IdwtJob) + sizeof(PixJob) + 1024;
 }
 
@@ -1416,19 +1419,26 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   // device job tables: blocks, then per-level inverse-DWT jobs, then pixel jobs
   std::vector<DecBlock> blk;
   blk.reserve(nblk);
+  uint64_t mask_words = 0;
   for (size_t i : ids)
     for (DecBlock b : pg[i].L.blocks) {
       b.plane_off += pg[i].plane_base;
       b.data_off += (uint32_t)pg[i].data_base;
+      b.mask_off = mask_words;
+      mask_words += dec_mask_words(b.npasses);
       blk.push_back(b);
     }
-  const size_t planes_bytes = (size_t)nplane * 4;
+  // the blocks' masks lie where the inverse DWT's scratch planes come later
+  const size_t planes_bytes = ((size_t)nplane * 4 + 15) & ~size_t(15);
+  const size_t tmp_bytes = std::max<size_t>(planes_bytes, mask_words * 8);
+  // and the blocks' order where the samples do
+  const size_t px_bytes = std::max<size_t>((size_t)npxb, (blk.size() + 2048) * 4);
   if (!reserve(c, c->t2out, std::max<uint64_t>(nbytes, 16)) ||
-      !reserve(c, c->recon, planes_bytes * 2 + (size_t)npxb + 256))
+      !reserve(c, c->recon, planes_bytes + tmp_bytes + px_bytes + 256))
     return JP2G_DECODE_FAILED;
   int32_t* planes = dptr<int32_t>(c->recon);
-  int32_t* tmp = planes + nplane;
-  uint8_t* dpx = reinterpret_cast<uint8_t*>(tmp + nplane);
+  int32_t* tmp = reinterpret_cast<int32_t*>(dptr<uint8_t>(c->recon) + planes_bytes);
+  uint8_t* dpx = reinterpret_cast<uint8_t*>(tmp) + tmp_bytes;
   std::vector<IdwtJob> jobs;
   std::vector<uint32_t> first(maxl + 2, 0), rows(maxl + 2, 0), tiles(maxl + 2, 0);
   for (int l = 1; l <= maxl; ++l) {
@@ -1486,15 +1496,10 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
       (!jobs.empty() && !cuda_ok(c, cudaMemcpyAsync(djobs, jobs.data(), jobs.size() * sizeof(IdwtJob),
                                                     cudaMemcpyHostToDevice, c->stream), "H2D jobs")) ||
       !cuda_ok(c, cudaMemcpyAsync(dpix, pix.data(), pix.size() * sizeof(PixJob), cudaMemcpyHostToDevice, c->stream),
-               "H2D pages") ||
-      !cuda_ok(c, cudaMemsetAsync(planes, 0, planes_bytes, c->stream), "memset planes"))
+               "H2D pages"))
     return JP2G_DECODE_FAILED;
-  // two decoders per warp once the blocks fill the warps the SMs hold at
-  // once (16 per SM) four times over: more chains in flight for batches
-  // (64 sRGB 2550x3300 files: 290 -> 251 ms end to end); one otherwise, so
-  // a file's heaviest chains run alone (one sRGB file: 10.0 against 13.4 ms)
-  const int per_warp = blk.size() > (size_t)c->num_sms * 64u ? 2 : 1;
-  launch_t1_decode(dblk, (uint32_t)blk.size(), dptr<uint8_t>(c->t2out), planes, per_warp, c->stream);
+  launch_t1_decode(dblk, (uint32_t)blk.size(), dptr<uint8_t>(c->t2out), reinterpret_cast<unsigned long long*>(tmp),
+                   planes, reinterpret_cast<uint32_t*>(dpx), c->stream);
   for (int l = 1; l <= maxl; ++l) launch_idwt_level(djobs + first[l], first[l + 1] - first[l], rows[l], tiles[l], c->stream);
   launch_dec_pixels(dpix, (uint32_t)pix.size(), total_px, c->stream);
   if (!cuda_ok(c, cudaGetLastError(), "decode kernels")) return JP2G_DECODE_FAILED;

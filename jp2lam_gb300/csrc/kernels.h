@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "jp2g_internal.h"
+#include "t1_logic.h"
 
 namespace jp2g {
 
@@ -164,6 +165,7 @@ void launch_t2(const T2Args& a, uint32_t* scan_scratch, int num_sms, cudaStream_
 // One code-block of a codestream being decoded.
 struct DecBlock {
   uint64_t plane_off;           // its first sample in the planes buffer (elements)
+  uint64_t mask_off;            // its masks (64-bit words): 64 columns per decoded bit-plane, then its signs
   uint32_t data_off, data_len;  // its segment in the input bytes
   uint32_t stride;              // its plane's row pitch (the image width)
   uint16_t w, h;
@@ -207,10 +209,14 @@ struct PixJob {
   uint64_t npx, pix_base;  // pix_base: the page's first global sample index
   uint32_t ncomp, mct, reversible, pad;
 };
-// Tier-1 decoding of every code-block (t1dec.cu) into zeroed planes, one
-// or two (per_warp) decoders per warp.
-void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, int32_t* planes, int per_warp,
-                      cudaStream_t st);
+// Bit-planes that a block's passes reach: its top one in one pass, then three each.
+JP2G_HD uint32_t dec_planes(uint32_t npasses) { return npasses ? (npasses + 4) / 3 : 0; }
+// 64-bit words of a block's masks.
+JP2G_HD uint32_t dec_mask_words(uint32_t npasses) { return npasses ? 64 * (dec_planes(npasses) + 1) : 0; }
+// Tier-1 decoding of every code-block into coefficients (t1dec.cu). masks: the
+// blocks' masks; scratch: nblocks + 2048 words.
+void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, unsigned long long* masks,
+                      int32_t* planes, uint32_t* scratch, cudaStream_t st);
 // One inverse-DWT level for njobs jobs (recon.cu).
 void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_rows, uint32_t total_tiles,
                        cudaStream_t st);

@@ -91,22 +91,6 @@ __global__ void t1_analyze_kernel(T1Args a) {
   a.nplanes[warp] = o.status ? 0u : (uint32_t)mbp;
 }
 
-// 32x32 bit-matrix transpose in registers: on entry bit j of t[i] is
-// element (i, j); on exit bit i of t[j] is.
-__device__ __forceinline__ void transpose32(uint32_t (&t)[32]) {
-  #pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const uint32_t m = s == 16 ? 0x0000ffffu : (s == 8 ? 0x00ff00ffu : (s == 4 ? 0x0f0f0f0fu : (s == 2 ? 0x33333333u : 0x55555555u)));
-    #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      if (i & s) continue;
-      const uint32_t x = ((t[i] >> s) ^ t[i + s]) & m;
-      t[i] ^= x << s;
-      t[i + s] ^= x;
-    }
-  }
-}
-
 // Distortion of one significant sample of a block at bit-plane 0: the
 // weights of pcrd_hull_kernel in f32.
 __device__ __forceinline__ float block_unit(const T1Args& a, uint32_t b, const BlockDesc& d) {

@@ -88,4 +88,22 @@ JP2G_HD void sign_planes(M n, M s, M w, M e, M gn, M gs, M gw, M ge, M* m, M* x)
   *x = hneg | (hz & vneg);
 }
 
+#ifdef __CUDACC__
+// 32x32 bit-matrix transpose in registers: on entry bit j of t[i] is
+// element (i, j); on exit bit i of t[j] is.
+__device__ __forceinline__ void transpose32(uint32_t (&t)[32]) {
+  #pragma unroll
+  for (int s = 16; s >= 1; s >>= 1) {
+    const uint32_t m = s == 16 ? 0x0000ffffu : (s == 8 ? 0x00ff00ffu : (s == 4 ? 0x0f0f0f0fu : (s == 2 ? 0x33333333u : 0x55555555u)));
+    #pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if (i & s) continue;
+      const uint32_t x = ((t[i] >> s) ^ t[i + s]) & m;
+      t[i] ^= x << s;
+      t[i + s] ^= x;
+    }
+  }
+}
+#endif
+
 }  // namespace jp2g

@@ -3,38 +3,32 @@
 // the MQ decoder of src/mq/mod.rs; the context rules of src/tier1/*).
 //
 // Decoding is sequential within a code-block (every decoded bit changes the
-// contexts of the samples after it), so one lane of a warp runs a block's
-// decoder while the warp's other lanes wait; a CTA holds 8 such warps.
-//  - State: significance, sign, visited and refined flags as 64-bit row
-//    masks in shared memory (a row per mask, zero rows above and below).
-//    A stripe's rows (4, plus the rows above and below for significance and
-//    sign) are held in registers while the stripe is coded, so a sample's
-//    neighbourhood is a few shifts.
-//  - Skipping: each pass visits only the columns of a stripe that can hold
-//    a decision: significance propagation the columns with an insignificant
-//    sample next to a significant one (recomputed when a decision makes a
-//    sample significant), refinement the columns with a significant
-//    unvisited sample, cleanup the columns with an unvisited insignificant
-//    one. Samples are still decided in the standard's scan order.
-//  - Magnitudes: the decoded bits of a bit-plane are gathered as row masks;
-//    after each bit-plane the whole warp ORs them into the component plane
-//    (lane l owns columns l and l + 32). At the end it writes the block's
-//    signed coefficients (reversible codestreams) or their midpoint
-//    dequantised values (irreversible: sign * (|q| + 0.5) * step,
-//    src/simd/scalar.rs:122-129) in place.
+// contexts of the samples after it). A warp decodes a block, every lane in
+// the same control flow, so that what a symbol needs is spread over the
+// lanes' registers and reached by shuffles:
+//  - lane L owns columns L and L + 32 of the block (64-bit masks, bit y =
+//    row y: significant, sign, visited, refined) and prepares, for 32
+//    columns of a stripe at once, which of their samples the pass may code
+//    and from which neighbourhood;
+//  - lane c < 19 holds context c of the coder and its state's successors;
+//  - the interval and code registers are the same in all lanes.
+// What remains per symbol is one chain: context (a table lookup in shared
+// memory), its state (a shuffle), the decision.
+// The decoded bits go out as masks per bit-plane, and a second kernel turns
+// a block's masks into coefficients (t1_coefficients_kernel).
 #include <cuda_runtime.h>
 
 #include <cstring>
 
 #include "jp2g_internal.h"
 #include "kernels.h"
+#include "t1_logic.h"
 
 namespace jp2g {
 
 namespace {
 
-constexpr int kDecWarps = 8;
-constexpr int kCtxZC0 = 0, kCtxMR = 14, kCtxAGG = 17, kCtxUNI = 18;
+constexpr uint32_t kCtxZC0 = 0, kCtxAGG = 17, kCtxUNI = 18;
 
 struct DecTables {
   uint8_t zc[4 * 512];
@@ -44,374 +38,409 @@ struct DecTables {
 };
 __constant__ DecTables c_dec;
 
-struct WarpState {
-  uint64_t sig[66], sgn[66], vis[66], ref[66];  // row y at y + 1
-  uint64_t bits[64];                             // the current bit-plane's decoded 1 bits
-  uint8_t ctx[20];
-};
+constexpr int kDecWarps = 4;
+constexpr uint32_t kDecStates = 94;
 
-// The MQ decoder (ISO/IEC 15444-1 C.3; src/mq/mod.rs): bytes beyond the
-// segment read as 0xFF.
-struct MqDecoder {
+// Context word: Qe << 16 | state << 3 | MPS. The table holds per state (state,
+// MPS pair) the words after an MPS and an LPS renormalisation.
+struct DecShared {
+  uint2 next[kDecStates];
+  uint8_t zc[4][512];  // zero-coding context by neighbourhood (neighbour_index)
+  uint8_t sc[256];     // sign context | prediction bit << 7 (cross_index)
+};
+__device__ __forceinline__ uint32_t dec_word(uint32_t state) {
+  return (c_dec.mq[state] & 0xffffu) << 16 | state << 3 | (state & 1u);
+}
+// The tables in the layouts used here, from those of c_dec (src/tier1/
+// consts.rs: zero coding bit 0 NW, 1 N, 2 NE, 3 W, 5 E, 6 SW, 7 S, 8 SE; sign
+// coding bit 3 W, 0 W negative, 1 N, 4 N negative, 5 E, 2 E negative, 7 S, 6 S
+// negative).
+__device__ __forceinline__ void load_dec_shared(DecShared& sh) {
+  for (uint32_t i = threadIdx.x; i < kDecStates; i += blockDim.x)
+    sh.next[i] = make_uint2(dec_word((c_dec.mq[i] >> 16) & 0xffu), dec_word(c_dec.mq[i] >> 24));
+  for (uint32_t i = threadIdx.x; i < 4 * 512; i += blockDim.x) {
+    const uint32_t f = i & 511u;
+    const uint32_t g = (f & 1u) | (f >> 3 & 1u) << 1 | (f >> 6 & 1u) << 2 | (f >> 1 & 1u) << 3 | (f >> 7 & 1u) << 5 |
+                       (f >> 2 & 1u) << 6 | (f >> 5 & 1u) << 7 | (f >> 8 & 1u) << 8;
+    sh.zc[i >> 9][f] = c_dec.zc[(i & ~511u) | g];
+  }
+  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
+    const uint32_t s = i & 15u, g = i >> 4;  // W, N, E, S
+    const uint32_t lu = (s & 1u) << 3 | (s & g & 1u) | (s >> 1 & 1u) << 1 | ((s & g) >> 1 & 1u) << 4 |
+                        (s >> 2 & 1u) << 5 | ((s & g) >> 2 & 1u) << 2 | (s >> 3 & 1u) << 7 | ((s & g) >> 3 & 1u) << 6;
+    sh.sc[i] = (uint8_t)(c_dec.sc[lu] | c_dec.spb[lu] << 7);
+  }
+}
+
+// Six rows of a column of a stripe (bits 1..4 the stripe's, 0 and 5 the rows
+// above and below it) beside its two neighbours': bits 0..5 the column to
+// the west, 11..16 the column, 22..27 the one to the east (the spacing lets
+// two shifts gather three bits of each).
+__device__ __forceinline__ uint32_t window(uint32_t west, uint32_t own, uint32_t east) {
+  return west | own << 11 | east << 22;
+}
+__device__ __forceinline__ uint32_t own_rows(uint32_t win) { return (win >> 12) & 0xfu; }
+// Neighbourhood of row r: bits NW, W, SW, N, (itself), S, NE, E, SE.
+__device__ __forceinline__ uint32_t neighbour_index(uint32_t win, int r) {
+  const uint32_t t = (win >> r) & 0x01c03807u;
+  return (t | t >> 8 | t >> 16) & 0x1ffu;
+}
+// The four direct neighbours of row r: bits W, N, E, S.
+__device__ __forceinline__ uint32_t cross_index(uint32_t win, int r) {
+  const uint32_t t = (win >> r) & 0x00802802u;
+  return ((t | t >> 9 | t >> 20) >> 1) & 0xfu;
+}
+// Rows of the column with a significant neighbour.
+__device__ __forceinline__ uint32_t rows_near(uint32_t win) {
+  const uint32_t s = (win | win >> 22) & 0x3fu, m = (win >> 11) & 0x3fu;
+  return ((s | s << 1 | s >> 1 | m << 1 | m >> 1) >> 1) & 0xfu;
+}
+
+constexpr uint32_t kAll = 0xffffffffu;
+
+// One of a lane's two columns.
+struct Column {
+  unsigned long long sig, sgn, vis, ref;
+  unsigned long long ones;  // the bit-plane's decoded 1 bits
+};
+// Rows 4 k - 1 .. 4 k + 4 of a mask.
+__device__ __forceinline__ uint32_t six_rows(unsigned long long v, int k) {
+  return (uint32_t)(k > 0 ? v >> (4 * k - 1) : v << 1) & 0x3fu;
+}
+__device__ __forceinline__ uint32_t four_rows(unsigned long long v, int k) { return (uint32_t)(v >> (4 * k)) & 0xfu; }
+
+struct BlockDecoder {
+  const DecShared& sh;
+  const uint8_t* zc;
+  uint8_t* list;  // of the warp, in shared memory
+  uint32_t lane;
+  int w, h;
+  // the MQ decoder (ISO/IEC 15444-1 C.3; src/mq/mod.rs:38-160), the same in
+  // all lanes: C as it is, A << 16; cur and nxt are the segment's bytes bp and
+  // bp + 1, 0xFF beyond its end
   const uint8_t* b;
-  uint32_t n, bp;
-  uint32_t a, c, ct;
-  uint8_t* ctx;
-  __device__ uint32_t at(uint32_t i) const { return i < n ? b[i] : 0xffu; }
-  __device__ void bytein() {
-    const uint32_t next = at(bp + 1);
-    if (at(bp) == 0xffu) {
-      if (next > 0x8fu) {
-        c += 0xff00u;
-        ct = 8;
-      } else {
-        ++bp;
-        c += next << 9;
-        ct = 7;
-      }
-    } else {
-      ++bp;
-      c += next << 8;
+  uint32_t n, bp, cur, nxt, a, c;
+  int ct;
+  uint32_t word, mps_next, lps_next;  // this lane's context, and its successors
+  Column col[2];
+
+  __device__ __forceinline__ uint32_t at(uint32_t i) const { return i < n ? b[i] : 0xffu; }
+  __device__ __forceinline__ void bytein() {
+    if (cur == 0xffu && nxt > 0x8fu) {
+      c += 0xff00u;
       ct = 8;
+    } else {
+      c += cur == 0xffu ? nxt << 9 : nxt << 8;
+      ct = cur == 0xffu ? 7 : 8;
+      ++bp;
+      cur = nxt;
+      nxt = at(bp + 1);
     }
   }
-  __device__ void init(const uint8_t* data, uint32_t len, uint8_t* contexts) {
+  __device__ __forceinline__ void start(const uint8_t* data, uint32_t len) {
+    // initial context states (src/mq/mod.rs:195-200)
+    const uint32_t st = lane == kCtxUNI ? 92u : lane == kCtxAGG ? 6u : lane == kCtxZC0 ? 8u : 0u;
+    word = dec_word(st);
+    mps_next = sh.next[st].x;
+    lps_next = sh.next[st].y;
     b = data;
     n = len;
     bp = 0;
-    ctx = contexts;
-    c = n == 0 ? (0xffu << 16) : ((uint32_t)b[0] << 16);
-    ct = 0;
+    cur = at(0);
+    nxt = at(1);
+    c = cur << 16;
     bytein();
     c <<= 7;
-    ct = ct >= 7 ? ct - 7 : 0;
-    a = 0x8000u;
+    ct -= 7;
+    a = 0x80000000u;
   }
-  __device__ __forceinline__ uint32_t decode(int cx) {
-    const uint32_t st = ctx[cx], e = c_dec.mq[st];
-    const uint32_t qe = e & 0xffffu, mps = st & 1u;
-    uint32_t bit;
-    a -= qe;
-    if ((c >> 16) < qe) {
-      const bool mps_path = a < qe;
-      a = qe;
-      ctx[cx] = (uint8_t)(mps_path ? (e >> 16) & 0xffu : e >> 24);
-      bit = mps_path ? mps : mps ^ 1u;
-    } else {
-      c -= qe << 16;
-      if ((a & 0x8000u) == 0) {
-        const bool lps_path = a < qe;
-        ctx[cx] = (uint8_t)(lps_path ? e >> 24 : (e >> 16) & 0xffu);
-        bit = lps_path ? mps ^ 1u : mps;
-      } else {
-        return mps;
-      }
+  // After A -= Qe the coder takes Qe when C lies below it, else A (and takes
+  // Qe off C); the decision is the LPS when that differs from A < Qe, and the
+  // context moves on when the result is renormalised.
+  __device__ __forceinline__ bool decode(uint32_t cx) {
+    const uint32_t e = __shfl_sync(kAll, word, (int)cx);
+    const uint32_t qe = e & 0xffff0000u;
+    const uint32_t d = a - qe;
+    const bool low = c < qe;
+    const bool lps = low != (d < qe);
+    if ((low || (int)d >= 0) && lane == cx) {
+      word = lps ? lps_next : mps_next;
+      const uint2 t = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(sh.next) + (word & 0x3f8u));
+      mps_next = t.x;
+      lps_next = t.y;
     }
-    // renormalise: shift until a >= 0x8000, reading a byte whenever the bit
-    // count runs out first (the one-bit-at-a-time loop of C.3.3, in runs)
-    uint32_t n = (uint32_t)__clz(a) - 16u;  // 0 < a < 0x8000 here
-    while (n > ct) {
-      a <<= ct;
+    const uint32_t v = low ? qe : d;
+    if (!low) c -= qe;
+    int k = __clz((int)v);
+    a = v << k;
+    while (k > ct) {
       c <<= ct;
-      n -= ct;
-      ct = 0;
+      k -= ct;
       bytein();
     }
-    a <<= n;
-    c <<= n;
-    ct -= n;
-    return bit;
+    c <<= k;
+    ct -= k;
+    return ((e & 1u) != 0) != lps;
   }
-};
 
-// Bits x-1, x, x+1 of a row mask (bit 0 = column x - 1).
-__device__ __forceinline__ uint32_t win3(uint64_t row, int x) {
-  return (uint32_t)(x == 0 ? row << 1 : row >> (x - 1)) & 7u;
-}
-__device__ __forceinline__ uint64_t spread(uint64_t m) { return m | (m << 1) | (m >> 1); }
-__device__ __forceinline__ uint64_t above(int x) { return x >= 63 ? 0ull : ~0ull << (x + 1); }
-
-// One stripe's state while it is coded: S/G rows k-1 .. k+4, V/R rows k .. k+3,
-// B the stripe's decoded 1 bits of the current bit-plane.
-struct Stripe {
-  uint64_t S[6], G[6], V[4], R[4], B[4];
-};
-
-struct BlockDecoder {
-  WarpState& s;
-  MqDecoder mq;
-  const uint8_t* zc;
-  uint64_t wmask;
-
-  // A pass loads (and writes back) only the masks it uses: significance
-  // and visited always, signs for the passes that decode signs, refined for
-  // the refinement pass (fewer live registers, more decoders per SM).
-  template <bool kSigns, bool kRefined>
-  __device__ void load(int k, Stripe& t) const {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      t.S[i] = s.sig[k + i];
-      if (kSigns) t.G[i] = s.sgn[k + i];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      t.V[i] = s.vis[k + 1 + i];
-      if (kRefined) t.R[i] = s.ref[k + 1 + i];
-      t.B[i] = 0;
-    }
+  // The windows in a mask of the half's columns (half 0: columns 0..31).
+  __device__ __forceinline__ uint32_t windows(int half, unsigned long long m0, unsigned long long m1, int k) const {
+    const uint32_t r0 = six_rows(m0, k), r1 = six_rows(m1, k), own = half ? r1 : r0;
+    uint32_t west = __shfl_up_sync(kAll, own, 1), east = __shfl_down_sync(kAll, own, 1);
+    const uint32_t edge = __shfl_sync(kAll, half ? r0 : r1, half ? 31 : 0);
+    if (lane == 0) west = half ? edge : 0u;
+    if (lane == 31) east = half ? 0u : edge;
+    return window(west, own, east);
   }
-  template <bool kSigns, bool kRefined>
-  __device__ void store(int k, const Stripe& t) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (kSigns) {  // the passes that can make samples significant
-        s.sig[k + 1 + i] = t.S[i + 1];
-        s.sgn[k + 1 + i] = t.G[i + 1];
-        s.vis[k + 1 + i] = t.V[i];
+
+  // A column's plan: a byte for each of its rows to be coded, in order:
+  // context, row << 5, and kLast in the last one. Lanes make the plans of 32
+  // columns at once, so that most symbols (those of columns with no new
+  // significant sample beside or above them) find their context made.
+  static constexpr uint32_t kLast = 0x80u;
+  static constexpr uint32_t kRunPlan = kLast | kCtxAGG;
+  template <class F>
+  __device__ __forceinline__ uint32_t plan_of(uint32_t rows, F context) const {
+    uint32_t plan = 0;
+    #pragma unroll
+    for (int r = 3; r >= 0; --r)
+      if ((rows >> r) & 1u) plan = plan << 8 | (plan ? 0u : kLast) | (uint32_t)r << 5 | context(r);
+    return plan;
+  }
+  __device__ __forceinline__ uint32_t zero_plan(uint32_t win, uint32_t rows) const {
+    return plan_of(rows, [&](int r) { return (uint32_t)zc[neighbour_index(win, r)]; });
+  }
+
+  // Significance propagation (clean false) or cleanup of 32 columns of a
+  // stripe, `cand` the columns still to come. (One copy of the code for both
+  // passes and both halves: with one each, warps in different passes ran out
+  // of instruction cache, 18.6 against 13.7 ms for a 12-page batch.)
+  __device__ __forceinline__ void zero_coding(int half, int k, uint32_t valid, bool clean) {
+    const bool inside = (int)lane + 32 * half < w;
+    uint32_t win = windows(half, col[0].sig, col[1].sig, k);
+    const uint32_t vis = four_rows(half ? col[1].vis : col[0].vis, k);
+    uint32_t todo = inside ? (clean ? ~vis : rows_near(win)) & ~own_rows(win) & valid : 0u;
+    uint32_t cand = __ballot_sync(kAll, todo != 0);
+    if (cand == 0) return;
+    // in cleanup, four rows with nothing significant around are a run
+    // (src/tier1/flags.rs:219-235)
+    uint32_t plan_me = clean && todo == 0xfu && win == 0 ? kRunPlan : zero_plan(win, todo);
+    uint32_t gwin = windows(half, col[0].sgn, col[1].sgn, k);
+    uint32_t fresh_me = 0, neg_me = 0;
+    do {
+      const int x = __ffs((int)cand) - 1;
+      cand &= cand - 1;
+      uint32_t plan = __shfl_sync(kAll, plan_me, x);
+      bool bit;
+      #pragma unroll 1
+      for (;;) {
+        bit = decode(plan & 0x1fu);
+        if (bit || (plan & kLast)) break;
+        plan >>= 8;
       }
-      if (kRefined) s.ref[k + 1 + i] = t.R[i];
-      s.bits[k + i] |= t.B[i];
-    }
-  }
-
-  // Neighbour-significance index of (x, k + r) (bit 0 NW, 1 N, 2 NE, 3 W,
-  // 5 E, 6 SW, 7 S, 8 SE; src/tier1/consts.rs).
-  template <int r>
-  __device__ __forceinline__ uint32_t nmask(const Stripe& t, int x) const {
-    const uint32_t up = win3(t.S[r], x), mid = win3(t.S[r + 1], x), dn = win3(t.S[r + 2], x);
-    return up | ((mid & 1u) << 3) | ((mid & 4u) << 3) | (dn << 6);
-  }
-
-  // Sign of a newly significant sample (src/tier1/helpers.rs:52-88).
-  template <int r>
-  __device__ __forceinline__ void sign(Stripe& t, int x) {
-    const uint64_t bx = 1ull << x;
-    const uint32_t sw = win3(t.S[r + 1], x), gw = win3(t.G[r + 1], x);  // bit 0 west, bit 2 east
-    const uint32_t ws = sw & 1u, wg = gw & 1u, es = sw >> 2, eg = gw >> 2;
-    const uint32_t ns = (uint32_t)(t.S[r] >> x) & 1u, ng = (uint32_t)(t.G[r] >> x) & 1u;
-    const uint32_t ss = (uint32_t)(t.S[r + 2] >> x) & 1u, sg = (uint32_t)(t.G[r + 2] >> x) & 1u;
-    const uint32_t lu = (ws << 3) | (ws & wg) | (ns << 1) | ((ns & ng) << 4) | (es << 5) | ((es & eg) << 2) |
-                        (ss << 7) | ((ss & sg) << 6);
-    const uint32_t neg = mq.decode(c_dec.sc[lu]) ^ c_dec.spb[lu];
-    t.S[r + 1] |= bx;
-    if (neg) t.G[r + 1] |= bx;
-  }
-
-  // Columns of the stripe with an insignificant sample next to a
-  // significant one.
-  __device__ __forceinline__ uint64_t sig_candidates(const Stripe& t, int lim) const {
-    uint64_t m = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      if (r < lim) m |= ~t.S[r + 1] & (spread(t.S[r]) | spread(t.S[r + 2]) | (t.S[r + 1] << 1) | (t.S[r + 1] >> 1));
-    return m & wmask;
-  }
-
-  template <int r>
-  __device__ __forceinline__ bool sig_one(Stripe& t, int x, uint64_t bx) {
-    if (t.S[r + 1] & bx) return false;
-    const uint32_t nm = nmask<r>(t, x);
-    if (!nm) return false;
-    const uint32_t bit = mq.decode(zc[nm]);
-    t.V[r] |= bx;
-    if (!bit) return false;
-    t.B[r] |= bx;
-    sign<r>(t, x);
-    return true;
-  }
-
-  __device__ void sigpass(int k, int lim) {
-    Stripe t;
-    load<true, false>(k, t);
-    uint64_t cols = sig_candidates(t, lim);
-    while (cols) {
-      const int x = __ffsll((long long)cols) - 1;
-      const uint64_t bx = 1ull << x;
-      bool grew = sig_one<0>(t, x, bx);
-      if (lim > 1) grew |= sig_one<1>(t, x, bx);
-      if (lim > 2) grew |= sig_one<2>(t, x, bx);
-      if (lim > 3) grew |= sig_one<3>(t, x, bx);
-      cols &= above(x);
-      if (grew) cols = sig_candidates(t, lim) & above(x);
-    }
-    store<true, false>(k, t);
-  }
-
-  template <int r>
-  __device__ __forceinline__ void ref_one(Stripe& t, int x, uint64_t bx) {
-    if (!(t.S[r + 1] & ~t.V[r] & bx)) return;
-    const int cx = (t.R[r] & bx) ? kCtxMR + 2 : (nmask<r>(t, x) ? kCtxMR + 1 : kCtxMR);
-    if (mq.decode(cx)) t.B[r] |= bx;
-    t.R[r] |= bx;
-  }
-
-  __device__ void refpass(int k, int lim) {
-    Stripe t;
-    load<false, true>(k, t);
-    uint64_t cols = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      if (r < lim) cols |= t.S[r + 1] & ~t.V[r];
-    cols &= wmask;
-    while (cols) {
-      const int x = __ffsll((long long)cols) - 1;
-      const uint64_t bx = 1ull << x;
-      ref_one<0>(t, x, bx);
-      if (lim > 1) ref_one<1>(t, x, bx);
-      if (lim > 2) ref_one<2>(t, x, bx);
-      if (lim > 3) ref_one<3>(t, x, bx);
-      cols &= above(x);
-    }
-    store<false, true>(k, t);
-  }
-
-  template <int r>
-  __device__ __forceinline__ void cleanup_one(Stripe& t, int x, uint64_t bx) {
-    if ((t.S[r + 1] | t.V[r]) & bx) return;
-    const uint32_t nm = nmask<r>(t, x);
-    if (mq.decode(nm ? zc[nm] : kCtxZC0)) {
-      t.B[r] |= bx;
-      sign<r>(t, x);
-    }
-  }
-
-  __device__ void cleanup(int k, int lim) {
-    Stripe t;
-    load<true, false>(k, t);
-    uint64_t busy = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      if (r < lim) busy |= t.S[r + 1] | t.V[r];
-    uint64_t cols = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      if (r < lim) cols |= ~(t.S[r + 1] | t.V[r]);
-    cols &= wmask;
-    while (cols) {
-      const int x = __ffsll((long long)cols) - 1;
-      const uint64_t bx = 1ull << x;
-      cols &= above(x);
-      // a full stripe's column with nothing significant or visited in it or
-      // around it is coded as a run (src/tier1/flags.rs:219-235)
-      if (lim == 4 && !(busy & bx) && win3(t.S[0] | t.S[1] | t.S[2] | t.S[3] | t.S[4] | t.S[5], x) == 0) {
-        if (mq.decode(kCtxAGG) == 0) continue;
-        int rl = (int)mq.decode(kCtxUNI) << 1;
-        rl |= (int)mq.decode(kCtxUNI);
-        if (rl == 0) {
-          t.B[0] |= bx;
-          sign<0>(t, x);
-          cleanup_one<1>(t, x, bx);
-          cleanup_one<2>(t, x, bx);
-          cleanup_one<3>(t, x, bx);
-        } else if (rl == 1) {
-          t.B[1] |= bx;
-          sign<1>(t, x);
-          cleanup_one<2>(t, x, bx);
-          cleanup_one<3>(t, x, bx);
-        } else if (rl == 2) {
-          t.B[2] |= bx;
-          sign<2>(t, x);
-          cleanup_one<3>(t, x, bx);
+      if (!bit) continue;
+      // the rest of the column, its window changing with each new sample
+      enum { kSign, kZero, kHigh, kLow };
+      int mode = plan == kRunPlan ? kHigh : kSign;
+      uint32_t r = (plan >> 5) & 3u, fresh = 0, neg = 0, rest = 0;
+      const uint32_t pair = __shfl_sync(kAll, win | todo << 28, x), gn = __shfl_sync(kAll, gwin, x);
+      uint32_t wn = pair & 0x0fffffffu, td = pair >> 28;
+      #pragma unroll 1
+      for (;;) {
+        uint32_t cx = kCtxUNI, flip = 0;
+        if (mode == kSign) {
+          const uint32_t sc = sh.sc[cross_index(wn, (int)r) | cross_index(gn | neg << 12, (int)r) << 4];
+          cx = sc & 0x7fu;
+          flip = sc >> 7;
+        } else if (mode == kZero) {
+          r = (uint32_t)__ffs((int)rest) - 1;
+          rest &= rest - 1;
+          cx = zc[neighbour_index(wn, (int)r)];
+        }
+        const uint32_t b1 = (decode(cx) ? 1u : 0u) ^ flip;
+        if (mode == kSign) {
+          neg |= b1 << r;
+          fresh |= 1u << r;
+          wn |= 0x1000u << r;
+          rest = (clean ? td : rows_near(wn) & ~own_rows(wn) & valid) & (0xeu << r);
+          td = (td & ~(0xeu << r)) | rest;  // coded, or to be coded
+          mode = kZero;
+        } else if (mode == kZero) {
+          mode = b1 ? kSign : kZero;
         } else {
-          t.B[3] |= bx;
-          sign<3>(t, x);
+          r = mode == kHigh ? b1 << 1 : r | b1;
+          mode = mode == kHigh ? kLow : kSign;
         }
-      } else {
-        cleanup_one<0>(t, x, bx);
-        if (lim > 1) cleanup_one<1>(t, x, bx);
-        if (lim > 2) cleanup_one<2>(t, x, bx);
-        if (lim > 3) cleanup_one<3>(t, x, bx);
+        if (mode == kZero && rest == 0) break;
       }
+      if ((int)lane == x) {
+        fresh_me = fresh;
+        neg_me = neg;
+        todo = td;
+      } else if ((int)lane == x + 1) {  // the column to the east sees them
+        win |= fresh << 1;
+        gwin |= neg << 1;
+        if (!clean) todo = inside ? rows_near(win) & ~own_rows(win) & valid : 0u;
+        plan_me = zero_plan(win, todo);
+      }
+      if (!clean) cand = __ballot_sync(kAll, todo != 0) & (0xfffffffeu << x);
+    } while (cand);
+    const unsigned long long f = (unsigned long long)fresh_me << (4 * k), g = (unsigned long long)neg_me << (4 * k),
+                             v = clean ? 0ull : (unsigned long long)todo << (4 * k);
+    #pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const bool it = i == half;
+      col[i].sig |= it ? f : 0ull;
+      col[i].ones |= it ? f : 0ull;
+      col[i].sgn |= it ? g : 0ull;
+      col[i].vis |= it ? v : 0ull;
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) t.V[r] = 0;
-    store<true, false>(k, t);
+  }
+
+  // Refinement changes no context but its own, so the contexts of a stripe's
+  // 32 columns are listed in shared memory first, and what is left per symbol
+  // is its decision.
+  __device__ __forceinline__ void refinement(int half, int k) {
+    const uint32_t win = windows(half, col[0].sig, col[1].sig, k);
+    const uint32_t todo = own_rows(win) & ~four_rows(half ? col[1].vis : col[0].vis, k);
+    const uint32_t in[4] = {__ballot_sync(kAll, (todo & 1u) != 0), __ballot_sync(kAll, (todo & 2u) != 0),
+                            __ballot_sync(kAll, (todo & 4u) != 0), __ballot_sync(kAll, (todo & 8u) != 0)};
+    const int total = __popc(in[0]) + __popc(in[1]) + __popc(in[2]) + __popc(in[3]);
+    if (total == 0) return;
+    // contexts 14 + (a significant neighbour), 16 once refined
+    const uint32_t near = rows_near(win), ref = four_rows(half ? col[1].ref : col[0].ref, k), before = (1u << lane) - 1u;
+    const int first = __popc(in[0] & before) + __popc(in[1] & before) + __popc(in[2] & before) + __popc(in[3] & before);
+    int at_row = first;
+    #pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if ((todo >> r) & 1u) list[at_row++] = (uint8_t)((ref >> r) & 1u ? 16u : 14u + ((near >> r) & 1u));
+    __syncwarp();
+    #pragma unroll 1
+    for (int i = 0; i < total; i += 4) {
+      const uint32_t four = *reinterpret_cast<const uint32_t*>(list + i);
+      uint32_t got = decode(four & 0xffu) ? 1u : 0u;
+      if (i + 1 < total && decode((four >> 8) & 0xffu)) got |= 2u;
+      if (i + 2 < total && decode((four >> 16) & 0xffu)) got |= 4u;
+      if (i + 3 < total && decode(four >> 24)) got |= 8u;
+      if (lane == 0) list[i >> 2] = (uint8_t)got;  // in the place of a context that has been read
+    }
+    __syncwarp();
+    uint32_t bits = (uint32_t)(list[first >> 2] | list[(first >> 2) + 1] << 4) >> (first & 3), ones = 0;
+    #pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if ((todo >> r) & 1u) {
+        ones |= (bits & 1u) << r;
+        bits >>= 1;
+      }
+    __syncwarp();
+    #pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      col[i].ones |= i == half ? (unsigned long long)ones << (4 * k) : 0ull;
+      col[i].ref |= i == half ? (unsigned long long)todo << (4 * k) : 0ull;
+    }
+  }
+
+  // pass 0 significance propagation, 1 refinement, 2 cleanup
+  __device__ __forceinline__ void run_pass(int pass) {
+    const int halves = w > 32 ? 2 : 1, parts = halves * ((h + 3) / 4);
+    #pragma unroll 1
+    for (int part = 0; part < parts; ++part) {
+      const int k = halves == 2 ? part >> 1 : part, half = halves == 2 ? part & 1 : 0;
+      const uint32_t valid = h - 4 * k >= 4 ? 0xfu : (1u << (h - 4 * k)) - 1u;
+      if (pass == 1) refinement(half, k);
+      else zero_coding(half, k, valid, pass == 2);
+    }
+    if (pass == 2) col[0].vis = col[1].vis = 0;
   }
 };
 
-// H decoders per warp: with H = 2 each half-warp decodes its own block
-// (its lane 0 running the chain, its 16 lanes merging), so two chains share
-// a warp's instruction stream: more decoders per SM for batches, at some
-// cost to each chain where the two diverge.
-template <int H>
-__global__ void __launch_bounds__(kDecWarps * 32) t1_decode_kernel(const DecBlock* blocks, uint32_t nblocks,
-                                                                     const uint8_t* data, int32_t* planes) {
-  constexpr int HL = 32 / H;  // lanes per decoder
-  constexpr int NX = 64 / HL;  // columns each lane merges
-  __shared__ WarpState st_all[kDecWarps * H];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int half = lane / HL, hl = lane % HL;
-  const uint32_t hmask = H == 1 ? 0xffffffffu : (0xffffu << (16 * half));
-  const uint32_t blk = (blockIdx.x * kDecWarps + wid) * H + half;
-  if (blk >= nblocks) return;
-  WarpState& s = st_all[wid * H + half];
-  const DecBlock d = blocks[blk];
-  for (int i = hl; i < 66; i += HL) s.sig[i] = s.sgn[i] = s.vis[i] = s.ref[i] = 0;
-  for (int i = hl; i < 64; i += HL) s.bits[i] = 0;
-  // initial context states (src/mq/mod.rs:195-200)
-  for (int i = hl; i < 20; i += HL) s.ctx[i] = i == kCtxUNI ? 92 : i == kCtxAGG ? 6 : i == kCtxZC0 ? 8 : 0;
+__global__ void __launch_bounds__(kDecWarps * 32) t1_decode_kernel(const DecBlock* blocks, const uint32_t* order,
+                                                                   uint32_t nblocks, const uint8_t* data,
+                                                                   unsigned long long* masks) {
+  __shared__ DecShared sh;
+  __shared__ __align__(4) uint8_t lists[kDecWarps][132];
+  load_dec_shared(sh);
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31, slot = blockIdx.x * kDecWarps + (threadIdx.x >> 5);
+  if (slot >= nblocks) return;
+  const DecBlock d = blocks[order[slot]];
+  if (d.npasses == 0) return;
+  BlockDecoder dec{sh, sh.zc[d.orient & 3], lists[threadIdx.x >> 5], lane, d.w, d.h};
+  dec.start(data + d.data_off, d.data_len);
+  unsigned long long* out = masks + d.mask_off;
+  // cleanup of the top bit-plane, then significance, refinement and cleanup
+  // per bit-plane until the block's passes end
+  int left = d.npasses, pass = 2;
+  while (left > 0) {
+    dec.run_pass(pass);
+    --left;
+    if (pass == 2 || left == 0) {  // the bit-plane's masks
+      out[lane] = dec.col[0].ones;
+      out[lane + 32] = dec.col[1].ones;
+      dec.col[0].ones = dec.col[1].ones = 0;
+      out += 64;
+    }
+    pass = pass == 2 ? 0 : pass + 1;
+  }
+  out[lane] = dec.col[0].sgn;
+  out[lane + 32] = dec.col[1].sgn;
+}
+
+// Coefficients of every code-block from its masks, a warp per block: a lane
+// takes 32 rows of a column, and a 32x32 bit transpose in registers turns its
+// bit-planes into magnitudes. Signed integers (reversible codestreams) or
+// midpoint-dequantised values (sign * (|q| + 0.5) * step,
+// src/simd/scalar.rs:122-129).
+__global__ void __launch_bounds__(128) t1_coefficients_kernel(const DecBlock* blocks, uint32_t nblocks,
+                                                              const unsigned long long* masks, int32_t* planes) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (b >= nblocks) return;
+  const DecBlock d = blocks[b];
   int32_t* plane = planes + d.plane_off;
-  const int w = d.w, h = d.h;
-  __syncwarp(hmask);
-  BlockDecoder dec{s, {}, c_dec.zc + (d.orient & 3) * 512, w == 64 ? ~0ull : (1ull << w) - 1};
-  if (hl == 0 && d.npasses > 0) dec.mq.init(data + d.data_off, d.data_len, s.ctx);
-  // pass sequence: cleanup of the top bit-plane, then significance,
-  // refinement and cleanup per bit-plane until the block's passes end
-  const int top = (int)d.mb - (int)d.zbp - 1;  // checked on the host: 0..30
-  int remaining = d.npasses;
-  for (int bp = top; bp >= 0 && remaining > 0; --bp) {
-    if (hl == 0) {
-      if (bp < top) {
-        for (int k = 0; k < h; k += 4) dec.sigpass(k, min(4, h - k));
-        if (--remaining > 0) {
-          for (int k = 0; k < h; k += 4) dec.refpass(k, min(4, h - k));
-          if (--remaining > 0) {
-            for (int k = 0; k < h; k += 4) dec.cleanup(k, min(4, h - k));
-            --remaining;
-          }
+  const int top = (int)d.mb - (int)d.zbp - 1, np = (int)dec_planes(d.npasses);
+  const uint32_t* mw = reinterpret_cast<const uint32_t*>(masks + d.mask_off);
+  #pragma unroll 1
+  for (int x = lane; x < d.w; x += 32)
+    #pragma unroll 1
+    for (int half = 0; 32 * half < d.h; ++half) {
+      uint32_t t[32];
+      #pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const int j = top - k;  // bit-plane k is the block's plane j
+        t[k] = j >= 0 && j < np ? mw[(64 * j + x) * 2 + half] : 0u;
+      }
+      const uint32_t sg = np > 0 ? mw[(64 * np + x) * 2 + half] : 0u;
+      transpose32(t);
+      #pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int y = 32 * half + i;
+        if (y >= d.h) break;
+        const bool neg = (sg >> i) & 1u;
+        int32_t v = neg ? -(int32_t)t[i] : (int32_t)t[i];
+        if (!d.reversible) {
+          float f = 0.0f;
+          if (t[i] != 0) f = __fmul_rn(__fmul_rn(neg ? -1.0f : 1.0f, __fadd_rn((float)t[i], 0.5f)), d.step);
+          v = __float_as_int(f);
         }
-      } else {
-        for (int k = 0; k < h; k += 4) dec.cleanup(k, min(4, h - k));
-        --remaining;
-      }
-    } else {
-      remaining -= bp < top ? min(3, remaining) : 1;
-    }
-    __syncwarp(hmask);
-    const int32_t one = (int32_t)(1u << bp);
-    for (int y = 0; y < h; ++y) {
-      const uint64_t bits = s.bits[y];
-      if (!bits) continue;
-      int32_t* row = plane + (size_t)y * d.stride;
-#pragma unroll
-      for (int m = 0; m < NX; ++m) {
-        const int x = hl + HL * m;
-        if (x < w && ((bits >> x) & 1u)) row[x] |= one;
+        plane[(size_t)y * d.stride + x] = v;
       }
     }
-    __syncwarp(hmask);
-    for (int i = hl; i < 64; i += HL) s.bits[i] = 0;
-    __syncwarp(hmask);
-  }
-  // signed coefficients, or their midpoint dequantised values
-  for (int y = 0; y < h; ++y) {
-    const uint64_t neg = s.sgn[y + 1];
-    int32_t* row = plane + (size_t)y * d.stride;
-#pragma unroll
-    for (int m = 0; m < NX; ++m) {
-      const int x = hl + HL * m;
-      if (x >= w) continue;
-      const int32_t mag = row[x];
-      const bool n = (neg >> x) & 1u;
-      if (d.reversible) {
-        row[x] = n ? -mag : mag;
-      } else {
-        float v = 0.0f;
-        if (mag != 0) v = __fmul_rn(__fmul_rn(n ? -1.0f : 1.0f, __fadd_rn((float)(uint32_t)mag, 0.5f)), d.step);
-        row[x] = __float_as_int(v);
-      }
-    }
-  }
+}
+
+// Decoding order: longest segments first (counting sort on 1024 buckets of 16
+// bytes), so that the longest chains start first.
+constexpr uint32_t kDecBuckets = 1024;
+__device__ __forceinline__ uint32_t dec_bucket(const DecBlock& d) {
+  return kDecBuckets - 1 - min(d.data_len >> 4, kDecBuckets - 1);
+}
+__global__ void dec_hist_kernel(const DecBlock* blocks, uint32_t n, uint32_t* hist) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n) atomicAdd(hist + dec_bucket(blocks[b]), 1u);
+}
+__global__ void dec_scatter_kernel(const DecBlock* blocks, uint32_t n, uint32_t* cursor, uint32_t* order) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n) order[atomicAdd(cursor + dec_bucket(blocks[b]), 1u)] = b;
 }
 
 }  // namespace
@@ -425,16 +454,19 @@ bool upload_decode_tables(const uint8_t* zc, const uint8_t* sc, const uint8_t* s
   return cudaMemcpyToSymbol(c_dec, &t, sizeof t) == cudaSuccess;
 }
 
-void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, int32_t* planes, int per_warp,
-                      cudaStream_t st) {
+void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, unsigned long long* masks,
+                      int32_t* planes, uint32_t* scratch, cudaStream_t st) {
   if (nblocks == 0) return;
-  if (per_warp == 2) {
-    const uint32_t per_cta = kDecWarps * 2;
-    t1_decode_kernel<2><<<(nblocks + per_cta - 1) / per_cta, kDecWarps * 32, 0, st>>>(blocks, nblocks, data, planes);
-  } else {
-    t1_decode_kernel<1><<<(nblocks + kDecWarps - 1) / kDecWarps, kDecWarps * 32, 0, st>>>(blocks, nblocks, data,
-                                                                                           planes);
-  }
+  uint32_t* hist = scratch;
+  uint32_t* cursor = scratch + kDecBuckets;
+  uint32_t* order = scratch + 2 * kDecBuckets;
+  cudaMemsetAsync(hist, 0, kDecBuckets * sizeof(uint32_t), st);
+  const uint32_t g = (nblocks + 255) / 256;
+  dec_hist_kernel<<<g, 256, 0, st>>>(blocks, nblocks, hist);
+  launch_scan_u32(hist, 1, kDecBuckets - 1, cursor, order, st);  // `order` is filled after the scan
+  dec_scatter_kernel<<<g, 256, 0, st>>>(blocks, nblocks, cursor, order);
+  t1_decode_kernel<<<(nblocks + kDecWarps - 1) / kDecWarps, kDecWarps * 32, 0, st>>>(blocks, order, nblocks, data, masks);
+  t1_coefficients_kernel<<<(nblocks + 3) / 4, 128, 0, st>>>(blocks, nblocks, masks, planes);
 }
 
 }  // namespace jp2g

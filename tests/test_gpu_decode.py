@@ -206,3 +206,17 @@ def test_large_decode_batch_two_decoders_per_warp(eng, orc):
         assert not isinstance(g, Exception), g
         assert np.array_equal(np.asarray(g[0]), np.asarray(eng.decode(f, **flags)[0]))
     assert np.array_equal(np.asarray(got[1][0]), orc.decode(files[1], **flags)[3])
+
+
+@pytest.mark.parametrize("q", [100, 80, 20])
+@pytest.mark.parametrize("w,h", [(31, 4), (32, 5), (33, 3), (63, 64), (65, 66), (96, 1), (2, 130), (161, 97)])
+def test_decode_at_the_edges_of_stripes_and_halves(eng, orc, w, h, q):
+    # code-blocks of one to sixteen stripes, the last one of one to four
+    # rows, and of one and both halves of 32 columns; noise, so that every
+    # neighbourhood occurs
+    px = np.random.default_rng(w * 131 + h).integers(0, 256, w * h, dtype=np.uint8)
+    data = eng.encode(px, w, h, 1, q, 0)
+    want = orc.decode(data, accept_empty_segments=True)[3]
+    assert np.array_equal(eng.decode(data, accept_empty_segments=True)[0], want)
+    if q == 100:
+        assert np.array_equal(want, px)
