@@ -41,7 +41,7 @@ __constant__ DecTables c_dec;
 constexpr int kDecWarps = 4;
 constexpr uint32_t kDecStates = 94;
 
-// Context word: Qe << 16 | state << 3 | MPS. The table holds per state (state,
+// Context word: Qe << 15 | state << 3 | MPS. The table holds per state (state,
 // MPS pair) the words after an MPS and an LPS renormalisation.
 struct DecShared {
   uint2 next[kDecStates];
@@ -49,7 +49,7 @@ struct DecShared {
   uint8_t sc[256];     // sign context | prediction bit << 7 (cross_index)
 };
 __device__ __forceinline__ uint32_t dec_word(uint32_t state) {
-  return (c_dec.mq[state] & 0xffffu) << 16 | state << 3 | (state & 1u);
+  return (c_dec.mq[state] & 0xffffu) << 15 | state << 3 | (state & 1u);
 }
 // The tables in the layouts used here, from those of c_dec (src/tier1/
 // consts.rs: zero coding bit 0 NW, 1 N, 2 NE, 3 W, 5 E, 6 SW, 7 S, 8 SE; sign
@@ -116,21 +116,24 @@ struct BlockDecoder {
   uint32_t lane;
   int w, h;
   // the MQ decoder (ISO/IEC 15444-1 C.3; src/mq/mod.rs:38-160), the same in
-  // all lanes: C as it is, A << 16; cur and nxt are the segment's bytes bp and
+  // all lanes: A << 15 and C >> 1 (its lowest bit is always 0), so that a
+  // difference's sign bit compares; cur and nxt are the segment's bytes bp and
   // bp + 1, 0xFF beyond its end
   const uint8_t* b;
   uint32_t n, bp, cur, nxt, a, c;
-  int ct;
+  int ct;               // below 0: C is still to be shifted, from shift_from by `shift`
+  uint32_t shift_from;
+  int shift;
   uint32_t word, mps_next, lps_next;  // this lane's context, and its successors
   Column col[2];
 
   __device__ __forceinline__ uint32_t at(uint32_t i) const { return i < n ? b[i] : 0xffu; }
   __device__ __forceinline__ void bytein() {
     if (cur == 0xffu && nxt > 0x8fu) {
-      c += 0xff00u;
+      c += 0x7f80u;
       ct = 8;
     } else {
-      c += cur == 0xffu ? nxt << 9 : nxt << 8;
+      c = (c + (cur == 0xffu ? nxt << 8 : nxt << 7)) & 0x7fffffffu;
       ct = cur == 0xffu ? 7 : 8;
       ++bp;
       cur = nxt;
@@ -148,39 +151,49 @@ struct BlockDecoder {
     bp = 0;
     cur = at(0);
     nxt = at(1);
-    c = cur << 16;
+    c = cur << 15;
     bytein();
     c <<= 7;
     ct -= 7;
-    a = 0x80000000u;
+    a = 0x40000000u;
   }
   // After A -= Qe the coder takes Qe when C lies below it, else A (and takes
   // Qe off C); the decision is the LPS when that differs from A < Qe, and the
-  // context moves on when the result is renormalised.
+  // context moves on when the result is renormalised. The comparisons are
+  // masks (a predicate takes longer to reach its users than a sign bit), and
+  // the bytes that a shift has run out of are read at the next symbol, while
+  // its context is on its way.
   __device__ __forceinline__ bool decode(uint32_t cx) {
     const uint32_t e = __shfl_sync(kAll, word, (int)cx);
-    const uint32_t qe = e & 0xffff0000u;
-    const uint32_t d = a - qe;
-    const bool low = c < qe;
-    const bool lps = low != (d < qe);
-    if ((low || (int)d >= 0) && lane == cx) {
-      word = lps ? lps_next : mps_next;
-      const uint2 t = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(sh.next) + (word & 0x3f8u));
-      mps_next = t.x;
-      lps_next = t.y;
+    if (ct < 0) {
+      c = shift_from;
+      ct += shift;
+      int k = shift;
+      while (k > ct) {
+        c = (c << ct) & 0x7fffffffu;
+        k -= ct;
+        bytein();
+      }
+      c = (c << k) & 0x7fffffffu;
+      ct -= k;
     }
-    const uint32_t v = low ? qe : d;
-    if (!low) c -= qe;
-    int k = __clz((int)v);
-    a = v << k;
-    while (k > ct) {
-      c <<= ct;
-      k -= ct;
-      bytein();
+    const uint32_t qe = e & 0x7fff8000u;
+    const uint32_t d = a - qe, t = c - qe;
+    const uint32_t low = (uint32_t)((int)t >> 31), lps = low ^ (uint32_t)((int)(d - qe) >> 31);
+    const uint32_t move = (low | ((d >> 30) - 1u)) & (lane == cx ? kAll : 0u);
+    word = (((lps_next & lps) | (mps_next & ~lps)) & move) | (word & ~move);
+    if (move) {
+      const uint2 n = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(sh.next) + (word & 0x3f8u));
+      mps_next = n.x;
+      lps_next = n.y;
     }
-    c <<= k;
-    ct -= k;
-    return ((e & 1u) != 0) != lps;
+    const uint32_t v = (qe & low) | (d & ~low);
+    shift_from = (c & low) | (t & ~low);
+    shift = __clz((int)v) - 1;
+    a = v << shift;
+    c = (shift_from << shift) & 0x7fffffffu;
+    ct -= shift;
+    return ((e ^ lps) & 1u) != 0;
   }
 
   // The windows in a mask of the half's columns (half 0: columns 0..31).
@@ -240,38 +253,29 @@ struct BlockDecoder {
       }
       if (!bit) continue;
       // the rest of the column, its window changing with each new sample
-      enum { kSign, kZero, kHigh, kLow };
-      int mode = plan == kRunPlan ? kHigh : kSign;
-      uint32_t r = (plan >> 5) & 3u, fresh = 0, neg = 0, rest = 0;
+      uint32_t r = (plan >> 5) & 3u, fresh = 0, neg = 0;
       const uint32_t pair = __shfl_sync(kAll, win | todo << 28, x), gn = __shfl_sync(kAll, gwin, x);
       uint32_t wn = pair & 0x0fffffffu, td = pair >> 28;
+      if (plan == kRunPlan) {
+        r = 0;
+        #pragma unroll 1
+        for (int i = 0; i < 2; ++i) r = r << 1 | (decode(kCtxUNI) ? 1u : 0u);
+      }
       #pragma unroll 1
-      for (;;) {
-        uint32_t cx = kCtxUNI, flip = 0;
-        if (mode == kSign) {
-          const uint32_t sc = sh.sc[cross_index(wn, (int)r) | cross_index(gn | neg << 12, (int)r) << 4];
-          cx = sc & 0x7fu;
-          flip = sc >> 7;
-        } else if (mode == kZero) {
+      while (bit) {
+        const uint32_t sc = sh.sc[cross_index(wn, (int)r) | cross_index(gn | neg << 12, (int)r) << 4];
+        neg |= ((decode(sc & 0x7fu) ? 1u : 0u) ^ (sc >> 7)) << r;
+        fresh |= 1u << r;
+        wn |= 0x1000u << r;
+        uint32_t rest = (clean ? td : rows_near(wn) & ~own_rows(wn) & valid) & (0xeu << r);
+        td = (td & ~(0xeu << r)) | rest;  // coded, or to be coded
+        bit = false;
+        #pragma unroll 1
+        while (rest && !bit) {
           r = (uint32_t)__ffs((int)rest) - 1;
           rest &= rest - 1;
-          cx = zc[neighbour_index(wn, (int)r)];
+          bit = decode(zc[neighbour_index(wn, (int)r)]);
         }
-        const uint32_t b1 = (decode(cx) ? 1u : 0u) ^ flip;
-        if (mode == kSign) {
-          neg |= b1 << r;
-          fresh |= 1u << r;
-          wn |= 0x1000u << r;
-          rest = (clean ? td : rows_near(wn) & ~own_rows(wn) & valid) & (0xeu << r);
-          td = (td & ~(0xeu << r)) | rest;  // coded, or to be coded
-          mode = kZero;
-        } else if (mode == kZero) {
-          mode = b1 ? kSign : kZero;
-        } else {
-          r = mode == kHigh ? b1 << 1 : r | b1;
-          mode = mode == kHigh ? kLow : kSign;
-        }
-        if (mode == kZero && rest == 0) break;
       }
       if ((int)lane == x) {
         fresh_me = fresh;
@@ -315,14 +319,20 @@ struct BlockDecoder {
     for (int r = 0; r < 4; ++r)
       if ((todo >> r) & 1u) list[at_row++] = (uint8_t)((ref >> r) & 1u ? 16u : 14u + ((near >> r) & 1u));
     __syncwarp();
+    int i = 0;
     #pragma unroll 1
-    for (int i = 0; i < total; i += 4) {
+    for (; i + 4 <= total; i += 4) {
       const uint32_t four = *reinterpret_cast<const uint32_t*>(list + i);
-      uint32_t got = decode(four & 0xffu) ? 1u : 0u;
-      if (i + 1 < total && decode((four >> 8) & 0xffu)) got |= 2u;
-      if (i + 2 < total && decode((four >> 16) & 0xffu)) got |= 4u;
-      if (i + 3 < total && decode(four >> 24)) got |= 8u;
+      uint32_t got = 0;
+      #pragma unroll
+      for (int j = 0; j < 4; ++j) got |= decode((four >> (8 * j)) & 0xffu) ? 1u << j : 0u;
       if (lane == 0) list[i >> 2] = (uint8_t)got;  // in the place of a context that has been read
+    }
+    if (i < total) {
+      uint32_t four = *reinterpret_cast<const uint32_t*>(list + i), got = 0;
+      #pragma unroll 1
+      for (int j = i; j < total; ++j, four >>= 8) got |= decode(four & 0xffu) ? 1u << (j & 3) : 0u;
+      if (lane == 0) list[i >> 2] = (uint8_t)got;
     }
     __syncwarp();
     uint32_t bits = (uint32_t)(list[first >> 2] | list[(first >> 2) + 1] << 4) >> (first & 3), ones = 0;
