@@ -807,7 +807,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
       !reserve(c, c->blocks, std::max<size_t>(nb, 1) * sizeof(BlockDesc)) ||
       !reserve(c, c->bands, bands.size() * sizeof(BandParam)) ||
       !reserve(c, c->comps, comps.size() * sizeof(CompParam)) ||
-      !reserve(c, c->maxslope, std::max<size_t>(comps.size(), 8) * (sizeof(unsigned long long) + sizeof(uint32_t))) ||
+      !reserve(c, c->maxslope, std::max<size_t>(comps.size(), 8) * (sizeof(unsigned long long) + 4 * sizeof(uint32_t))) ||
       !reserve(c, c->hullp, std::max<size_t>(nb, 1) * pcap * sizeof(uint16_t)) ||
       !reserve(c, c->hulls, std::max<size_t>(nb, 1) * pcap * sizeof(double)) ||
       !reserve(c, c->hulln, std::max<size_t>(nb, 1)) ||
@@ -882,8 +882,8 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   ta.comps = dptr<CompParam>(c->comps);
   // the inspection entry points see every pass of every block
   ta.settled = dbg ? nullptr : reinterpret_cast<uint32_t*>(dptr<unsigned long long>(c->maxslope) + comps.size());
-  if (!cuda_ok(c, cudaMemsetAsync(c->stats.p, 0, 8, c->stream), "memset") ||
-      (ta.settled && !cuda_ok(c, cudaMemsetAsync(ta.settled, 0, comps.size() * 4, c->stream), "memset")))
+  if (!cuda_ok(c, cudaMemsetAsync(c->stats.p, 0, 64, c->stream), "memset") ||
+      (ta.settled && !cuda_ok(c, cudaMemsetAsync(ta.settled, 0, comps.size() * 16, c->stream), "memset")))
     return kEncodeFailed;
   launch_t1_analyze(ta, c->stream);
   launch_scan_u32(ta.nplanes, 1, nb, ta.plane_base, dptr<uint32_t>(c->scratch), c->stream);
@@ -904,9 +904,15 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   ta.planes = dptr<uint32_t>(c->planes);
   ta.signs = dptr<uint32_t>(c->signs);
   ta.sym = dptr<uint8_t>(c->sym);
+  ta.counts = dptr<uint32_t>(c->stats) + 4;
+  // Modelling every bit-plane costs a small wave less than a second round;
+  // for large ones it is the largest stage, and two thirds of it would be for
+  // bit-planes that are never coded.
+  ta.foresee = ta.settled && nb > (uint32_t)c->num_sms * 48u &&
+               std::any_of(live.begin(), live.end(), [](const PageJob* j) { return !j->plan.lossless; });
   launch_t1_planes(ta, c->stream);
   record(c, kEvAnalyzeEnd);
-  launch_t1_model(ta, c->num_sms, c->stream);
+  launch_t1_model(ta, c->num_sms, 0, c->stream);
   record(c, kEvModelEnd);
   // Blocks are coded heaviest first, one per lane: a warp's lanes then carry
   // similar symbol counts, and the longest chains start first.
@@ -914,8 +920,16 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
     return kEncodeFailed;
   launch_mq_order(ta, dptr<uint32_t>(c->mqorder), dptr<uint32_t>(c->mqscratch), c->stream);
   ta.mq_order = dptr<uint32_t>(c->mqorder);
-  launch_t1_mq(ta, c->num_sms, (int)c->opt[JP2G_OPT_MQ_BLOCKS_PER_WARP], c->stream);
-  c->counters[5] += 8 + (nb > 1024 ? 1 : 0);
+  ta.unfinished = dptr<uint32_t>(c->mqscratch);  // the order has been made
+  const int bpw = (int)c->opt[JP2G_OPT_MQ_BLOCKS_PER_WARP];
+  launch_t1_mq(ta, c->num_sms, bpw, 0, c->stream);
+  if (ta.foresee) {
+    ta.again = dptr<uint32_t>(c->mqorder);
+    launch_t1_recheck(ta, c->num_sms, c->stream);
+    launch_t1_model(ta, c->num_sms, 1, c->stream);
+    launch_t1_mq(ta, c->num_sms, bpw, 1, c->stream);
+  }
+  c->counters[5] += 8 + (nb > 1024 ? 1 : 0) + (ta.foresee ? 3 : 0);
   record(c, 3);
   // ---- PCRD ----
   PcrdArgs pa{};

@@ -59,10 +59,14 @@ struct T1Args {
   uint32_t pass_cap;  // pass records available per block
   BlockOut* res;
   // (block, bit-plane) modelling items
-  uint32_t* nplanes;     // per block: magnitude bit-planes to model
-  uint32_t* plane_base;  // per block: first item (exclusive prefix of nplanes)
-  uint32_t* items;       // per item: its block
-  uint32_t nitems;
+  uint32_t* nplanes;     // per block: magnitude bit-planes, then (t1_planes_kernel) those to model at first
+  uint32_t* plane_base;  // per block: its first item (exclusive prefix of the magnitude bit-planes)
+  uint32_t* items;       // items to model, block << 6 | index within the block: the first round's, then the second's
+  uint32_t nitems;       // all items
+  uint32_t* counts;      // zeroed: [0] items of the first round, [1] of the second, [2] unfinished, [3] again
+  uint32_t* unfinished;  // blocks that ended the first round with bit-planes to go
+  uint32_t* again;       // those of them that the second round codes on
+  bool foresee;          // model only the bit-planes a block is likely to need; a second round takes the others
   uint32_t* planes;      // per item: column masks of its plane (t1_planes_kernel), 1 KiB
   uint32_t* signs;       // per block: sign column masks, 512 B
   ItemRec* item_rec;
@@ -72,17 +76,21 @@ struct T1Args {
   const uint32_t* mq_order;       // MQ processing order of the blocks
   const BandParam* bands;
   const CompParam* comps;
-  // per component key, zeroed: 1 once a block has shown a slope that settles
-  // the component's lambda; null: code every pass of every block
+  // four per component key, zeroed: 1 once a block has shown a slope that
+  // settles the component's lambda, a half, a quarter, an eighth of it; null:
+  // code every pass of every block
   uint32_t* settled;
 };
 
 void launch_t1_analyze(const T1Args& a, cudaStream_t st);
 // Items list and per-item bit-plane column masks (after the plane-count scan).
 void launch_t1_planes(const T1Args& a, cudaStream_t st);
-void launch_t1_model(const T1Args& a, int num_sms, cudaStream_t st);
+// round 0: the items foreseen, 1: the others of the blocks that are coded again.
+void launch_t1_model(const T1Args& a, int num_sms, int round, cudaStream_t st);
 // bpw: code-blocks per warp, 1..32, or 0 for automatic.
-void launch_t1_mq(const T1Args& a, int num_sms, int bpw, cudaStream_t st);
+void launch_t1_mq(const T1Args& a, int num_sms, int bpw, int round, cudaStream_t st);
+// Between the rounds: which unfinished blocks are coded on.
+void launch_t1_recheck(const T1Args& a, int num_sms, cudaStream_t st);
 // Code-blocks per warp that launch_t1_mq uses for `bpw` (0 = automatic).
 int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw);
 // Orders the blocks by their MQ symbol count, largest first (counting sort

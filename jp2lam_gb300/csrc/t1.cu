@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(256) t1_planes_kernel(T1Args a) {
   const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= a.nblocks) return;
   const uint32_t np = a.nplanes[b], base = a.plane_base[b];
-  for (uint32_t j = lane; j < np; j += 32) a.items[base + j] = b;
   const BlockDesc d = a.blocks[b];
   const int w = d.w, h = d.h, mbp = (int)np;
   const int32_t* blk = a.coef + (size_t)d.coef_slot * a.cbw * a.cbh;
@@ -174,8 +173,48 @@ __global__ void __launch_bounds__(256) t1_planes_kernel(T1Args a) {
     if (lane >= o) below += v;
   }
   below = __shfl_up_sync(0xffffffffu, below, 1);  // planes 0..k-1
+  const float unit = block_unit(a, b, d);
   if (lane < mbp)
-    a.item_rec[base + (uint32_t)(mbp - 1 - lane)].remain = lane == 0 ? 0.0f : below * block_unit(a, b, d) * 1.00001f;
+    a.item_rec[base + (uint32_t)(mbp - 1 - lane)].remain = lane == 0 ? 0.0f : below * unit * 1.00001f;
+  // The bit-planes to model: to the one after which coding is likely to stop
+  // (see Stop), and one more. Bytes are estimated from the counts: a sample
+  // that may become significant costs the entropy of doing so, less a share
+  // for its context, and a sign; one already significant nearly a bit.
+  // On a 2550x3300 page 2 blocks of 2,107 need more than that.
+  uint32_t count = (uint32_t)mbp;
+  const CompParam& cp = a.comps[d.comp_key];
+  if (a.foresee && !cp.lossless) {
+    const float before = (float)(sig - newly), open = (float)(w * h) - before, n = (float)newly;
+    const float p = open > 0.0f ? n / open : 0.0f;
+    const float entropy = p > 0.0f && p < 1.0f ? -(p * __log2f(p) + (1.0f - p) * __log2f(1.0f - p)) : 0.0f;
+    float bytes = lane < mbp ? (0.7f * open * entropy + n + 0.9f * before) * 0.125f : 0.0f;
+    float removed = lane < mbp ? gain * unit : 0.0f;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {  // planes k and above
+      const float vb = __shfl_down_sync(0xffffffffu, bytes, o), vr = __shfl_down_sync(0xffffffffu, removed, o);
+      if (lane + o < 32) {
+        bytes += vb;
+        removed += vr;
+      }
+    }
+    const float value = removed - cp.lambda * (bytes + 2.0f);
+    float best = lane < mbp ? fmaxf(value, 0.0f) : 0.0f;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_down_sync(0xffffffffu, best, o);
+      if (lane + o < 32) best = fmaxf(best, v);
+    }
+    const float rest = lane == 0 ? 0.0f : below * unit;
+    const uint32_t stops = __ballot_sync(0xffffffffu, lane < mbp && value + rest < best);
+    if (stops) count = min(count, (uint32_t)(mbp - (31 - __clz((int)stops))) + 1u);
+  }
+  uint32_t at = 0;
+  if (lane == 0) {
+    a.nplanes[b] = count;
+    at = atomicAdd(a.counts, count);
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  for (uint32_t j = lane; j < count; j += 32) a.items[at + j] = b << 6 | j;
 }
 
 // Modelling works on the code-block in column layout: lane L owns columns
@@ -349,7 +388,7 @@ __device__ __forceinline__ void emit_column(uint32_t v, uint32_t sm, uint32_t c,
 //    run), so each lane writes its two columns' symbols into the three
 //    streams (SP | MR | cleanup, whose starts are known from the totals) at
 //    offsets from two packed warp scans.
-__global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a) {
+__global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a, int round) {
   __shared__ ModelSmem sm_all[kModelWarps];
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
@@ -357,12 +396,14 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a)
   const uint32_t nwarps = gridDim.x * kModelWarps;
   const int xa = lane, xb = lane + 32;
 
-  for (uint32_t item = blockIdx.x * kModelWarps + wid; item < a.nitems; item += nwarps) {
-    const uint32_t blkno = a.items[item];
+  const uint32_t from = round ? a.counts[0] : 0u, count = a.counts[round];
+  for (uint32_t i = blockIdx.x * kModelWarps + wid; i < count; i += nwarps) {
+    const uint32_t blkno = a.items[from + i] >> 6;
     const BlockDesc d = a.blocks[blkno];
     const int w = d.w, h = d.h;
     const int mbp = a.res[blkno].mbp;
-    const int j = (int)(item - a.plane_base[blkno]);
+    const int j = (int)(a.items[from + i] & 63u);
+    const uint32_t item = a.plane_base[blkno] + (uint32_t)j;
     const int p = mbp - 1 - j;
     const bool top = j == 0;
     const uint64_t rows = h >= 64 ? ~0ull : ((1ull << h) - 1);
@@ -655,7 +696,7 @@ __device__ __forceinline__ uint32_t sym_sign(uint32_t w, int i) { return w << (2
 __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, const uint4 q) {
   const uint32_t w[5] = {q.x, q.y, q.z, q.w, kPadSymbol};
   const uint32_t table = (uint32_t)__cvta_generic_to_shared(&sm.table) - 3u;
-  uint32_t add[16], ex[16];
+  uint32_t ops[16];  // exponent of the result (127 - the shift) << 23 | addition to C
   uint64_t acc = 0;
   int room = 31;  // fractional bits left: 31 - shifts so far
   uint32_t cx = sym_ctx(w[0], 0, lane);
@@ -674,10 +715,10 @@ __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, con
     const float v = take_a ? a : qe;
     const uint32_t vb = __float_as_uint(v);
     m.a = __uint_as_float((vb & 0x7fffffu) | 0x3f800000u);
-    add[i] = take_a ? e.y >> 16 : 0u;
-    ex[i] = vb >> 23;  // 127 - the shift
-    acc += (uint64_t)add[i] * __funnelshift_l(0u, 1u, (uint32_t)room);
-    room += (int)ex[i] - 127;
+    const uint32_t add = take_a ? e.y >> 16 : 0u;
+    ops[i] = (vb & 0xff800000u) | add;
+    acc += (uint64_t)add * __funnelshift_l(0u, 1u, (uint32_t)room);
+    room += (int)(vb >> 23) - 127;
     // the next state, loaded only when renormalised (selecting from a load
     // made ahead costs more in selects than it hides)
     asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, 0f3F800000;\n\t@p ld.shared.v2.u32 {%0, %1}, [%3];\n\t}"
@@ -715,8 +756,14 @@ __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, con
     }
   }
   if (one_by_one) {
-    #pragma unroll
-    for (int i = 0; i < 16; ++i) mq_shift(m, add[i], 127 - (int)ex[i]);
+    // (rolled: unrolled sixteen times it took the registers of the code above)
+    #pragma unroll 1
+    for (int h = 0; h < 4; ++h) {
+      #pragma unroll
+      for (int i = 0; i < 4; ++i) mq_shift(m, ops[i] & 0xffffu, 127 - (int)(ops[i] >> 23));
+      #pragma unroll
+      for (int i = 0; i < 12; ++i) ops[i] = ops[i + 4];
+    }
   }
 }
 
@@ -729,40 +776,82 @@ __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, con
 // are then final too: lead > 0 means that bytes were cut after them, and a
 // byte is final once the next one is cut.
 //
-// lambda is lambda_raw unless the component's largest slope is small, so a
-// block may only stop once some block of its component (not necessarily this
-// one) has shown a slope that settles it; a block that has not been stopped
-// gives its largest slope as before.
+// lambda is lambda_raw unless the component's largest slope is small, and
+// then in proportion to that slope. So a block may only stop once some block
+// of its component (not necessarily this one) has shown a slope that settles
+// lambda, or a half, a quarter or an eighth as large: lambda is then at least
+// that share of lambda_raw, and the block, measured with it, may stop unless a
+// later pass could still raise the largest slope. A block that has not been
+// stopped gives its largest slope as before.
 //
 // The sums are f32: `slack` bounds their rounding against the f64 curve (a
 // term is within 1e-6 of its value, and each of at most 124 passes adds two
 // roundings of the lead).
 // On a 2550x3300 gray q85 page 33 % of the symbols are coded, and 37 k of the
 // longest block's 58 k.
+constexpr int kLevels = 4;
+struct StopState {
+  float lead[kLevels];  // with lambda_raw, a half, a quarter, an eighth of it
+  float slack, total;
+  uint32_t prev;  // bytes after the last pass (a header of 2 counts to the first one)
+};
 struct Stop {
   float unit, lambda, slope;
-  float lead, slack, total;
-  uint32_t prev;  // bytes after the last pass (a header of 2 counts to the first one)
-  uint32_t* flag;
+  StopState s;
+  uint32_t* flag;  // [k]: a slope of 2^-k times the one that settles lambda was seen
+  __device__ __forceinline__ void start(const T1Args& a, uint32_t b, const BlockDesc& d) {
+    const CompParam& cp = a.comps[d.comp_key];
+    unit = block_unit(a, b, d);
+    lambda = cp.lambda;
+    slope = cp.settled;
+    flag = a.settled + kLevels * d.comp_key;
+    s = StopState{};
+    s.prev = 0u - 2u;
+  }
+  __device__ __forceinline__ bool seen(int k) const { return reinterpret_cast<const volatile uint32_t*>(flag)[k] != 0u; }
   __device__ __forceinline__ void pass(uint32_t pos, float samples, int bitplane) {
+    if (!flag) return;
     const float gain = samples * unit * plane_energy(bitplane);
-    const float cost = lambda * (float)(pos - prev);
-    lead = fmaxf(0.0f, lead - gain + cost);
-    slack += 2e-5f * (gain + cost);
-    total += gain;
-    prev = pos;
-    if (flag && total * 0.9999f >= slope * (float)(pos + 2u)) *reinterpret_cast<volatile uint32_t*>(flag) = 1u;
+    float cost = lambda * (float)(pos - s.prev);
+    s.slack += 2e-5f * (gain + cost);
+    s.total += gain;
+    s.prev = pos;
+    float need = slope * (float)(pos + 2u);
+    #pragma unroll
+    for (int k = 0; k < kLevels; ++k) {
+      s.lead[k] = fmaxf(0.0f, s.lead[k] - gain + cost);
+      if (s.total * 0.9999f >= need) reinterpret_cast<volatile uint32_t*>(flag)[k] = 1u;
+      cost *= k == 0 ? 0.49999f : 0.5f;
+      need *= 0.5f;
+    }
   }
   __device__ __forceinline__ bool here(float remain) const {
-    return flag && remain + slack < lead && *reinterpret_cast<volatile uint32_t*>(flag) != 0u;
+    if (!flag) return false;
+    const float most = (s.total + remain) * 1.0001f;  // over bytes: the largest slope a later pass can give
+    float shown = slope * (float)(s.prev + 2u);
+    #pragma unroll
+    for (int k = 0; k < kLevels; ++k, shown *= 0.5f)
+      if (remain + s.slack < s.lead[k] && (k == 0 || most < shown) && seen(k)) return true;
+    return false;
   }
 };
+
+// What a block's coding goes on from in the second round, at the end of its
+// payload slot (which no block of pixels comes near).
+struct MqState {
+  Mq m;
+  StopState stop;
+  uint16_t context[kMqCtx];
+};
+constexpr uint32_t kStateBytes = 144;
+static_assert(sizeof(MqState) <= kStateBytes && kCtxNone <= kMqCtx, "the slot's end");
 
 // MQ-codes code-block b on the calling lane, or nothing when b is kNoBlock;
 // every lane of the warp calls. The lanes meet at every chunk (the vote):
 // left to themselves, a lane that ends a pass falls behind the others and
 // each would run the chunk code on its own.
 constexpr uint32_t kNoBlock = 0xffffffffu;
+template <int round>
 __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSmem& sm) {
   const uint32_t lane = threadIdx.x * 8u;
   BlockOut o{};
@@ -771,43 +860,43 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
   bool active = mbp > 0;
   BlockDesc d{};
   uint32_t base = 0;
+  int j = 0, modelled = 0;  // item; those of the round end before this one
   ItemRec r{};
   const uint4* src = nullptr;
-  uint4 c0 = make_uint4(0u, 0u, 0u, 0u), c1 = c0;
+  uint4 c0 = make_uint4(0u, 0u, 0u, 0u);
   if (active) {
     d = a.blocks[b];
+    modelled = round ? mbp : (int)a.nplanes[b];
+    j = round ? (int)a.nplanes[b] : 0;
     base = a.plane_base[b];
-    r = a.item_rec[base];
-    src = reinterpret_cast<const uint4*>(a.sym + (size_t)base * a.sym_slot);
-    c0 = src[0];
-    c1 = src[1];  // the slot and buffer are padded for these reads
+    r = a.item_rec[base + j];
+    src = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j) * a.sym_slot);
+    c0 = src[0];  // the slot and buffer are padded for these reads
     // contexts: state 0 except UNI 46, AGG 3, ZC 4 (src/mq/mod.rs:195-200)
     for (uint32_t c = 0; c < kMqCtx; ++c)
       ctx_at(sm, c * kCtxStride + lane) = c == kCtxNone ? make_uint2(kPadQe, 0u)
                                                         : mq_entry(c == kCtxUNI ? 92 : c == kCtxAGG ? 6 : c == 0 ? 8 : 0);
   }
   Stop stop{};
-  if (active && a.settled && !a.comps[d.comp_key].lossless) {
-    const CompParam& cp = a.comps[d.comp_key];
-    stop.unit = block_unit(a, b, d);
-    stop.lambda = cp.lambda;
-    stop.slope = cp.settled;
-    stop.prev = 0u - 2u;
-    stop.flag = a.settled + d.comp_key;
-  }
+  if (active && a.settled && !a.comps[d.comp_key].lossless) stop.start(a, b, d);
   uint8_t* const slot = a.out + d.out_off;
-  const uint8_t* const slot_end = slot + d.out_cap - 40;  // a chunk cuts at most 35 bytes
+  MqState* const state = reinterpret_cast<MqState*>(slot + d.out_cap - kStateBytes);
+  const uint8_t* const slot_end = slot + d.out_cap - kStateBytes - 40;  // a chunk cuts at most 35 bytes
   Mq m{1.0f, 0u, 12, 0u, slot};
   bool ovf = false;
   PassRec* pr = a.passes + d.pass_off;
+  if (round && active) {
+    m = state->m;
+    stop.s = state->stop;
+    for (uint32_t c = 0; c < kCtxNone; ++c) ctx_at(sm, c * kCtxStride + lane) = mq_entry(state->context[c] >> 4);
+    pr += 1 + 3 * (j - 1);
+  }
   // One flat loop over the chunks of all items (bit-planes); the next item's
-  // record and first chunks are fetched during the current item's last chunk.
+  // record and first chunk are fetched during the current item's last chunk.
   ItemRec rn = r;
-  uint4 n0 = c0, n1 = c0;
-  uint32_t nsym = r.n_cl;
-  int j = 0, k = 2;                     // item and pass (SP, MR, cleanup; the first item has only its cleanup)
-  uint32_t left = (r.n_cl + 15u) >> 4;  // chunks of the pass
-  uint32_t ahead = left;                // chunks of the item
+  uint4 n0 = c0;
+  uint32_t nsym = 0, left = 0, ahead = 0;  // symbols; chunks of the pass and of the item
+  int k = 0;                               // pass: SP, MR, cleanup (the first item has only its cleanup)
   auto record = [&] {                   // numbytes() after the pass
     const uint32_t pos = (uint32_t)(m.at - slot);
     const uint8_t bp = (uint8_t)r.bitplane;
@@ -820,18 +909,29 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
     ++pr;
     stop.pass(pos, k == 2 ? 0.85f * (float)r.ns_cl : (k == 0 ? (float)r.ns_sp : 0.25f * (float)r.sig_before), bp);
   };
-  bool stopped = false;
+  // the first pass of item j that has symbols
+  auto start_item = [&] {
+    nsym += r.n_sp + r.n_mr + r.n_cl;
+    ahead = ((r.n_sp + 15u) >> 4) + ((r.n_mr + 15u) >> 4) + ((r.n_cl + 15u) >> 4);
+    k = j == 0 ? 2 : 0;
+    left = ((j == 0 ? r.n_cl : r.n_sp) + 15u) >> 4;
+    while (k < 2 && left == 0) {
+      record();
+      ++k;
+      left = ((k == 1 ? r.n_mr : r.n_cl) + 15u) >> 4;
+    }
+  };
+  if (active) start_item();
+  bool stopped = false, unfinished = false;
   while (__any_sync(0xffffffffu, active)) {
     if (!active) continue;
-    if (ahead == 1 && j + 1 < mbp) {
+    if (ahead == 1 && j + 1 < modelled) {
       rn = a.item_rec[base + j + 1];
       const uint4* ns = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j + 1) * a.sym_slot);
       n0 = ns[0];
-      n1 = ns[1];
     }
     const uint4 q = c0;
-    c0 = c1;
-    c1 = src[2];  // 32 bytes ahead: inside the slot or the buffer's pad
+    c0 = src[1];  // 16 bytes ahead: inside the slot or the buffer's pad
     ++src;
     mq_chunk16(m, sm, lane, q);
     if (m.at > slot_end) {  // no room for another chunk: the block has failed
@@ -848,29 +948,29 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
       }
       if (left == 0) {  // the next item
         stopped = j + 1 < mbp && stop.here(r.remain);
-        if (++j == mbp || stopped) {
+        ++j;
+        unfinished = !stopped && j == modelled && j < mbp;
+        if (stopped || j == modelled) {
           active = false;
         } else {
           r = rn;
           src = reinterpret_cast<const uint4*>(a.sym + (size_t)(base + j) * a.sym_slot);
           c0 = n0;
-          c1 = n1;
-          nsym += r.n_sp + r.n_mr + r.n_cl;
-          ahead = ((r.n_sp + 15u) >> 4) + ((r.n_mr + 15u) >> 4) + ((r.n_cl + 15u) >> 4);
-          k = 0;
-          left = (r.n_sp + 15u) >> 4;
-          while (k < 2 && left == 0) {
-            record();
-            ++k;
-            left = ((k == 1 ? r.n_mr : r.n_cl) + 15u) >> 4;
-          }
+          start_item();
         }
       }
     }
   }
   if (mbp == 0) return;
   atomicAdd(a.sym_count, (unsigned long long)nsym);
-  if (stopped) {  // the coded passes stand, each with its bytes so far
+  if (unfinished && !ovf) {  // the second round goes on with the other bit-planes
+    state->m = m;
+    state->stop = stop.s;
+    for (uint32_t c = 0; c < kCtxNone; ++c) state->context[c] = (uint16_t)(ctx_at(sm, c * kCtxStride + lane).y & 0x7ffu);
+    a.unfinished[atomicAdd(a.counts + 2, 1u)] = b;
+    return;
+  }
+  if (stopped || unfinished) {  // the coded passes stand, each with its bytes so far
     o.npasses = (uint16_t)(1 + 3 * (j - 1));
     o.payload_len = (uint32_t)(m.at - slot);
     o.status = ovf ? 1 : 0;
@@ -893,14 +993,51 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
 }
 
 // Warp w codes blocks order[w * bpw + lane], lanes < bpw.
+template <int round>
 __global__ void __launch_bounds__(kMqWarps * 32) t1_mq_kernel(T1Args a, int bpw) {
   __shared__ MqSmem sm;
   load_mq_table(sm.table);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
-  const uint32_t slot = (blockIdx.x * kMqWarps + wid) * (uint32_t)bpw + (uint32_t)lane;
-  mq_code_block(a, lane < bpw && slot < a.nblocks ? a.mq_order[slot] : kNoBlock, sm);
+  if constexpr (round == 0) {
+    const uint32_t slot = (blockIdx.x * kMqWarps + wid) * (uint32_t)bpw + (uint32_t)lane;
+    mq_code_block<0>(a, lane < bpw && slot < a.nblocks ? a.mq_order[slot] : kNoBlock, sm);
+  } else {  // the blocks that t1_recheck_kernel listed, over a fixed grid
+    const uint32_t per_cta = kMqWarps * (uint32_t)bpw, count = a.counts[3];
+    for (uint32_t first = blockIdx.x * per_cta; first < count; first += gridDim.x * per_cta) {
+      const uint32_t slot = first + (uint32_t)(wid * bpw + lane);
+      mq_code_block<1>(a, lane < bpw && slot < count ? a.again[slot] : kNoBlock, sm);
+    }
+  }
+}
+
+// Between the rounds: of the blocks left unfinished, those that may stop
+// where they are (their component's lambda was not settled when they got
+// there) are done; the others are listed for the second round with their
+// remaining items.
+__global__ void t1_recheck_kernel(T1Args a) {
+  const uint32_t count = a.counts[2];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    const uint32_t b = a.unfinished[i];
+    const BlockDesc d = a.blocks[b];
+    BlockOut o = a.res[b];
+    uint8_t* const slot = a.out + d.out_off;
+    const MqState& state = *reinterpret_cast<const MqState*>(slot + d.out_cap - kStateBytes);
+    const uint32_t done = a.nplanes[b], all = o.mbp;
+    Stop stop;
+    stop.start(a, b, d);
+    stop.s = state.stop;
+    if (stop.here(a.item_rec[a.plane_base[b] + done - 1].remain)) {
+      o.npasses = (uint16_t)(1 + 3 * (done - 1));
+      o.payload_len = (uint32_t)(state.m.at - slot);
+      a.res[b] = o;
+      continue;
+    }
+    a.again[atomicAdd(a.counts + 3, 1u)] = b;
+    const uint32_t at = a.counts[0] + atomicAdd(a.counts + 1, all - done);
+    for (uint32_t j = done; j < all; ++j) a.items[at + j - done] = b << 6 | j;
+  }
 }
 
 }  // namespace
@@ -947,11 +1084,11 @@ void launch_t1_planes(const T1Args& a, cudaStream_t st) {
   t1_planes_kernel<<<(uint32_t)(((uint64_t)a.nblocks * 32 + 255) / 256), 256, 0, st>>>(a);
 }
 
-void launch_t1_model(const T1Args& a, int num_sms, cudaStream_t st) {
+void launch_t1_model(const T1Args& a, int num_sms, int round, cudaStream_t st) {
   if (a.nitems == 0) return;
   uint32_t need = (a.nitems + kModelWarps - 1) / kModelWarps;
-  uint32_t cap = (uint32_t)num_sms * 6 * 4;  // CTAs loop over the items
-  t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a);
+  uint32_t cap = (uint32_t)num_sms * (round ? 2 : 6 * 4);  // CTAs loop over the items; few are left for round 1
+  t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a, round);
 }
 
 // Automatic: as few blocks per warp as keep at most one warp on each of
@@ -963,11 +1100,17 @@ int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw) {
   return (int)std::min<uint32_t>(32u, std::max<uint32_t>(1u, (a.nblocks + warps - 1) / warps));
 }
 
-void launch_t1_mq(const T1Args& a, int num_sms, int bpw, cudaStream_t st) {
+void launch_t1_mq(const T1Args& a, int num_sms, int bpw, int round, cudaStream_t st) {
   if (a.nblocks == 0) return;
   bpw = mq_blocks_per_warp(a, num_sms, bpw);
-  const uint32_t per_cta = (uint32_t)bpw * kMqWarps;
-  t1_mq_kernel<<<(a.nblocks + per_cta - 1) / per_cta, kMqWarps * 32, 0, st>>>(a, bpw);
+  const uint32_t per_cta = (uint32_t)bpw * kMqWarps, all = (a.nblocks + per_cta - 1) / per_cta;
+  // the second round's blocks are few
+  if (round) t1_mq_kernel<1><<<(uint32_t)num_sms, kMqWarps * 32, 0, st>>>(a, std::min(bpw, 4));
+  else t1_mq_kernel<0><<<all, kMqWarps * 32, 0, st>>>(a, bpw);
+}
+
+void launch_t1_recheck(const T1Args& a, int num_sms, cudaStream_t st) {
+  t1_recheck_kernel<<<(uint32_t)num_sms, 128, 0, st>>>(a);
 }
 
 namespace {
@@ -978,7 +1121,7 @@ constexpr uint32_t kOrderBuckets = 1024;
 // slopes settle their components' lambda).
 __device__ __forceinline__ uint32_t order_bucket(const T1Args& a, uint32_t b) {
   if (a.blocks[b].orient == 0) return 0;
-  const uint32_t i0 = a.plane_base[b], i1 = a.plane_base[b + 1];
+  const uint32_t i0 = a.plane_base[b], i1 = i0 + a.nplanes[b];
   uint32_t n = 0;
   for (uint32_t i = i0; i < i1; ++i) {
     const ItemRec r = a.item_rec[i];

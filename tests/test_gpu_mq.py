@@ -91,3 +91,25 @@ def test_block_inspection_shows_every_pass(eng, orc):
     full = eng.counters()[2]
     eng.encode(px, w, h, 1, 60, 0)
     assert 0 < eng.counters()[2] < full
+
+
+def test_second_round_of_a_large_wave(eng, orc):
+    # a wave large enough that only the bit-planes foreseen are modelled at
+    # first, of contents that mislead the forecast: sparse outliers over much
+    # faint detail, chroma whose slopes never settle lambda, blocks of every
+    # size; each page against the oracle
+    pages, want = [], []
+    kinds = ["outlier", "faint", "texture", "checks"]
+    for i in range(28):
+        w, h, c = (1024, 768, 3) if i % 7 == 0 else (640 + 7 * i, 512 + 5 * i, 1 + 2 * (i % 2))
+        px = _stop_content(kinds[i % 4], w, h, c)
+        q = (85, 50, 97, 30, 100)[i % 5]
+        pages.append({"px": px, "w": w, "h": h, "ncomp": c, "quality": q, "fmt": 0})
+    pages = pages * 4
+    outs = eng.encode_batch(pages)
+    assert eng.counters()[0] > 48 * 152
+    for i in range(28):
+        p = pages[i]
+        ref = orc.encode(p["px"], p["w"], p["h"], p["ncomp"], p["quality"], 0)
+        for r in range(4):
+            assert outs[i + 28 * r] == ref, (i, r)
