@@ -1404,12 +1404,17 @@ struct DecodePage {
   uint64_t data_base = 0, plane_base = 0, px_base = 0;
 };
 
+// Bytes of a component's second largest resolution.
+size_t half_plane_bytes(const DecodePage& p) {
+  return p.L.levels > 0 ? (size_t)((p.L.width + 1) / 2) * ((p.L.height + 1) / 2) * 4 : 0;
+}
+
 uint64_t decode_device_bytes(const DecodePage& p, size_t nbytes) {
   // bytes, planes, tmp planes or masks, samples, code-blocks, jobs
   uint64_t masks = 0;
   for (const DecBlock& b : p.L.blocks) masks += 8ull * dec_mask_words(b.npasses);
-  return nbytes + p.npx * p.L.ncomp * 5 + std::max<uint64_t>(p.npx * p.L.ncomp * 4, masks) +
-         p.L.blocks.size() * sizeof(DecBlock) +
+  return nbytes + p.npx * p.L.ncomp * 4 + std::max<uint64_t>(p.npx, half_plane_bytes(p)) * p.L.ncomp +
+         std::max<uint64_t>(p.npx * p.L.ncomp * 4, masks) + p.L.blocks.size() * sizeof(DecBlock) +
          (uint64_t)(p.L.levels * p.L.ncomp + 1) * sizeof(IdwtJob) + sizeof(PixJob) + 1024;
 }
 
@@ -1445,36 +1450,36 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   // the blocks' masks lie where the inverse DWT's scratch planes come later
   const size_t planes_bytes = ((size_t)nplane * 4 + 15) & ~size_t(15);
   const size_t tmp_bytes = std::max<size_t>(planes_bytes, mask_words * 8);
-  // and the blocks' order where the samples do
-  const size_t px_bytes = std::max<size_t>((size_t)npxb, (blk.size() + 2048) * 4);
+  // and the blocks' order, and then every other level's samples, where the pixels do
+  size_t half_bytes = 0;
+  for (size_t i : ids) half_bytes += half_plane_bytes(pg[i]) * pg[i].L.ncomp;
+  const size_t px_bytes = std::max({(size_t)npxb, (blk.size() + 2048) * 4, half_bytes});
   if (!reserve(c, c->t2out, std::max<uint64_t>(nbytes, 16)) ||
       !reserve(c, c->recon, planes_bytes + tmp_bytes + px_bytes + 256))
     return JP2G_DECODE_FAILED;
   int32_t* planes = dptr<int32_t>(c->recon);
   int32_t* tmp = reinterpret_cast<int32_t*>(dptr<uint8_t>(c->recon) + planes_bytes);
   uint8_t* dpx = reinterpret_cast<uint8_t*>(tmp) + tmp_bytes;
-  std::vector<IdwtJob> jobs;
-  std::vector<uint32_t> first(maxl + 2, 0), rows(maxl + 2, 0), tiles(maxl + 2, 0);
-  for (int l = 1; l <= maxl; ++l) {
-    first[l] = (uint32_t)jobs.size();
+  std::vector<std::vector<IdwtJob>> by_level(maxl + 1);
+  {
+    uint8_t* other = dpx;
     for (size_t i : ids) {
       const DecodePage& p = pg[i];
-      if (p.L.levels < l) continue;
-      const uint32_t rw = (uint32_t)p.L.ladder[l].first, rh = (uint32_t)p.L.ladder[l].second;
       for (int comp = 0; comp < p.L.ncomp; ++comp) {
-        IdwtJob j{};
-        j.plane = planes + p.plane_base + (uint64_t)comp * p.npx;
-        j.tmp = tmp + p.plane_base + (uint64_t)comp * p.npx;
-        j.stride = p.L.width;
-        j.rw = rw;
-        j.rh = rh;
-        j.reversible = p.L.reversible ? 1u : 0u;
-        j.row_base = rows[l];
-        j.tile_base = tiles[l];
-        rows[l] += rh;
-        tiles[l] += ((rw + 31) / 32) * ((rh + kIdwtTileRows - 1) / kIdwtTileRows);
-        jobs.push_back(j);
+        const uint64_t at = p.plane_base + (uint64_t)comp * p.npx;
+        idwt_jobs(planes + at, tmp + at, other, p.L.ladder.data(), p.L.levels, p.L.reversible, &by_level);
+        other += half_plane_bytes(p);
       }
+    }
+  }
+  std::vector<IdwtJob> jobs;
+  std::vector<uint32_t> first(maxl + 2, 0), tiles(maxl + 2, 0);
+  for (int l = 1; l <= maxl; ++l) {
+    first[l] = (uint32_t)jobs.size();
+    for (IdwtJob j : by_level[l]) {
+      j.tile_base = tiles[l];
+      tiles[l] += idwt_tiles(j.rw, j.rh);
+      jobs.push_back(j);
     }
   }
   first[maxl + 1] = (uint32_t)jobs.size();
@@ -1483,7 +1488,7 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   for (size_t i : ids) {
     const DecodePage& p = pg[i];
     PixJob j{};
-    j.planes = planes + p.plane_base;
+    j.planes = (p.L.levels > 0 ? tmp : planes) + p.plane_base;
     j.px = dpx + p.px_base;
     j.npx = p.npx;
     j.pix_base = total_px;
@@ -1514,7 +1519,7 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
     return JP2G_DECODE_FAILED;
   launch_t1_decode(dblk, (uint32_t)blk.size(), dptr<uint8_t>(c->t2out), reinterpret_cast<unsigned long long*>(tmp),
                    planes, reinterpret_cast<uint32_t*>(dpx), c->stream);
-  for (int l = 1; l <= maxl; ++l) launch_idwt_level(djobs + first[l], first[l + 1] - first[l], rows[l], tiles[l], c->stream);
+  for (int l = 1; l <= maxl; ++l) launch_idwt_level(djobs + first[l], first[l + 1] - first[l], tiles[l], c->stream);
   launch_dec_pixels(dpix, (uint32_t)pix.size(), total_px, c->stream);
   if (!cuda_ok(c, cudaGetLastError(), "decode kernels")) return JP2G_DECODE_FAILED;
   if (ids.size() >= 8) {

@@ -198,17 +198,25 @@ struct DecodeLayout {
 // code-blocks whose segment has zero bytes (the JP2G_DECODE_* flags).
 bool parse_codestream(const uint8_t* bytes, size_t n, int flags, DecodeLayout* out, Failure* err);
 
-// One component of one page at one inverse-DWT level: its planes hold
-// int32 (5/3) or f32 (9/7) samples, rows `stride` apart; the level's
-// rw x rh region is transformed rows first (plane -> tmp), then columns
-// (tmp -> plane). row_base / tile_base: the job's first global row and
-// first 32-column tile in the level's launch.
+// One component of one page at one inverse-DWT level: int32 (5/3) or f32
+// (9/7) samples; the level's LL band (the level below, whole), its other
+// bands (where they lie in the component's plane) and its rw x rh samples.
+// tile_base: the job's first tile in the level's launch.
 struct IdwtJob {
-  void* plane;
-  void* tmp;
-  uint32_t stride, rw, rh, reversible;
-  uint32_t row_base, tile_base;
+  const void* ll;
+  const void* detail;
+  void* out;
+  uint32_t ll_pitch, detail_pitch, out_pitch;
+  uint32_t rw, rh, reversible;
+  uint32_t tile_base;
 };
+constexpr int kIdwtTileCols = 128, kIdwtTileRows = 64;
+uint32_t idwt_tiles(uint32_t rw, uint32_t rh);
+// Adds a component's jobs to by_level[1..levels] (tile_base unset): plane
+// holds its bands, ladder[0..levels] the resolutions' sizes; the samples come
+// to `out`, by way of `other` (room for the second largest resolution).
+void idwt_jobs(void* plane, void* out, void* other, const std::pair<int, int>* ladder, int levels, bool reversible,
+               std::vector<std::vector<IdwtJob>>* by_level);
 // One page's final samples: inverse RCT/ICT (when mct and 3 components),
 // level shift and clamp into interleaved 8-bit samples.
 struct PixJob {
@@ -226,9 +234,7 @@ JP2G_HD uint32_t dec_mask_words(uint32_t npasses) { return npasses ? 64 * (dec_p
 void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, unsigned long long* masks,
                       int32_t* planes, uint32_t* scratch, cudaStream_t st);
 // One inverse-DWT level for njobs jobs (recon.cu).
-void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_rows, uint32_t total_tiles,
-                       cudaStream_t st);
-constexpr int kIdwtTileRows = 64;  // rows per column tile of launch_idwt_level
+void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_tiles, cudaStream_t st);
 void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint64_t total_px, cudaStream_t st);
 bool upload_decode_tables(const uint8_t* zc, const uint8_t* sc, const uint8_t* spb, const uint32_t* mq);
 
@@ -254,6 +260,7 @@ struct ReconArgs {
   const uint8_t* px;  // the page's interleaved pixels on the device
   float* plane;       // ncomp planes of width * height
   float* tmp;         // ncomp planes of scratch
+  float* samples;     // the decoded samples, ncomp planes (set by launch_recon)
   IdwtJob* jobs;      // device room for ncomp * levels inverse-DWT jobs
   float* luma_orig;
   float* luma_dec;
@@ -263,7 +270,7 @@ struct ReconArgs {
 // Dequantisation of the retained bit-planes, inverse 9/7 per component
 // (ladder[0..levels], index 0 the smallest resolution), colour and the two
 // sums of the metrics.
-void launch_recon(const ReconArgs& r, const std::pair<int, int>* ladder, int levels, cudaStream_t st);
+void launch_recon(ReconArgs r, const std::pair<int, int>* ladder, int levels, cudaStream_t st);
 
 // Packs the retained payload bytes of every block, in work-list order, into
 // `dst`; offsets[b] receives the byte offset of block b and offsets[n] the

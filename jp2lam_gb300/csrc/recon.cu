@@ -13,6 +13,7 @@
 // the oracle's; only the f64 sums run in a different order.
 #include <cuda_runtime.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "jp2g_internal.h"
@@ -67,143 +68,151 @@ __device__ __forceinline__ float lifted(float x, float c, float l, float rr) {
   return __fadd_rn(x, __fmul_rn(c, __fadd_rn(l, rr)));
 }
 
-// The job holding global index g (rows or tiles) of a level's launch.
-__device__ __forceinline__ const IdwtJob& job_of(const IdwtJob* jobs, uint32_t njobs, uint32_t g, bool tiles) {
+// The job holding tile g of a level's launch.
+__device__ __forceinline__ const IdwtJob& job_of(const IdwtJob* jobs, uint32_t njobs, uint32_t g) {
   uint32_t lo = 0, hi = njobs;
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
-    if ((tiles ? jobs[mid].tile_base : jobs[mid].row_base) <= g) lo = mid;
+    if (jobs[mid].tile_base <= g) lo = mid;
     else hi = mid;
   }
   return jobs[lo];
 }
 
-// Inverse 1-D transform of one row (rw samples, low half first) of a job's
-// plane into the same row of its tmp, interleaved: a warp per row, each
-// lifting step's positions in parallel.
-//  9/7 (src/dwt/irrev97.rs:639-796): scale by K / 1/K, then the four
-//    lifting steps x[j] += c (x[j-1] + x[j+1]) over whole-sample symmetric
-//    extension, each rounded as written.
+// One level of the inverse 2-D transform over 128x64 tiles, rows then
+// columns:
+//  9/7 (src/dwt/irrev97.rs:639-796): scale by K / 1/K, then four lifting
+//    steps x[j] += c (x[j-1] + x[j+1]), each rounded as written;
 //  5/3 (src/dwt/rev53.rs:96-129, 419-497): even samples
-//    s[i] - ((d[i-1] + d[i] + 2) >> 2) with the edges clamped, then odd
-//    samples d[i] + ((e[i] + e[i+1]) >> 1), or d[i] + e[i] at the right edge.
-__global__ void idwt_rows_kernel(const IdwtJob* jobs, uint32_t njobs, uint32_t total_rows) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (g >= total_rows) return;
-  const IdwtJob& jb = job_of(jobs, njobs, g, false);
-  const uint32_t y = g - jb.row_base;
-  const int n = (int)jb.rw, sn = (n + 1) / 2, dn = n - sn;
-  if (jb.reversible) {
-    const int32_t* x = static_cast<const int32_t*>(jb.plane) + (size_t)y * jb.stride;
-    int32_t* t = static_cast<int32_t*>(jb.tmp) + (size_t)y * jb.stride;
-    if (n == 1) {
-      if (lane == 0) t[0] = x[0];
-      return;
-    }
-    for (int i = lane; i < sn; i += 32) {
-      const int l = min(max(i - 1, 0), dn - 1), r = min(i, dn - 1);
-      t[2 * i] = x[i] - ((x[sn + l] + x[sn + r] + 2) >> 2);
-    }
-    __syncwarp();
-    for (int i = lane; i < dn; i += 32)
-      t[2 * i + 1] = i + 1 < sn ? x[sn + i] + ((t[2 * i] + t[2 * i + 2]) >> 1) : x[sn + i] + t[2 * i];
-  } else {
-    const float* x = static_cast<const float*>(jb.plane) + (size_t)y * jb.stride;
-    float* t = static_cast<float*>(jb.tmp) + (size_t)y * jb.stride;
-    if (n == 1) {
-      if (lane == 0) t[0] = __fmul_rn(x[0], kRK);
-      return;
-    }
-    for (int i = lane; i < n; i += 32) {
-      const float v = i & 1 ? x[sn + (i >> 1)] : x[i >> 1];
-      t[i] = __fmul_rn(v, i & 1 ? kRInvK : kRK);
-    }
-    __syncwarp();
-    const float c[4] = {-kRDelta, -kRGamma, -kRBeta, -kRAlpha};
-    #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      for (int j = (s & 1) + 2 * lane; j < n; j += 64)
-        t[j] = lifted(t[j], c[s], t[sym_at(j - 1, n)], t[sym_at(j + 1, n)]);
-      __syncwarp();
-    }
-  }
+//    s[i] - ((d[i-1] + d[i] + 2) >> 2), then odd samples
+//    d[i] + ((e[i] + e[i+1]) >> 1).
+// A CTA loads a tile and 4 samples around it, interleaving the bands,
+// positions beyond the region's ends from their mirror images: whole-sample
+// symmetric extension commutes with each lifting step (a position and its
+// mirror have the same parity and mirrored neighbours, and l + r = r + l
+// exactly), so every output equals whole-row and whole-column lifting; the 5/3
+// edge clamps are the same extension. A thread lifts 40 samples of a row, then
+// of a column, in registers.
+// A level is read once and written once (the samples beside a tile come from
+// L2), into a buffer of its own, as neighbouring tiles still read the old
+// bands. Bound by the latency of the loads at 4 CTAs per SM: 12 sRGB 2550x3300
+// pages, all levels, 0.93 ms, the last one 0.66 (3.7 TB/s); a warp per row
+// lifting in global memory, then column tiles, took 3.9, and loading sample by
+// sample in place of pairs of columns 2.1.
+constexpr int kTileW = kIdwtTileCols, kTileH = kIdwtTileRows, kHalo = 4;
+constexpr int kSpanW = kTileW + 2 * kHalo, kSpanH = kTileH + 2 * kHalo, kPitch = kSpanW + 2;
+constexpr int kJob = 40;  // samples of a register job: 32 outputs and a halo
+constexpr int kIdwtThreads = 288, kWarps = kIdwtThreads / 32;
+static_assert(kSpanH % kWarps == 0 && kSpanW / 2 > 64 && kSpanW / 2 <= 96, "rows and pairs of the load");
+static_assert(kPitch % 4 == 2, "pairs are aligned and 32 rows' pairs lie in different banks");
+static_assert(kIdwtThreads == kSpanH * (kTileW / 32) && kIdwtThreads >= kTileW * (kTileH / 32), "a job per thread");
+
+template <class T>
+struct alignas(8) Pair {
+  T x, y;
+};
+
+// Outputs x[4..35] from x[1..39] (9/7) or x[3..37] (5/3), in place. single:
+// the region is one sample long (only scaled).
+__device__ __forceinline__ void unlift(float (&x)[kJob], bool single) {
+  #pragma unroll
+  for (int i = 1; i < kJob; ++i) x[i] = __fmul_rn(x[i], i & 1 ? kRInvK : kRK);
+  if (single) return;
+  #pragma unroll
+  for (int i = 2; i <= 38; i += 2) x[i] = lifted(x[i], -kRDelta, x[i - 1], x[i + 1]);
+  #pragma unroll
+  for (int i = 3; i <= 37; i += 2) x[i] = lifted(x[i], -kRGamma, x[i - 1], x[i + 1]);
+  #pragma unroll
+  for (int i = 4; i <= 36; i += 2) x[i] = lifted(x[i], -kRBeta, x[i - 1], x[i + 1]);
+  #pragma unroll
+  for (int i = 5; i <= 35; i += 2) x[i] = lifted(x[i], -kRAlpha, x[i - 1], x[i + 1]);
+}
+__device__ __forceinline__ void unlift(int32_t (&x)[kJob], bool single) {
+  if (single) return;
+  #pragma unroll
+  for (int i = 4; i <= 36; i += 2) x[i] -= (x[i - 1] + x[i + 1] + 2) >> 2;
+  #pragma unroll
+  for (int i = 5; i <= 35; i += 2) x[i] += (x[i - 1] + x[i + 1]) >> 1;
 }
 
-// Inverse 1-D transform of the columns of a job's tmp (low half of the rows
-// first) into its plane, interleaved. A CTA takes 32 columns x 64 output
-// rows and the 4 (9/7) or 2 (5/3) rows of halo each side in shared memory;
-// positions beyond the column's ends are loaded from their mirror images.
-// Whole-sample symmetric extension commutes with each lifting step (a
-// position and its mirror have the same parity and mirrored neighbours, and
-// l + r = r + l exactly), so every kept row equals the reference's value;
-// the 5/3 edge clamps are the same extension. The halo rows, whose outer
-// neighbours are missing, are not written.
-constexpr int kTileRows = kIdwtTileRows;
-__global__ void __launch_bounds__(256) idwt_cols_kernel(const IdwtJob* jobs, uint32_t njobs, uint32_t total_tiles) {
-  __shared__ float sh[(kTileRows + 8) * 33];
-  const uint32_t g = blockIdx.x;
-  if (g >= total_tiles) return;
-  const IdwtJob& jb = job_of(jobs, njobs, g, true);
-  const uint32_t tiles_x = (jb.rw + 31) / 32, t = g - jb.tile_base;
-  const int tx = (int)(t % tiles_x), ty = (int)(t / tiles_x);
-  const int lane = threadIdx.x & 31, ry = threadIdx.x >> 5;  // 8 row groups
-  const int x = tx * 32 + lane;
-  const bool col = x < (int)jb.rw;
-  const int n = (int)jb.rh, sn = (n + 1) / 2;
-  const size_t stride = jb.stride;
-  const int r0 = ty * kTileRows;
-  if (jb.reversible) {
-    const int32_t* src = static_cast<const int32_t*>(jb.tmp) + x;
-    int32_t* dst = static_cast<int32_t*>(jb.plane) + x;
-    int32_t* si = reinterpret_cast<int32_t*>(sh);
-    if (n == 1) {
-      if (ry == 0 && col) dst[0] = src[0];
-      return;
-    }
-    constexpr int halo = 2, m = kTileRows + 2 * halo;
-    for (int li = ry; li < m; li += 8) {
-      const int p = sym_at(r0 - halo + li, n);
-      si[li * 33 + lane] = col ? src[(size_t)(p & 1 ? sn + (p >> 1) : p >> 1) * stride] : 0;
-    }
-    __syncthreads();
-    for (int li = 1 + ry; li < m - 1; li += 8)  // even positions (r0 is even)
-      if (!(li & 1)) si[li * 33 + lane] -= (si[(li - 1) * 33 + lane] + si[(li + 1) * 33 + lane] + 2) >> 2;
-    __syncthreads();
-    for (int li = 1 + ry; li < m - 1; li += 8)
-      if (li & 1) si[li * 33 + lane] += (si[(li - 1) * 33 + lane] + si[(li + 1) * 33 + lane]) >> 1;
-    __syncthreads();
-    for (int li = halo + ry; li < halo + kTileRows; li += 8) {
-      const int i = r0 + li - halo;
-      if (col && i < n) dst[(size_t)i * stride] = si[li * 33 + lane];
-    }
-  } else {
-    const float* src = static_cast<const float*>(jb.tmp) + x;
-    float* dst = static_cast<float*>(jb.plane) + x;
-    if (n == 1) {
-      if (ry == 0 && col) dst[0] = __fmul_rn(src[0], kRK);
-      return;
-    }
-    constexpr int halo = 4, m = kTileRows + 2 * halo;
-    for (int li = ry; li < m; li += 8) {
-      const int p = sym_at(r0 - halo + li, n);
-      const float v = col ? src[(size_t)(p & 1 ? sn + (p >> 1) : p >> 1) * stride] : 0.0f;
-      sh[li * 33 + lane] = __fmul_rn(v, p & 1 ? kRInvK : kRK);
-    }
-    __syncthreads();
-    const float c[4] = {-kRDelta, -kRGamma, -kRBeta, -kRAlpha};
+template <class T>
+__device__ __forceinline__ void idwt_tile(const IdwtJob& jb, int x0, int y0, T* s) {
+  const int tid = threadIdx.x, rw = (int)jb.rw, rh = (int)jb.rh;
+  const int lw = (rw + 1) / 2, lh = (rh + 1) / 2;
+  {
+    // a warp per row: a lane's pairs of columns stay the same
+    const T* ll = static_cast<const T*>(jb.ll);
+    const T* detail = static_cast<const T*>(jb.detail);
+    const int lane = tid & 31, warp = tid >> 5;
+    int even[3], odd[3];  // where the pairs' samples lie in a row of bands
+    bool mirrored[3];     // an odd position of a single column takes the even sample
     #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      for (int li = 1 + ry; li < m - 1; li += 8)
-        if ((li & 1) == (s & 1))
-          sh[li * 33 + lane] = lifted(sh[li * 33 + lane], c[s], sh[(li - 1) * 33 + lane], sh[(li + 1) * 33 + lane]);
-      __syncthreads();
+    for (int k = 0; k < 3; ++k) {
+      const int j = x0 - kHalo + 2 * min(lane + 32 * k, kSpanW / 2 - 1);
+      const int q = sym_at(j + 1, rw);
+      even[k] = sym_at(j, rw) >> 1;
+      odd[k] = (q & 1 ? lw : 0) + (q >> 1);
+      mirrored[k] = !(q & 1);
     }
-    for (int li = halo + ry; li < halo + kTileRows; li += 8) {
-      const int i = r0 + li - halo;
-      if (col && i < n) dst[(size_t)i * stride] = sh[li * 33 + lane];
+    #pragma unroll 4
+    for (int i = 0; i < kSpanH / kWarps; ++i) {
+      const int li = i * kWarps + warp, p = sym_at(y0 - kHalo + li, rh);
+      const T* high = detail + (size_t)((p & 1 ? lh : 0) + (p >> 1)) * jb.detail_pitch;
+      const T* low = p & 1 ? high : ll + (size_t)(p >> 1) * jb.ll_pitch;
+      #pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (k < 2 || lane < kSpanW / 2 - 64) {
+          Pair<T> v;
+          v.x = low[even[k]];
+          v.y = (mirrored[k] ? low : high)[odd[k]];
+          *reinterpret_cast<Pair<T>*>(s + li * kPitch + 2 * (lane + 32 * k)) = v;
+        }
     }
   }
+  __syncthreads();
+  T x[kJob];
+  {
+    const int row = tid % kSpanH, first = 32 * (tid / kSpanH);
+    T* at = s + row * kPitch + first;
+    #pragma unroll
+    for (int i = 0; i < kJob; i += 2) {
+      const Pair<T> v = *reinterpret_cast<const Pair<T>*>(at + i);
+      x[i] = v.x;
+      x[i + 1] = v.y;
+    }
+    __syncthreads();
+    unlift(x, rw == 1);
+    #pragma unroll
+    for (int i = kHalo; i < kHalo + 32; i += 2) *reinterpret_cast<Pair<T>*>(at + i) = Pair<T>{x[i], x[i + 1]};
+    const int end = rw - 1 - (x0 - kHalo + first);
+    if (std::is_same<T, int32_t>::value && rw > 1 && !(rw & 1) && end >= kHalo && end < kHalo + 32) {
+      // a row's last sample adds its even neighbour itself: half of its double
+      // differs where a sample is too large to be doubled
+      const int32_t e = at[end - 1];
+      at[end] += e - ((int32_t)(2u * (uint32_t)e) >> 1);
+    }
+  }
+  __syncthreads();
+  if (tid >= kTileW * (kTileH / 32)) return;
+  const int cx = x0 + tid % kTileW, first = 32 * (tid / kTileW);
+  const T* at = s + first * kPitch + kHalo + tid % kTileW;
+  #pragma unroll
+  for (int i = 1; i < kJob; ++i) x[i] = at[i * kPitch];
+  unlift(x, rh == 1);
+  if (cx >= rw) return;
+  T* out = static_cast<T*>(jb.out) + (size_t)(y0 + first) * jb.out_pitch + cx;
+  #pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (y0 + first + i < rh) out[(size_t)i * jb.out_pitch] = x[kHalo + i];
+}
+
+__global__ void __launch_bounds__(kIdwtThreads) idwt_kernel(const IdwtJob* jobs, uint32_t njobs) {
+  __shared__ alignas(16) float s[kSpanH * kPitch];
+  const IdwtJob& jb = job_of(jobs, njobs, blockIdx.x);
+  const uint32_t tiles_x = (jb.rw + kTileW - 1) / kTileW, t = blockIdx.x - jb.tile_base;
+  const int x0 = (int)(t % tiles_x) * kTileW, y0 = (int)(t / tiles_x) * kTileH;
+  if (jb.reversible) idwt_tile(jb, x0, y0, reinterpret_cast<int32_t*>(s));
+  else idwt_tile(jb, x0, y0, s);
 }
 
 __device__ __forceinline__ float clamp255(float v) { return fminf(fmaxf(v, 0.0f), 255.0f); }
@@ -228,14 +237,14 @@ __global__ void recon_pixels_kernel(ReconArgs r) {
   double e = 0.0;
   if (i < n) {
     if (r.ncomp == 1) {
-      const float dec = clamp255(__fadd_rn(r.plane[i], 128.0f));
+      const float dec = clamp255(__fadd_rn(r.samples[i], 128.0f));
       const float orig = (float)r.px[i];
       const float diff = __fadd_rn(dec, -orig);
       e = (double)__fmul_rn(diff, diff);
       r.luma_dec[i] = dec;
       r.luma_orig[i] = orig;
     } else {
-      const float yc = r.plane[i], cb = r.plane[n + i], cr = r.plane[2 * n + i];
+      const float yc = r.samples[i], cb = r.samples[n + i], cr = r.samples[2 * n + i];
       // inverse ICT (ISO/IEC 15444-1 G.2) and level shift, backend.rs:392-400
       const float R = clamp255(__fadd_rn(__fadd_rn(yc, __fmul_rn(1.402f, cr)), 128.0f));
       const float G = clamp255(
@@ -332,11 +341,41 @@ __global__ void dec_pixels_kernel(const PixJob* jobs, uint32_t njobs, uint64_t t
 
 }  // namespace
 
-void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_rows, uint32_t total_tiles,
-                       cudaStream_t st) {
-  if (njobs == 0) return;
-  if (total_rows) idwt_rows_kernel<<<(unsigned)(((size_t)total_rows * 32 + 255) / 256), 256, 0, st>>>(jobs, njobs, total_rows);
-  if (total_tiles) idwt_cols_kernel<<<total_tiles, 256, 0, st>>>(jobs, njobs, total_tiles);
+uint32_t idwt_tiles(uint32_t rw, uint32_t rh) {
+  return ((rw + kIdwtTileCols - 1) / kIdwtTileCols) * ((rh + kIdwtTileRows - 1) / kIdwtTileRows);
+}
+
+// Jobs of one component, smallest level first. Level l reads its LL band
+// from where level l - 1 left it (the plane's own corner at first) and its
+// other bands from the plane, and writes whole samples to `out` or `other` in
+// turn, so that the last level's come to `out`.
+void idwt_jobs(void* plane, void* out, void* other, const std::pair<int, int>* ladder, int levels, bool reversible,
+               std::vector<std::vector<IdwtJob>>* by_level) {
+  const uint32_t width = (uint32_t)ladder[levels].first;
+  const void* ll = plane;
+  uint32_t ll_pitch = width;
+  for (int l = 1; l <= levels; ++l) {
+    const uint32_t rw = (uint32_t)ladder[l].first, rh = (uint32_t)ladder[l].second;
+    if (rw == 0 || rh == 0) continue;
+    IdwtJob j{};
+    j.detail = plane;
+    j.detail_pitch = width;
+    j.ll = ll;
+    j.ll_pitch = ll_pitch;
+    j.out = (levels - l) % 2 == 0 ? out : other;
+    j.out_pitch = rw;
+    j.rw = rw;
+    j.rh = rh;
+    j.reversible = reversible ? 1u : 0u;
+    ll = j.out;
+    ll_pitch = rw;
+    (*by_level)[l].push_back(j);
+  }
+}
+
+void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_tiles, cudaStream_t st) {
+  if (njobs == 0 || total_tiles == 0) return;
+  idwt_kernel<<<total_tiles, kIdwtThreads, 0, st>>>(jobs, njobs);
 }
 
 void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint64_t total_px, cudaStream_t st) {
@@ -344,36 +383,32 @@ void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint64_t total_px, cu
   dec_pixels_kernel<<<(unsigned)((total_px + 255) / 256), 256, 0, st>>>(jobs, njobs, total_px);
 }
 
-void launch_recon(const ReconArgs& r, const std::pair<int, int>* ladder, int levels, cudaStream_t st) {
+void launch_recon(ReconArgs r, const std::pair<int, int>* ladder, int levels, cudaStream_t st) {
   const size_t n = (size_t)r.width * r.height;
   cudaMemsetAsync(r.plane, 0, n * r.ncomp * sizeof(float), st);
   cudaMemsetAsync(r.stats, 0, 2 * sizeof(double), st);
   if (r.nblocks) recon_dequant_kernel<<<(unsigned)(((size_t)r.nblocks * 32 + 255) / 256), 256, 0, st>>>(r);
-  // every component of a level in one launch, each with its own tmp plane
+  // every component of a level in one launch; the levels alternate between
+  // tmp and the luma planes, which are made only afterwards, and end in tmp
+  std::vector<std::vector<IdwtJob>> by_level(levels + 1);
+  const size_t half = (size_t)((r.width + 1) / 2) * ((r.height + 1) / 2);
+  for (int c = 0; c < r.ncomp; ++c)
+    idwt_jobs(r.plane + (size_t)c * n, r.tmp + (size_t)c * n, r.luma_orig + (size_t)c * half, ladder, levels, false,
+              &by_level);
   std::vector<IdwtJob> jobs;
-  std::vector<uint32_t> first(levels + 2, 0), rows(levels + 2, 0), tiles(levels + 2, 0);
+  std::vector<uint32_t> first(levels + 2, 0), tiles(levels + 1, 0);
   for (int l = 1; l <= levels; ++l) {
     first[l] = (uint32_t)jobs.size();
-    const uint32_t rw = (uint32_t)ladder[l].first, rh = (uint32_t)ladder[l].second;
-    for (int c = 0; c < r.ncomp && rw && rh; ++c) {
-      IdwtJob j{};
-      j.plane = r.plane + (size_t)c * n;
-      j.tmp = r.tmp + (size_t)c * n;
-      j.stride = r.width;
-      j.rw = rw;
-      j.rh = rh;
-      j.reversible = 0;
-      j.row_base = rows[l];
+    for (IdwtJob j : by_level[l]) {
       j.tile_base = tiles[l];
-      rows[l] += rh;
-      tiles[l] += ((rw + 31) / 32) * ((rh + kIdwtTileRows - 1) / kIdwtTileRows);
+      tiles[l] += idwt_tiles(j.rw, j.rh);
       jobs.push_back(j);
     }
   }
   first[levels + 1] = (uint32_t)jobs.size();
   if (!jobs.empty()) cudaMemcpyAsync(r.jobs, jobs.data(), jobs.size() * sizeof(IdwtJob), cudaMemcpyHostToDevice, st);
-  for (int l = 1; l <= levels; ++l)
-    launch_idwt_level(r.jobs + first[l], first[l + 1] - first[l], rows[l], tiles[l], st);
+  for (int l = 1; l <= levels; ++l) launch_idwt_level(r.jobs + first[l], first[l + 1] - first[l], tiles[l], st);
+  r.samples = levels > 0 ? r.tmp : r.plane;
   recon_pixels_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(r);
   const int nb8 = (int)(r.width / 8) * (int)(r.height / 8);
   if (nb8 > 0) recon_ssim_kernel<<<(unsigned)((nb8 + 255) / 256), 256, 0, st>>>(r);

@@ -220,3 +220,17 @@ def test_decode_at_the_edges_of_stripes_and_halves(eng, orc, w, h, q):
     assert np.array_equal(eng.decode(data, accept_empty_segments=True)[0], want)
     if q == 100:
         assert np.array_equal(want, px)
+
+
+@pytest.mark.parametrize("q", [100, 75])
+@pytest.mark.parametrize("w,h", [(127, 63), (128, 64), (129, 65), (257, 130), (132, 61), (1, 200), (300, 1), (2, 3)])
+def test_inverse_transform_at_the_edges_of_tiles(eng, orc, w, h, q):
+    # tiles of 128 x 64 samples that are whole, that end one sample early and
+    # that hold one row or column, each level ending in either buffer
+    px = np.random.default_rng(w * 977 + h).integers(0, 256, w * h * 3, dtype=np.uint8)
+    data = eng.encode(px, w, h, 3, q, 0)
+    flags = dict(accept_empty_segments=True, rct_chroma_extra_bitplane=q == 100)
+    want = orc.decode(data, **flags)[3]
+    assert np.array_equal(eng.decode(data, **flags)[0], want)
+    pair = eng.decode_batch([data, data], **flags)
+    assert all(np.array_equal(np.asarray(p[0]), want) for p in pair)
