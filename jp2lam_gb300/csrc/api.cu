@@ -120,6 +120,9 @@ struct jp2g_ctx {
   // current one computes), alternating between px and px2; its DWT waits
   // on ev_up
   cudaStream_t copy_stream = nullptr;
+  // part 0 of a split wave is coded on mq_stream, whose CTAs start before others
+  cudaStream_t mq_stream = nullptr;
+  cudaEvent_t ev_mq[2] = {};
   cudaEvent_t ev_up[2] = {};
   uint8_t* wave_px = nullptr;  // the current wave's device pixels
   float stage_ms[kNumStages + 4] = {};
@@ -893,7 +896,19 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
       !cuda_ok(c, cudaStreamSynchronize(c->stream), "tier-1 analysis"))
     return kEncodeFailed;
   ta.nitems = *reinterpret_cast<uint32_t*>(c->hcount.p);
-  if (!reserve(c, c->items, std::max<size_t>(ta.nitems, 1) * 4) ||
+  // A large wave's blocks fill the chip's lanes many times over.
+  const bool large = nb > (uint32_t)c->num_sms * 48u;
+  // Modelling keeps the chip busy and coding ends in a few long chains, so
+  // the long ones go first and run beside the modelling of the others. In a
+  // small wave these are the chains that the call waits for (three quarters of
+  // the longest and more); a large one's coding takes long after them too, and
+  // more of it goes first. With eight blocks per SM or fewer, modelling is too
+  // short to gain anything (48 pages of 256x256: 2.08 ms whole, 2.11 split). Modelling and coding, ms, with 3/4, 1/2 and 5/12 in
+  // part 0 and without the split: 2550x3300 sRGB page 1.92, 2.01, 2.07 and 2.30;
+  // 5100x6600 sRGB lossless 3.45, 3.24, 3.40 and 3.81; 24 sRGB pages -, 5.93,
+  // 5.53 and 7.1.
+  const bool split = nb > (uint32_t)c->num_sms * 8u;
+  if (!reserve(c, c->items, std::max<size_t>(ta.nitems, 1) * 4 * (split ? 2 : 1)) ||
       !reserve(c, c->itemrec, std::max<size_t>(ta.nitems, 1) * sizeof(ItemRec)) ||
       !reserve(c, c->planes, std::max<size_t>(ta.nitems, 1) * 1024) ||
       !reserve(c, c->signs, std::max<size_t>(nb, 1) * 512) ||
@@ -904,32 +919,54 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   ta.planes = dptr<uint32_t>(c->planes);
   ta.signs = dptr<uint32_t>(c->signs);
   ta.sym = dptr<uint8_t>(c->sym);
+  static_assert((4 + kCounts) * 4 <= 64, "counts");
   ta.counts = dptr<uint32_t>(c->stats) + 4;
   // Modelling every bit-plane costs a small wave less than a second round;
   // for large ones it is the largest stage, and two thirds of it would be for
   // bit-planes that are never coded.
-  ta.foresee = ta.settled && nb > (uint32_t)c->num_sms * 48u &&
+  ta.foresee = ta.settled && large &&
                std::any_of(live.begin(), live.end(), [](const PageJob* j) { return !j->plan.lossless; });
-  launch_t1_planes(ta, c->stream);
-  record(c, kEvAnalyzeEnd);
-  launch_t1_model(ta, c->num_sms, 0, c->stream);
-  record(c, kEvModelEnd);
   // Blocks are coded heaviest first, one per lane: a warp's lanes then carry
   // similar symbol counts, and the longest chains start first.
-  if (!reserve(c, c->mqorder, (size_t)nb * 4) || !reserve(c, c->mqscratch, ((size_t)nb + 2048) * 4))
+  if (!reserve(c, c->mqorder, (size_t)nb * 4) ||
+      !reserve(c, c->mqscratch, (split ? (size_t)nb * 3 + 2 * kOrderScratch : (size_t)nb + kOrderScratch) * 4))
     return kEncodeFailed;
-  launch_mq_order(ta, dptr<uint32_t>(c->mqorder), dptr<uint32_t>(c->mqscratch), c->stream);
-  ta.mq_order = dptr<uint32_t>(c->mqorder);
-  ta.unfinished = dptr<uint32_t>(c->mqscratch);  // the order has been made
+  uint32_t* const order = dptr<uint32_t>(c->mqorder);
+  uint32_t* const scratch = dptr<uint32_t>(c->mqscratch);
+  uint32_t* const key = scratch + (split ? 2 : 1) * kOrderScratch;
+  ta.mq_order = order;
+  ta.unfinished = split ? key + nb : key;  // not split: the order has been made
+  if (split) ta.weight = key + 2 * (size_t)nb;
+  ta.share = large ? 5 : 9;
   const int bpw = (int)c->opt[JP2G_OPT_MQ_BLOCKS_PER_WARP];
-  launch_t1_mq(ta, c->num_sms, bpw, 0, c->stream);
+  launch_t1_planes(ta, c->stream);
+  if (split) launch_t1_split(ta, c->stream);
+  record(c, kEvAnalyzeEnd);
+  if (split) {
+    launch_t1_model(ta, c->num_sms, kT1Part0, c->stream);
+    if (!cuda_ok(c, cudaEventRecord(c->ev_mq[0], c->stream), "part modelled") ||
+        !cuda_ok(c, cudaStreamWaitEvent(c->mq_stream, c->ev_mq[0], 0), "wait for a part"))
+      return kEncodeFailed;
+    launch_mq_order(ta, kT1Part0, order, key, scratch + kOrderScratch, c->mq_stream);
+    launch_t1_mq(ta, c->num_sms, bpw, kT1Part0, c->mq_stream);
+  }
+  const T1Part rest = split ? kT1Part1 : kT1All;
+  launch_t1_model(ta, c->num_sms, rest, c->stream);
+  record(c, kEvModelEnd);
+  launch_mq_order(ta, rest, order, key, scratch, c->stream);
+  launch_t1_mq(ta, c->num_sms, bpw, rest, c->stream);
+  if (split && (!cuda_ok(c, cudaEventRecord(c->ev_mq[1], c->mq_stream), "part coded") ||
+                !cuda_ok(c, cudaStreamWaitEvent(c->stream, c->ev_mq[1], 0), "wait for a part's coding"))) {
+    cudaStreamSynchronize(c->mq_stream);
+    return kEncodeFailed;
+  }
   if (ta.foresee) {
     ta.again = dptr<uint32_t>(c->mqorder);
     launch_t1_recheck(ta, c->num_sms, c->stream);
-    launch_t1_model(ta, c->num_sms, 1, c->stream);
-    launch_t1_mq(ta, c->num_sms, bpw, 1, c->stream);
+    launch_t1_model(ta, c->num_sms, kT1Again, c->stream);
+    launch_t1_mq(ta, c->num_sms, bpw, kT1Again, c->stream);
   }
-  c->counters[5] += 8 + (nb > 1024 ? 1 : 0) + (ta.foresee ? 3 : 0);
+  c->counters[5] += 8 + (nb > 1024 ? 1 : 0) + (split ? 6 : 0) + (ta.foresee ? 3 : 0);
   record(c, 3);
   // ---- PCRD ----
   PcrdArgs pa{};
@@ -1199,7 +1236,11 @@ int jp2g_create(jp2g_ctx** out, int device, uint64_t hbm_budget_bytes) {
   for (auto& ev : c->ev) cudaEventCreate(&ev);
   cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
   cudaStreamCreateWithFlags(&c->serve_stream, cudaStreamNonBlocking);
+  int least = 0, greatest = 0;
+  cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  cudaStreamCreateWithPriority(&c->mq_stream, cudaStreamNonBlocking, greatest);
   for (int k = 0; k < 2; ++k) {
+    cudaEventCreateWithFlags(&c->ev_mq[k], cudaEventDisableTiming);
     cudaEventCreateWithFlags(&c->ev_up[k], cudaEventDisableTiming);
     cudaEventCreateWithFlags(&c->serve_ev[k], cudaEventDisableTiming);
   }
@@ -1228,6 +1269,10 @@ void jp2g_destroy(jp2g_ctx* c) {
                     &c->mqorder, &c->mqscratch, &c->recon, &c->reconblk, &c->t2pk, &c->t2bd, &c->t2pg,
                     &c->t2tmpl, &c->t2tree, &c->t2raw, &c->t2hdr, &c->t2hdrlen, &c->t2pktoff, &c->t2pagelen,
                     &c->t2pageoff, &c->t2nchunks, &c->t2chunkbase, &c->t2out};
+  if (c->mq_stream) {
+    cudaStreamSynchronize(c->mq_stream);
+    cudaStreamDestroy(c->mq_stream);
+  }
   if (c->copy_stream) {
     cudaStreamSynchronize(c->copy_stream);
     cudaStreamDestroy(c->copy_stream);
@@ -1247,6 +1292,7 @@ void jp2g_destroy(jp2g_ctx* c) {
   for (auto& ev : c->ev)
     if (ev) cudaEventDestroy(ev);
   for (int k = 0; k < 2; ++k) {
+    if (c->ev_mq[k]) cudaEventDestroy(c->ev_mq[k]);
     if (c->ev_up[k]) cudaEventDestroy(c->ev_up[k]);
     if (c->serve_ev[k]) cudaEventDestroy(c->serve_ev[k]);
   }

@@ -49,6 +49,17 @@ void launch_dwt_batch(const DwtLevelArgs* d_args, const uint32_t* d_tile_base, u
 // Tiles of one page's level in the flat tile list.
 uint32_t dwt_tiles(int rw, int rh, int ncomp);
 
+constexpr int kT1Parts = 2;
+enum T1Count {
+  kCountItems,                           // per part: items listed
+  kCountBlocks = kCountItems + kT1Parts, // per part: blocks (split waves)
+  kCountAgainItems = kCountBlocks + kT1Parts,
+  kCountAgainBlocks,                     // blocks that the second round codes on
+  kCountUnfinished,                      // blocks that ended the first round with bit-planes to go
+  kCountWeight,                          // largest weight
+  kCounts
+};
+
 struct T1Args {
   const BlockDesc* blocks;
   uint32_t nblocks;
@@ -61,9 +72,18 @@ struct T1Args {
   // (block, bit-plane) modelling items
   uint32_t* nplanes;     // per block: magnitude bit-planes, then (t1_planes_kernel) those to model at first
   uint32_t* plane_base;  // per block: its first item (exclusive prefix of the magnitude bit-planes)
-  uint32_t* items;       // items to model, block << 6 | index within the block: the first round's, then the second's
+  // items to model, block << 6 | index within the block: part p's from p * nitems
+  // on, and behind part 0's those of the second round
+  uint32_t* items;
   uint32_t nitems;       // all items
-  uint32_t* counts;      // zeroed: [0] items of the first round, [1] of the second, [2] unfinished, [3] again
+  // A split wave is modelled and coded in two parts, the blocks with the most
+  // symbols first, so that their coding runs beside the others' modelling.
+  // weight: per block, the symbols expected (top bit: in part 0 in any case);
+  // null: no split, everything is part 0. Part 0 reaches down to `share`
+  // twelfths of the largest weight.
+  uint32_t* weight;
+  uint32_t share;
+  uint32_t* counts;  // zeroed, kCounts words, see T1Count
   uint32_t* unfinished;  // blocks that ended the first round with bit-planes to go
   uint32_t* again;       // those of them that the second round codes on
   bool foresee;          // model only the bit-planes a block is likely to need; a second round takes the others
@@ -85,17 +105,23 @@ struct T1Args {
 void launch_t1_analyze(const T1Args& a, cudaStream_t st);
 // Items list and per-item bit-plane column masks (after the plane-count scan).
 void launch_t1_planes(const T1Args& a, cudaStream_t st);
-// round 0: the items foreseen, 1: the others of the blocks that are coded again.
-void launch_t1_model(const T1Args& a, int num_sms, int round, cudaStream_t st);
+// What a launch takes: in the first round every block, or a part of a split
+// wave; in the second round the blocks that are coded again.
+enum T1Part { kT1Part0, kT1Part1, kT1All, kT1Again };
+// Splits the blocks and lists the parts' items (after launch_t1_planes).
+void launch_t1_split(const T1Args& a, cudaStream_t st);
+void launch_t1_model(const T1Args& a, int num_sms, T1Part part, cudaStream_t st);
 // bpw: code-blocks per warp, 1..32, or 0 for automatic.
-void launch_t1_mq(const T1Args& a, int num_sms, int bpw, int round, cudaStream_t st);
+void launch_t1_mq(const T1Args& a, int num_sms, int bpw, T1Part part, cudaStream_t st);
 // Between the rounds: which unfinished blocks are coded on.
 void launch_t1_recheck(const T1Args& a, int num_sms, cudaStream_t st);
 // Code-blocks per warp that launch_t1_mq uses for `bpw` (0 = automatic).
 int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw);
-// Orders the blocks by their MQ symbol count, largest first (counting sort
-// on 1024 buckets), into order[nblocks]. scratch: nblocks + 2048 words.
-void launch_mq_order(const T1Args& a, uint32_t* order, uint32_t* scratch, cudaStream_t st);
+// Orders the blocks of a part (or all) by their MQ symbol count, largest
+// first (counting sort on 1024 buckets), into order[], one part behind the
+// other. key: nblocks words; scratch: kOrderScratch words.
+constexpr uint32_t kOrderScratch = 2048;
+void launch_mq_order(const T1Args& a, T1Part part, uint32_t* order, uint32_t* key, uint32_t* scratch, cudaStream_t st);
 
 // Exclusive prefix sum of n uint32 values read with a stride of `stride`
 // words: out[i] = sum of in[0..i), out[n] = total. `scratch` holds

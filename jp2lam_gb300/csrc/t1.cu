@@ -100,6 +100,8 @@ __device__ __forceinline__ float block_unit(const T1Args& a, uint32_t b, const B
   return bp.unit * (bp.is_ll ? base * 1.1f : base) * a.comps[d.comp_key].weight;
 }
 
+constexpr uint32_t kHeavy = 0x80000000u;  // T1Args::weight
+
 // 4^k: the energy of bit-plane k against bit-plane 0's (capped as in pcrd.cu).
 __device__ __forceinline__ float plane_energy(int k) { return __uint_as_float((uint32_t)(127 + 2 * min(k, 30)) << 23); }
 
@@ -149,7 +151,10 @@ __global__ void __launch_bounds__(256) t1_planes_kernel(T1Args a) {
       }
     }
   }
-  if (mbp == 0) return;
+  if (mbp == 0) {
+    if (lane == 0 && a.weight) a.weight[b] = 0;
+    return;
+  }
   // ItemRec::remain, by the distortion model of rate control (pcrd.cu), with
   // every newly significant sample taken as coded in significance propagation
   // (weight 1, cleanup has 0.85). Lane k holds bit-plane k.
@@ -208,13 +213,59 @@ __global__ void __launch_bounds__(256) t1_planes_kernel(T1Args a) {
     const uint32_t stops = __ballot_sync(0xffffffffu, lane < mbp && value + rest < best);
     if (stops) count = min(count, (uint32_t)(mbp - (31 - __clz((int)stops))) + 1u);
   }
-  uint32_t at = 0;
-  if (lane == 0) {
-    a.nplanes[b] = count;
-    at = atomicAdd(a.counts, count);
+  if (lane == 0) a.nplanes[b] = count;
+  if (a.weight) {
+    // symbols: a refinement or a sign each, and a zero coding of every sample
+    // near a significant one, of a quarter of the others
+    const uint32_t open = (uint32_t)(w * h) - (sig - newly), near = min(open, 6u * sig);
+    const bool coded = lane < mbp && lane >= mbp - (int)count;
+    const uint32_t n = __reduce_add_sync(0xffffffffu, coded ? sig + near + (open - near) / 4u : 0u);
+    if (lane == 0) {
+      a.weight[b] = n | (a.bands[d.band_param].is_ll ? kHeavy : 0u);
+      if (n > *const_cast<volatile uint32_t*>(a.counts + kCountWeight)) atomicMax(a.counts + kCountWeight, n);
+    }
+    return;
   }
+  uint32_t at = 0;
+  if (lane == 0) at = atomicAdd(a.counts + kCountItems, count);
   at = __shfl_sync(0xffffffffu, at, 0);
   for (uint32_t j = lane; j < count; j += 32) a.items[at + j] = b << 6 | j;
+}
+
+// The part of a block in a split wave: 0 from a share of the largest expected
+// symbol count on (and LL bands: few, and the ones whose slopes settle their
+// components' lambda), 1 below.
+__device__ __forceinline__ int part_of(const T1Args& a, uint32_t b) {
+  const uint32_t v = a.weight[b];
+  return v >= kHeavy || 12u * v >= a.share * a.counts[kCountWeight] ? 0 : 1;
+}
+
+// A thread per block: counts the parts' blocks and lists their items.
+__global__ void __launch_bounds__(256) t1_split_kernel(T1Args a) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int part = b < a.nblocks ? part_of(a, b) : -1;
+  const uint32_t n = part >= 0 ? a.nplanes[b] : 0u;
+  uint32_t at = 0;
+  #pragma unroll
+  for (int p = 0; p < kT1Parts; ++p) {
+    const uint32_t blocks = __ballot_sync(0xffffffffu, part == p);
+    if (blocks == 0) continue;
+    uint32_t sum = part == p ? n : 0u;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    uint32_t first = 0;
+    if (lane == 31) {
+      first = atomicAdd(a.counts + kCountItems + p, sum);
+      atomicAdd(a.counts + kCountBlocks + p, (uint32_t)__popc(blocks));
+    }
+    first = __shfl_sync(0xffffffffu, first, 31);
+    if (part == p) at = p * a.nitems + first + sum - n;
+  }
+  for (uint32_t j = 0; j < n; ++j) a.items[at + j] = b << 6 | j;
 }
 
 // Modelling works on the code-block in column layout: lane L owns columns
@@ -388,7 +439,7 @@ __device__ __forceinline__ void emit_column(uint32_t v, uint32_t sm, uint32_t c,
 //    run), so each lane writes its two columns' symbols into the three
 //    streams (SP | MR | cleanup, whose starts are known from the totals) at
 //    offsets from two packed warp scans.
-__global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a, int round) {
+__global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a, T1Part part) {
   __shared__ ModelSmem sm_all[kModelWarps];
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
@@ -396,7 +447,9 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a,
   const uint32_t nwarps = gridDim.x * kModelWarps;
   const int xa = lane, xb = lane + 32;
 
-  const uint32_t from = round ? a.counts[0] : 0u, count = a.counts[round];
+  const uint32_t p0 = part < kT1Parts ? part : kT1Part0;
+  const uint32_t count = a.counts[part == kT1Again ? kCountAgainItems : kCountItems + p0];
+  const uint32_t from = part == kT1Again ? a.counts[kCountItems] : p0 * a.nitems;
   for (uint32_t i = blockIdx.x * kModelWarps + wid; i < count; i += nwarps) {
     const uint32_t blkno = a.items[from + i] >> 6;
     const BlockDesc d = a.blocks[blkno];
@@ -967,7 +1020,7 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
     state->m = m;
     state->stop = stop.s;
     for (uint32_t c = 0; c < kCtxNone; ++c) state->context[c] = (uint16_t)(ctx_at(sm, c * kCtxStride + lane).y & 0x7ffu);
-    a.unfinished[atomicAdd(a.counts + 2, 1u)] = b;
+    a.unfinished[atomicAdd(a.counts + kCountUnfinished, 1u)] = b;
     return;
   }
   if (stopped || unfinished) {  // the coded passes stand, each with its bytes so far
@@ -992,19 +1045,36 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
   a.res[b] = o;
 }
 
-// Warp w codes blocks order[w * bpw + lane], lanes < bpw.
+// As few blocks per warp as keep at most one warp on each of the SMs' four
+// schedulers (a warp's lanes cost nothing, and a second warp on a scheduler
+// lengthens both warps' chains), up to 32.
+JP2G_HD int mq_blocks_auto(uint32_t nblocks, uint32_t warps) {
+  const uint32_t n = (nblocks + warps - 1) / warps;
+  return n < 1u ? 1 : n > 32u ? 32 : (int)n;
+}
+
+// The part's first block in the order.
+__device__ __forceinline__ uint32_t part_first(const T1Args& a, T1Part part) {
+  return part == kT1Part1 ? a.counts[kCountBlocks] : 0u;
+}
+
+// Warp w codes blocks order[w * bpw + lane], lanes < bpw. bpw 0: automatic
+// for `warps` warps.
 template <int round>
-__global__ void __launch_bounds__(kMqWarps * 32) t1_mq_kernel(T1Args a, int bpw) {
+__global__ void __launch_bounds__(kMqWarps * 32) t1_mq_kernel(T1Args a, T1Part part, int bpw, uint32_t warps) {
   __shared__ MqSmem sm;
   load_mq_table(sm.table);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
   if constexpr (round == 0) {
+    const uint32_t n = part == kT1All ? a.nblocks : a.counts[kCountBlocks + part];
+    const uint32_t first = part_first(a, part);
+    if (bpw == 0) bpw = mq_blocks_auto(n, warps);
     const uint32_t slot = (blockIdx.x * kMqWarps + wid) * (uint32_t)bpw + (uint32_t)lane;
-    mq_code_block<0>(a, lane < bpw && slot < a.nblocks ? a.mq_order[slot] : kNoBlock, sm);
+    mq_code_block<0>(a, lane < bpw && slot < n ? a.mq_order[first + slot] : kNoBlock, sm);
   } else {  // the blocks that t1_recheck_kernel listed, over a fixed grid
-    const uint32_t per_cta = kMqWarps * (uint32_t)bpw, count = a.counts[3];
+    const uint32_t per_cta = kMqWarps * (uint32_t)bpw, count = a.counts[kCountAgainBlocks];
     for (uint32_t first = blockIdx.x * per_cta; first < count; first += gridDim.x * per_cta) {
       const uint32_t slot = first + (uint32_t)(wid * bpw + lane);
       mq_code_block<1>(a, lane < bpw && slot < count ? a.again[slot] : kNoBlock, sm);
@@ -1017,7 +1087,7 @@ __global__ void __launch_bounds__(kMqWarps * 32) t1_mq_kernel(T1Args a, int bpw)
 // there) are done; the others are listed for the second round with their
 // remaining items.
 __global__ void t1_recheck_kernel(T1Args a) {
-  const uint32_t count = a.counts[2];
+  const uint32_t count = a.counts[kCountUnfinished];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     const uint32_t b = a.unfinished[i];
     const BlockDesc d = a.blocks[b];
@@ -1034,8 +1104,8 @@ __global__ void t1_recheck_kernel(T1Args a) {
       a.res[b] = o;
       continue;
     }
-    a.again[atomicAdd(a.counts + 3, 1u)] = b;
-    const uint32_t at = a.counts[0] + atomicAdd(a.counts + 1, all - done);
+    a.again[atomicAdd(a.counts + kCountAgainBlocks, 1u)] = b;
+    const uint32_t at = a.counts[kCountItems] + atomicAdd(a.counts + kCountAgainItems, all - done);
     for (uint32_t j = done; j < all; ++j) a.items[at + j - done] = b << 6 | j;
   }
 }
@@ -1084,29 +1154,36 @@ void launch_t1_planes(const T1Args& a, cudaStream_t st) {
   t1_planes_kernel<<<(uint32_t)(((uint64_t)a.nblocks * 32 + 255) / 256), 256, 0, st>>>(a);
 }
 
-void launch_t1_model(const T1Args& a, int num_sms, int round, cudaStream_t st) {
+void launch_t1_split(const T1Args& a, cudaStream_t st) {
+  if (a.nblocks == 0) return;
+  t1_split_kernel<<<(a.nblocks + 255) / 256, 256, 0, st>>>(a);
+}
+
+// CTAs loop over the items. Few are left for the second round; a split wave's
+// are short, as the coding of an earlier part waits for their places.
+void launch_t1_model(const T1Args& a, int num_sms, T1Part part, cudaStream_t st) {
   if (a.nitems == 0) return;
   uint32_t need = (a.nitems + kModelWarps - 1) / kModelWarps;
-  uint32_t cap = (uint32_t)num_sms * (round ? 2 : 6 * 4);  // CTAs loop over the items; few are left for round 1
-  t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a, round);
+  uint32_t cap = (uint32_t)num_sms * (part == kT1Again ? 2 : part == kT1All ? 6 * 4 : 6 * 24);
+  t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a, part);
 }
 
-// Automatic: as few blocks per warp as keep at most one warp on each of
-// the SMs' four schedulers (a warp's lanes cost nothing, and a second warp on
-// a scheduler lengthens both warps' chains), up to 32.
 int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw) {
-  if (bpw >= 1 && bpw <= 32) return bpw;
-  const uint32_t warps = (uint32_t)num_sms * 4u;
-  return (int)std::min<uint32_t>(32u, std::max<uint32_t>(1u, (a.nblocks + warps - 1) / warps));
+  return bpw >= 1 && bpw <= 32 ? bpw : mq_blocks_auto(a.nblocks, (uint32_t)num_sms * 4u);
 }
 
-void launch_t1_mq(const T1Args& a, int num_sms, int bpw, int round, cudaStream_t st) {
+void launch_t1_mq(const T1Args& a, int num_sms, int bpw, T1Part part, cudaStream_t st) {
   if (a.nblocks == 0) return;
-  bpw = mq_blocks_per_warp(a, num_sms, bpw);
-  const uint32_t per_cta = (uint32_t)bpw * kMqWarps, all = (a.nblocks + per_cta - 1) / per_cta;
-  // the second round's blocks are few
-  if (round) t1_mq_kernel<1><<<(uint32_t)num_sms, kMqWarps * 32, 0, st>>>(a, std::min(bpw, 4));
-  else t1_mq_kernel<0><<<all, kMqWarps * 32, 0, st>>>(a, bpw);
+  const uint32_t sms = (uint32_t)num_sms;
+  if (bpw < 1 || bpw > 32) bpw = 0;
+  const uint32_t most = (uint32_t)mq_blocks_per_warp(a, num_sms, bpw);
+  if (part == kT1Again) {  // few
+    t1_mq_kernel<1><<<sms, kMqWarps * 32, 0, st>>>(a, part, (int)std::min(most, 4u), 0u);
+    return;
+  }
+  // a part of the wave's blocks takes a CTA on each SM, or as many blocks per warp as the whole wave
+  const uint32_t per_cta = most * kMqWarps, all = (a.nblocks + per_cta - 1) / per_cta;
+  t1_mq_kernel<0><<<bpw ? all : std::max(all, sms), kMqWarps * 32, 0, st>>>(a, part, bpw, sms * 4u);
 }
 
 void launch_t1_recheck(const T1Args& a, int num_sms, cudaStream_t st) {
@@ -1114,7 +1191,7 @@ void launch_t1_recheck(const T1Args& a, int num_sms, cudaStream_t st) {
 }
 
 namespace {
-constexpr uint32_t kOrderBuckets = 1024;
+constexpr uint32_t kOrderBuckets = kOrderScratch / 2;
 
 // Bucket of a block: its MQ symbol count / 64, clamped, reversed so that
 // bucket 0 holds the largest blocks, and the LL bands' (few, and the ones whose
@@ -1131,9 +1208,13 @@ __device__ __forceinline__ uint32_t order_bucket(const T1Args& a, uint32_t b) {
   return kOrderBuckets - 1 - k;
 }
 
-__global__ void order_hist_kernel(T1Args a, uint32_t* key, uint32_t* hist) {
+__device__ __forceinline__ bool in_part(const T1Args& a, T1Part part, uint32_t b) {
+  return part == kT1All || part_of(a, b) == part;
+}
+
+__global__ void order_hist_kernel(T1Args a, T1Part part, uint32_t* key, uint32_t* hist) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.nblocks) return;
+  if (b >= a.nblocks || !in_part(a, part, b)) return;
   const uint32_t k = order_bucket(a, b);
   key[b] = k;
   atomicAdd(hist + k, 1u);
@@ -1163,23 +1244,22 @@ __global__ void order_scan_kernel(const uint32_t* hist, uint32_t* cursor) {
   cursor[t] = x - v + (wid > 0 ? warp_tot[wid - 1] : 0u);
 }
 
-__global__ void order_scatter_kernel(uint32_t n, const uint32_t* key, uint32_t* cursor, uint32_t* order) {
+__global__ void order_scatter_kernel(T1Args a, T1Part part, const uint32_t* key, uint32_t* cursor, uint32_t* order) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  order[atomicAdd(cursor + key[b], 1u)] = b;
+  if (b >= a.nblocks || !in_part(a, part, b)) return;
+  order[part_first(a, part) + atomicAdd(cursor + key[b], 1u)] = b;
 }
 }  // namespace
 
-void launch_mq_order(const T1Args& a, uint32_t* order, uint32_t* scratch, cudaStream_t st) {
+void launch_mq_order(const T1Args& a, T1Part part, uint32_t* order, uint32_t* key, uint32_t* scratch, cudaStream_t st) {
   if (a.nblocks == 0) return;
   uint32_t* hist = scratch;
   uint32_t* cursor = scratch + kOrderBuckets;
-  uint32_t* key = scratch + 2 * kOrderBuckets;
   cudaMemsetAsync(hist, 0, kOrderBuckets * sizeof(uint32_t), st);
   const uint32_t g = (a.nblocks + 255) / 256;
-  order_hist_kernel<<<g, 256, 0, st>>>(a, key, hist);
+  order_hist_kernel<<<g, 256, 0, st>>>(a, part, key, hist);
   order_scan_kernel<<<1, kOrderBuckets, 0, st>>>(hist, cursor);
-  order_scatter_kernel<<<g, 256, 0, st>>>(a.nblocks, key, cursor, order);
+  order_scatter_kernel<<<g, 256, 0, st>>>(a, part, key, cursor, order);
 }
 
 }  // namespace jp2g

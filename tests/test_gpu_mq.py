@@ -113,3 +113,23 @@ def test_second_round_of_a_large_wave(eng, orc):
         ref = orc.encode(p["px"], p["w"], p["h"], p["ncomp"], p["quality"], 0)
         for r in range(4):
             assert outs[i + 28 * r] == ref, (i, r)
+
+
+@pytest.mark.parametrize("q", [100, 75])
+@pytest.mark.parametrize("kind", ["flat", "noise", "one", "halves"])
+def test_split_wave(eng, orc, kind, q):
+    # a wave just large enough to be coded in two parts: nothing to code, every
+    # block in the first part, all but one in the second, and both alike
+    w, h = 2303, 2245
+    img = np.full((h, w), 128, np.uint8)
+    rng = np.random.default_rng(5)
+    if kind == "noise":
+        img = rng.integers(0, 256, (h, w), dtype=np.uint8)
+    elif kind == "one":
+        img[700:760, 900:960] = rng.integers(0, 256, (60, 60))
+    elif kind == "halves":
+        img[:, : w // 2] = rng.integers(0, 256, (h, w // 2))
+        img[:, w // 2:] = rng.integers(126, 130, (h, w - w // 2))
+    data = eng.encode(img.ravel(), w, h, 1, q, 0)
+    assert eng.counters()[0] > 8 * 152
+    assert data == orc.encode(img.ravel(), w, h, 1, q, 0)
