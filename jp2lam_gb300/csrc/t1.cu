@@ -653,27 +653,35 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a,
 // Measured (2550x3300 gray q85 page; batch of 24 sRGB q75 pages): MQ stage 3.04
 // and 5.2 ms (403 G symbols/s); 4.38 and 11.1 ms with an integer coder, split
 // over producer/consumer warp pairs on the page, branching at its byte output
-// in the batch. A lone chain takes 105 cycles per symbol.
+// in the batch. A lone chain takes 90 cycles per symbol; 106 when predicates
+// chose between A and Qe, and a renormalised context's state was read only then.
+//
 // Context entry, in shared memory: x = Qe / 2^15 as a float, its sign bit the
-// MPS; y = offset of the state's successors in the table | Qe << 16. The table
-// holds per state (state, MPS pair) its successors' entries: after an MPS
+// MPS; y = shared address of the state's successors in the table | MPS << 3. The
+// table holds per state (state, MPS pair) its successors' entries: after an MPS
 // renormalisation, then after an LPS.
 constexpr uint32_t kStates = 94;
-// Padding's Qe: too small to change A in a subtraction (1 - 2^-30 rounds to
-// 1), and its exponent's upper bits are those of every Qe (mq_code8).
-constexpr uint32_t kPadQe = 0x30800000u;
-struct MqTable {
+struct __align__(16) MqTable {
   uint2 next[kStates][2];
 };
-__device__ __forceinline__ uint2 mq_entry(uint32_t state) {
-  const uint32_t qe = c_tables.mq[state] & 0xffffu;
-  return make_uint2(__float_as_uint((float)qe * (1.0f / 32768.0f)) | (state & 1u) << 31, state * 16u | qe << 16);
+// Entry of a state; `table` is the table's shared address. kNoState: padding,
+// whose Qe of 0 changes nothing.
+constexpr uint32_t kNoState = kStates;
+__device__ __forceinline__ uint2 mq_entry(uint32_t state, uint32_t table) {
+  if (state == kNoState) return make_uint2(0u, table);
+  const uint32_t qe = c_tables.mq[state] & 0xffffu, mps = state & 1u;
+  return make_uint2(__float_as_uint((float)qe * (1.0f / 32768.0f)) | mps << 31, (table + state * 16u) | mps << 3);
+}
+__device__ __forceinline__ uint32_t mq_state(uint2 e, uint32_t table) { return (e.y - table) >> 4; }
+__device__ __forceinline__ uint32_t mq_table_at(const MqTable& t) {
+  return (uint32_t)__cvta_generic_to_shared(&t);
 }
 __device__ __forceinline__ void load_mq_table(MqTable& t) {
+  const uint32_t at = mq_table_at(t);
   for (uint32_t i = threadIdx.x; i < kStates; i += blockDim.x) {
     const uint32_t v = c_tables.mq[i];  // qe | nmps << 16 | nlps << 24
-    t.next[i][0] = mq_entry((v >> 16) & 0xffu);
-    t.next[i][1] = mq_entry(v >> 24);
+    t.next[i][0] = mq_entry((v >> 16) & 0xffu, at);
+    t.next[i][1] = mq_entry(v >> 24, at);
   }
 }
 
@@ -724,17 +732,20 @@ __device__ __forceinline__ uint2& ctx_at(MqSmem& sm, uint32_t off) {
   return *reinterpret_cast<uint2*>(sm.ce + off);
 }
 // Offset of the context entry of symbol i (0..3) of a word for the lane whose
-// entries start at `lane`; the symbol's decision as a sign bit.
+// entries start at `lane`; the symbol's decision as a sign bit; and as bit 3.
 __device__ __forceinline__ uint32_t sym_ctx(uint32_t w, int i, uint32_t lane) {
   return ((i < 2 ? w << (10 - 8 * i) : w >> (8 * i - 10)) & 0x7c00u) | lane;
 }
 __device__ __forceinline__ uint32_t sym_sign(uint32_t w, int i) { return w << (24 - 8 * i); }
+__device__ __forceinline__ uint32_t sym_bit3(uint32_t w, int i) { return (w >> (8 * i + 4)) & 8u; }
 
 // Codes the 16 symbols of a chunk.
 //
 // A symbol (C.2.4-C.2.7) with the decisions folded: after A -= Qe the coder
 // keeps A (and adds Qe to C) exactly when (A < Qe) equals "LPS", and
-// otherwise takes Qe (C unchanged). The context moves to its next state
+// otherwise takes Qe (C unchanged): of the two the larger for an MPS, the
+// smaller for an LPS, which with both negative is the larger again (predicates
+// would cost the chain more than signs). The context moves to its next state
 // exactly when the result is below 0x8000 and is renormalised.
 //
 // The code register is brought up to date once for the chunk: its 16
@@ -748,7 +759,6 @@ __device__ __forceinline__ uint32_t sym_sign(uint32_t w, int i) { return w << (2
 // bits.
 __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, const uint4 q) {
   const uint32_t w[5] = {q.x, q.y, q.z, q.w, kPadSymbol};
-  const uint32_t table = (uint32_t)__cvta_generic_to_shared(&sm.table) - 3u;
   uint32_t ops[16];  // exponent of the result (127 - the shift) << 23 | addition to C
   uint64_t acc = 0;
   int room = 31;  // fractional bits left: 31 - shifts so far
@@ -758,28 +768,27 @@ __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, con
   for (int i = 0; i < 16; ++i) {
     const uint32_t cxn = sym_ctx(w[(i + 1) >> 2], (i + 1) & 3, lane);
     const uint2 en = ctx_at(sm, cxn);  // the next symbol's entry, one step ahead
-    const float qe = fabsf(__uint_as_float(e.x));
+    const uint32_t next = e.y ^ sym_bit3(w[i >> 2], i & 3);
+    uint2 s;  // the state it may move to, read while A is found
+    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(s.x), "=r"(s.y) : "r"(next));
     const uint32_t xs = e.x ^ (sym_sign(w[i >> 2], i & 3) & 0x80000000u);
-    const bool lps = (int)xs < 0;
-    // bits 28..30 of every Qe are 3, so the top four bits are 8 * lps + 3
-    const uint32_t next = table + (((xs >> 28) & ~0x7f0u) | (e.y & 0x7f0u));
-    const float a = __fsub_rn(m.a, qe);
-    const bool take_a = (a < qe) == lps;
-    const float v = take_a ? a : qe;
+    const float a = __fsub_rn(m.a, fabsf(__uint_as_float(e.x)));
+    const float sa = __uint_as_float(__float_as_uint(a) | (xs & 0x80000000u)), sq = __uint_as_float(xs);
+    const float v = fmaxf(sa, sq);
+    // sa >= sq for an MPS, > for an LPS: both are multiples of 2^-15
+    const bool take_a = sa > __fmul_rn(sq, 1.0f - 1.0f / 1048576.0f);
     const uint32_t vb = __float_as_uint(v);
     m.a = __uint_as_float((vb & 0x7fffffu) | 0x3f800000u);
-    const uint32_t add = take_a ? e.y >> 16 : 0u;
-    ops[i] = (vb & 0xff800000u) | add;
+    // at 256 a unit of the last place is 2^-15
+    const uint32_t add = __float_as_uint(__fadd_rn(take_a ? fabsf(sq) : 0.0f, 256.0f)) & 0xffffu;
+    ops[i] = (vb & 0x7f800000u) | add;
     acc += (uint64_t)add * __funnelshift_l(0u, 1u, (uint32_t)room);
-    room += (int)(vb >> 23) - 127;
-    // the next state, loaded only when renormalised (selecting from a load
-    // made ahead costs more in selects than it hides)
-    asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, 0f3F800000;\n\t@p ld.shared.v2.u32 {%0, %1}, [%3];\n\t}"
-        : "+r"(e.x), "+r"(e.y)
-        : "f"(v), "r"(next));
-    ctx_at(sm, cx) = e;
-    e.x = cxn == cx ? e.x : en.x;
-    e.y = cxn == cx ? e.y : en.y;
+    room += (int)(ops[i] >> 23) - 127;
+    const bool renormalised = fabsf(v) < 1.0f;
+    if (renormalised) ctx_at(sm, cx) = s;
+    const bool same = renormalised && cxn == cx;
+    e.x = same ? s.x : en.x;
+    e.y = same ? s.y : en.y;
     cx = cxn;
   }
   bool one_by_one = room < 0;
@@ -906,7 +915,7 @@ static_assert(sizeof(MqState) <= kStateBytes && kCtxNone <= kMqCtx, "the slot's 
 constexpr uint32_t kNoBlock = 0xffffffffu;
 template <int round>
 __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSmem& sm) {
-  const uint32_t lane = threadIdx.x * 8u;
+  const uint32_t lane = threadIdx.x * 8u, table = mq_table_at(sm.table);
   BlockOut o{};
   if (b != kNoBlock) o = a.res[b];
   const int mbp = o.status ? 0 : o.mbp;
@@ -927,8 +936,8 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
     c0 = src[0];  // the slot and buffer are padded for these reads
     // contexts: state 0 except UNI 46, AGG 3, ZC 4 (src/mq/mod.rs:195-200)
     for (uint32_t c = 0; c < kMqCtx; ++c)
-      ctx_at(sm, c * kCtxStride + lane) = c == kCtxNone ? make_uint2(kPadQe, 0u)
-                                                        : mq_entry(c == kCtxUNI ? 92 : c == kCtxAGG ? 6 : c == 0 ? 8 : 0);
+      ctx_at(sm, c * kCtxStride + lane) =
+          mq_entry(c == kCtxNone ? kNoState : c == kCtxUNI ? 92 : c == kCtxAGG ? 6 : c == 0 ? 8 : 0, table);
   }
   Stop stop{};
   if (active && a.settled && !a.comps[d.comp_key].lossless) stop.start(a, b, d);
@@ -941,7 +950,7 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
   if (round && active) {
     m = state->m;
     stop.s = state->stop;
-    for (uint32_t c = 0; c < kCtxNone; ++c) ctx_at(sm, c * kCtxStride + lane) = mq_entry(state->context[c] >> 4);
+    for (uint32_t c = 0; c < kCtxNone; ++c) ctx_at(sm, c * kCtxStride + lane) = mq_entry(state->context[c], table);
     pr += 1 + 3 * (j - 1);
   }
   // One flat loop over the chunks of all items (bit-planes); the next item's
@@ -1019,7 +1028,7 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
   if (unfinished && !ovf) {  // the second round goes on with the other bit-planes
     state->m = m;
     state->stop = stop.s;
-    for (uint32_t c = 0; c < kCtxNone; ++c) state->context[c] = (uint16_t)(ctx_at(sm, c * kCtxStride + lane).y & 0x7ffu);
+    for (uint32_t c = 0; c < kCtxNone; ++c) state->context[c] = (uint16_t)mq_state(ctx_at(sm, c * kCtxStride + lane), table);
     a.unfinished[atomicAdd(a.counts + kCountUnfinished, 1u)] = b;
     return;
   }
