@@ -72,6 +72,18 @@ int jp2g_encode_with_psnr(jp2g_ctx* ctx, const uint8_t* px, uint32_t w, uint32_t
                           int interleaved, uint8_t quality, int format, uint8_t** out, size_t* out_len,
                           double* psnr_db, double* ssim);
 
+/* Where the encode calls of this context put their codestreams, so that a
+ * caller with memory of its own kind (a Python bytes object) needs no copy of
+ * the result: jp2g_encode, jp2g_encode_with_psnr, jp2g_encode_device (index 0)
+ * and jp2g_encode_batch (index: the request's) ask alloc for the codestream's
+ * bytes once its length is known, write into what it returns and return that
+ * pointer, which is not for jp2g_free. alloc runs on the calling thread, may be
+ * called more than once for an index (the last one counts) and may return
+ * NULL (JP2G_ENCODE_FAILED). A null alloc: malloc again. Served requests
+ * (jp2g_submit) always use malloc. */
+typedef uint8_t* (*jp2g_result_alloc)(void* user, uint32_t index, size_t bytes);
+int jp2g_set_result_alloc(jp2g_ctx* ctx, jp2g_result_alloc alloc, void* user);
+
 /* Decodes a J2K or JP2 file as decode_jp2 does (src/decode/mod.rs:56-61):
  * single tile, one quality layer, LRCP, one precinct per resolution, 8-bit
  * gray or 3-component, 64x64 or smaller code-blocks — the codestreams this

@@ -54,7 +54,7 @@ EXPORTS = [
     "jp2g_encode_batch", "jp2g_submit", "jp2g_poll", "jp2g_set_option", "jp2g_get_option",
     "jp2g_autotune", "jp2g_debug_assemble", "jp2g_debug_plan", "jp2g_cancel", "jp2g_debug_context_labels",
     "jp2g_debug_coefficients_f32", "jp2g_encode_with_psnr", "jp2g_debug_assemble_device", "jp2g_decode",
-    "jp2g_decode_batch",
+    "jp2g_decode_batch", "jp2g_set_result_alloc",
 ]
 
 PENDING = 6
@@ -73,6 +73,15 @@ class Request(ctypes.Structure):
     _fields_ = [("px", ctypes.c_void_p), ("width", ctypes.c_uint32), ("height", ctypes.c_uint32),
                 ("ncomp", ctypes.c_uint32), ("interleaved", ctypes.c_int32), ("on_device", ctypes.c_int32),
                 ("quality", ctypes.c_int32), ("format", ctypes.c_int32)]
+
+# jp2g_result_alloc, and the bytes objects whose memory it hands out
+_ResultAlloc = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_size_t)
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype = ctypes.py_object
+_new_bytes.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
+_bytes_at = ctypes.pythonapi.PyBytes_AsString
+_bytes_at.restype = ctypes.c_void_p
+_bytes_at.argtypes = [ctypes.py_object]
 
 _lib = None
 _lock = threading.Lock()
@@ -97,6 +106,7 @@ def load_library(path: str = LIB_PATH):
                                            ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint8, ctypes.c_int,
                                            ctypes.POINTER(_u8p), ctypes.POINTER(ctypes.c_size_t)]
         lib.jp2g_free.argtypes = [_u8p]
+        lib.jp2g_set_result_alloc.argtypes = [ctypes.c_void_p, _ResultAlloc, ctypes.c_void_p]
         lib.jp2g_last_error.argtypes = [ctypes.c_void_p]
         lib.jp2g_last_error.restype = ctypes.c_char_p
         lib.jp2g_stream.argtypes = [ctypes.c_void_p]
@@ -165,6 +175,16 @@ class Engine:
             _raise(rc, self.lib.jp2g_last_error(None).decode())
         self.handle = h
         self._lock = threading.Lock()
+        # codestreams are written straight into new bytes objects; filled by
+        # the library during a call (under _lock), by index
+        results = self._results = {}
+
+        def alloc(_, index, n):
+            results[index] = data = _new_bytes(None, n)
+            return _bytes_at(data)
+
+        self._alloc = _ResultAlloc(alloc)
+        self.lib.jp2g_set_result_alloc(h, self._alloc, None)
         self._inflight = {}  # ticket -> pixel buffer kept alive until polled
         self._inflight_lock = threading.Lock()
 
@@ -178,6 +198,12 @@ class Engine:
             self.close()
         except Exception:
             pass
+
+    def _take(self, rc: int) -> bytes:
+        """The codestream of a single-page call; called under _lock."""
+        data = self._results.pop(0, None)
+        self._check(rc)
+        return data
 
     def _check(self, rc: int):
         if rc != 0:
@@ -194,10 +220,7 @@ class Engine:
         with self._lock:
             rc = self.lib.jp2g_encode(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                       int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n))
-            self._check(rc)
-        data = ctypes.string_at(out, n.value)
-        self.lib.jp2g_free(out)
-        return data
+            return self._take(rc)
 
     def encode_with_psnr(self, px, w: int, h: int, ncomp: int, quality: int, fmt: int,
                          interleaved: bool = True):
@@ -214,10 +237,7 @@ class Engine:
             rc = self.lib.jp2g_encode_with_psnr(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                                 int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n),
                                                 ctypes.byref(psnr), ctypes.byref(ssim))
-            self._check(rc)
-        data = ctypes.string_at(out, n.value)
-        self.lib.jp2g_free(out)
-        return data, psnr.value, ssim.value
+            return self._take(rc), psnr.value, ssim.value
 
     @staticmethod
     def _decode_flags(rct_chroma_extra_bitplane, accept_empty_segments):
@@ -283,10 +303,7 @@ class Engine:
         with self._lock:
             rc = self.lib.jp2g_encode_device(self.handle, ctypes.c_void_p(dev_ptr), w, h, ncomp, quality,
                                              fmt, ctypes.byref(out), ctypes.byref(n))
-            self._check(rc)
-        data = ctypes.string_at(out, n.value)
-        self.lib.jp2g_free(out)
-        return data
+            return self._take(rc)
 
     @staticmethod
     def _request(page, keep):
@@ -321,11 +338,12 @@ class Engine:
         with self._lock:
             rc = self.lib.jp2g_encode_batch(self.handle, reqs, n, outs, lens, status)
             msg = self.lib.jp2g_last_error(self.handle).decode() if rc != 0 else ""
+            files = dict(self._results)
+            self._results.clear()
         result = []
         for i in range(n):
             if status[i] == 0:
-                result.append(ctypes.string_at(outs[i], lens[i]))
-                self.lib.jp2g_free(outs[i])
+                result.append(files[i])
             else:
                 result.append(_BY_CODE.get(status[i], Jp2LamError)(msg or f"page {i} failed"))
         return result

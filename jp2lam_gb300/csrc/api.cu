@@ -61,6 +61,12 @@ enum SubEvent { kEvAnalyzeEnd = kNumStages + 1, kEvModelEnd, kEvT2End, kNumEvent
 
 // One page of a wave: its request, its plan and, after the device phase,
 // the page-local retained blocks and bytes that Tier-2 needs.
+// jp2g_set_result_alloc
+struct ResultAlloc {
+  jp2g_result_alloc fn = nullptr;
+  void* user = nullptr;
+};
+
 struct PageJob {
   const uint8_t* host_px = nullptr;
   const uint8_t* dev_px = nullptr;
@@ -73,14 +79,16 @@ struct PageJob {
   size_t px_off = 0;        // the page's pixels in the wave's staging buffer
   bool staged = false;      // copied to the device from pinned staging
   bool laid_out = false;    // has a place (px_off) in the wave's pixel buffer
-  uint8_t* cs = nullptr;  // the finished codestream (J2K or JP2), malloc'd
+  uint8_t* cs = nullptr;  // the finished codestream (J2K or JP2), malloc'd or from `alloc`
   size_t cs_len = 0;
+  ResultAlloc alloc;
+  uint32_t index = 0;
   PageJob() = default;
   PageJob(const PageJob&) = delete;
   PageJob& operator=(const PageJob&) = delete;
-  ~PageJob() { std::free(cs); }
+  ~PageJob() { drop_output(); }
   void drop_output() {
-    std::free(cs);
+    if (!alloc.fn) std::free(cs);
     cs = nullptr;
     cs_len = 0;
   }
@@ -120,6 +128,7 @@ struct jp2g_ctx {
   // current one computes), alternating between px and px2; its DWT waits
   // on ev_up
   cudaStream_t copy_stream = nullptr;
+  ResultAlloc result_alloc;
   // part 0 of a split wave is coded on mq_stream, whose CTAs start before others
   cudaStream_t mq_stream = nullptr;
   cudaEvent_t ev_mq[2] = {};
@@ -726,23 +735,32 @@ int run_tier2(jp2g_ctx* c, const std::vector<PageJob*>& live, const BlockKeep* d
       !cuda_ok(c, cudaStreamSynchronize(c->stream), "D2H codestreams"))
     return kEncodeFailed;
   const uint8_t* hout = reinterpret_cast<const uint8_t*>(c->hout.p);
-  std::atomic<bool> oom{false};
-  auto take = [&](size_t i) {
+  // a result's memory is mostly fresh pages, so large ones are copied in
+  // pieces by the host threads
+  constexpr uint32_t kPiece = 1u << 20;
+  struct Piece {
+    uint8_t* dst;
+    const uint8_t* src;
+    size_t n;
+  };
+  std::vector<Piece> pieces;
+  for (size_t i = 0; i < pages.size(); ++i) {
     PageJob* j = pages[i];
     const size_t len = hoff[i + 1] - hoff[i];
     j->drop_output();
-    j->cs = static_cast<uint8_t*>(std::malloc(std::max<size_t>(len, 1)));
+    j->cs = j->alloc.fn ? j->alloc.fn(j->alloc.user, j->index, len)
+                        : static_cast<uint8_t*>(std::malloc(std::max<size_t>(len, 1)));
     if (!j->cs) {
-      oom = true;
       j->status = kEncodeFailed;
       j->err = "out of host memory";
-      return;
+      continue;
     }
-    std::memcpy(j->cs, hout + hoff[i], len);
     j->cs_len = len;
-  };
-  parallel_for(pages.size(), pages.size() >= 8 && total >= (8u << 20) ? host_threads(c) : 1, take);
-  (void)oom;
+    for (size_t at = 0; at < len; at += kPiece)
+      pieces.push_back({j->cs + at, hout + hoff[i] + at, std::min<size_t>(kPiece, len - at)});
+  }
+  parallel_for(pieces.size(), total >= (8u << 20) ? host_threads(c) : 1,
+               [&](size_t k) { std::memcpy(pieces[k].dst, pieces[k].src, pieces[k].n); });
   return kOk;
 }
 
@@ -1320,6 +1338,7 @@ int jp2g_encode(jp2g_ctx* c, const uint8_t* px, uint32_t w, uint32_t h, uint32_t
   if (!px) return set_err(c, JP2G_INVALID_INPUT, "pixel pointer is null");
   cudaSetDevice(c->device);
   PageJob j;
+  j.alloc = c->result_alloc;
   j.host_px = px;
   j.w = w;
   j.h = h;
@@ -1339,6 +1358,7 @@ int jp2g_encode_device(jp2g_ctx* c, const uint8_t* d_px, uint32_t w, uint32_t h,
   if (!d_px) return set_err(c, JP2G_INVALID_INPUT, "pixel pointer is null");
   cudaSetDevice(c->device);
   PageJob j;
+  j.alloc = c->result_alloc;
   j.dev_px = d_px;
   j.w = w;
   j.h = h;
@@ -1420,6 +1440,7 @@ int jp2g_encode_with_psnr(jp2g_ctx* c, const uint8_t* px, uint32_t w, uint32_t h
   if (!px) return set_err(c, JP2G_INVALID_INPUT, "pixel pointer is null");
   cudaSetDevice(c->device);
   PageJob j;
+  j.alloc = c->result_alloc;
   j.host_px = px;
   j.w = w;
   j.h = h;
@@ -1725,8 +1746,9 @@ static void job_from_request(const jp2g_request& r, PageJob* j) {
   j->format = r.format;
 }
 
-int jp2g_encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8_t** outs,
-                      size_t* out_lens, int* status) {
+// jp2g_encode_batch; own_results: the results in malloc'd memory in any case.
+static int encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8_t** outs, size_t* out_lens,
+                        int* status, bool own_results) {
   if (!c) return JP2G_INVALID_INPUT;
   std::lock_guard<std::mutex> lk(c->mu);
   if (n > 0 && (!reqs || !outs || !out_lens || !status))
@@ -1736,6 +1758,8 @@ int jp2g_encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8_t
   std::vector<PageJob*> ptrs(n);
   for (uint32_t i = 0; i < n; ++i) {
     job_from_request(reqs[i], &jobs[i]);
+    if (!own_results) jobs[i].alloc = c->result_alloc;
+    jobs[i].index = i;
     ptrs[i] = &jobs[i];
     outs[i] = nullptr;
     out_lens[i] = 0;
@@ -1850,6 +1874,11 @@ int jp2g_encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8_t
     }
   }
   return first_fail;
+}
+
+int jp2g_encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8_t** outs,
+                      size_t* out_lens, int* status) {
+  return encode_batch(c, reqs, n, outs, out_lens, status, false);
 }
 
 namespace {
@@ -2183,7 +2212,7 @@ int jp2g_autotune(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, int repeats
     for (int i = 0; i < JP2G_NUM_OPTS; ++i)
       if (jp2g_set_option(c, i, o[i]) != JP2G_OK) return -1.0;
     const auto t0 = std::chrono::steady_clock::now();
-    const int rc = jp2g_encode_batch(c, reqs, n, outs.data(), lens.data(), st.data());
+    const int rc = encode_batch(c, reqs, n, outs.data(), lens.data(), st.data(), true);
     const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     bool same = true;
     for (uint32_t i = 0; i < n; ++i) {
@@ -2254,6 +2283,13 @@ int jp2g_autotune(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, int repeats
 }
 
 void jp2g_free(uint8_t* p) { std::free(p); }
+
+int jp2g_set_result_alloc(jp2g_ctx* c, jp2g_result_alloc alloc, void* user) {
+  if (!c) return JP2G_INVALID_INPUT;
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->result_alloc = {alloc, user};
+  return JP2G_OK;
+}
 
 const char* jp2g_last_error(jp2g_ctx* c) { return c ? c->err.c_str() : g_create_error.c_str(); }
 

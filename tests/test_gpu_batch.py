@@ -271,3 +271,23 @@ def test_pipelines_with_many_blocks_per_chain_are_deterministic(eng, chains):
         for o, v in zip(opts, old):
             eng.set_option(o, v)
     assert ref[0] == _single(eng, pages[0])
+
+
+def test_results_are_objects_of_their_own(eng):
+    # codestreams are written straight into new bytes objects: a later call,
+    # a failing page in the batch or a page of many megabytes disturbs none
+    rng = np.random.default_rng(3)
+    small = rng.integers(0, 256, 40 * 30, dtype=np.uint8)
+    large = rng.integers(0, 256, 3100 * 3000, dtype=np.uint8)
+    first = eng.encode(small, 40, 30, 1, 100, 0)
+    copy = bytes(bytearray(first))
+    pages = [{"px": large, "w": 3100, "h": 3000, "ncomp": 1, "quality": 100, "fmt": 0},
+             {"px": small, "w": 20, "h": 30, "ncomp": 2, "quality": 100, "fmt": 0},
+             {"px": small, "w": 40, "h": 30, "ncomp": 1, "quality": 100, "fmt": 0}]
+    outs = eng.encode_batch(pages)
+    assert isinstance(outs[1], Exception)
+    assert outs[2] == copy and first == copy and outs[2] is not first
+    assert np.array_equal(eng.decode(outs[0])[0], large)
+    with pytest.raises(jl.Jp2LamError):
+        eng.encode(small, 20, 30, 2, 100, 0)
+    assert eng.encode(small, 40, 30, 1, 100, 0) == copy
