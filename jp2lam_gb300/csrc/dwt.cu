@@ -63,6 +63,42 @@ __device__ __forceinline__ int32_t quantize(float v, float step) {
   return __float2int_rz(__fdiv_rn(v, step));
 }
 
+// Quantises a run of samples (float bits) in place, as quantize() does each.
+// The quotient's integer part is taken from two truncated products with 1 /
+// step, one rounded safely down and one safely up (by 2^-21, eight times the
+// error of the reciprocal, the factor and the division together): where they
+// agree, so does the exact quotient's, and its rounded one's. The sum with 2^23
+// leaves the integer in the low bits. Where they don't (a quotient within a
+// millionth of an integer), or it has more than 23 bits, a group of samples is
+// divided out; so it is for a step of 0. All levels of 24 sRGB 2550x3300 pages:
+// 2.57 -> 2.31 ms against a division, with its branch, per sample; groups of
+// 16 take 96 registers, and a CTA fewer fits.
+constexpr int kGroup = 8;
+__device__ __forceinline__ void quantize_run(uint32_t (&v)[16], float step) {
+  const float inv = __frcp_rn(step);
+  const float below = __fmul_rn(inv, 1.0f - 1.0f / 2097152.0f), above = __fmul_rn(inv, 1.0f + 1.0f / 2097152.0f);
+  #pragma unroll
+  for (int g = 0; g < 16; g += kGroup) {
+    uint32_t q[kGroup], differ = 0, all = 0;
+    #pragma unroll
+    for (int i = 0; i < kGroup; ++i) {
+      const float m = fabsf(__uint_as_float(v[g + i]));
+      const uint32_t a = __float_as_uint(__fmaf_rz(m, below, 8388608.0f));
+      const uint32_t b = __float_as_uint(__fmaf_rz(m, above, 8388608.0f));
+      differ |= a ^ b;
+      all |= b;
+      const uint32_t s = (uint32_t)((int)v[g + i] >> 31);
+      q[i] = ((b & 0x7fffffu) ^ s) - s;
+    }
+    if (differ != 0 || (all >> 23) != 0x96u) {
+      #pragma unroll
+      for (int i = 0; i < kGroup; ++i) q[i] = (uint32_t)quantize(__uint_as_float(v[g + i]), step);
+    }
+    #pragma unroll
+    for (int i = 0; i < kGroup; ++i) v[g + i] = q[i];
+  }
+}
+
 template <bool REV>
 struct Cfg {
   using T = typename std::conditional<REV, int32_t, float>::type;
@@ -454,31 +490,19 @@ __device__ __forceinline__ void dwt_tile(const DwtLevelArgs& args, int comp, int
   T* const ll_out = args.ll ? reinterpret_cast<T*>(args.ll) + (size_t)comp * args.ll_comp : nullptr;
   const DwtBandOut bhi = args.band[comp][p ? 3 : 1];  // HL or HH
   uint32_t lo[16], hi[16];
+  lift_wave<REV>(x, [&](int i, T val) {
+    if constexpr (REV) (i & 1 ? hi[(i - 5) >> 1] : lo[(i - 4) >> 1]) = (uint32_t)val;
+    else (i & 1 ? hi[(i - 5) >> 1] : lo[(i - 4) >> 1]) = __float_as_uint(__fmul_rn(val, i & 1 ? kK : kInvK));
+  });
   if (p == 0 && ll_out != nullptr) {
     // even rows of an intermediate level: LL to the next plane, unquantised
-    lift_wave<REV>(x, [&](int i, T val) {
-      if (i & 1) {
-        if constexpr (REV) hi[(i - 5) >> 1] = (uint32_t)val;
-        else hi[(i - 5) >> 1] = (uint32_t)quantize(__fmul_rn(val, kK), bhi.step);
-      } else {
-        if constexpr (REV) lo[(i - 4) >> 1] = (uint32_t)val;
-        else lo[(i - 4) >> 1] = __float_as_uint(__fmul_rn(val, kInvK));
-      }
-    });
     if (lo_ok) store_run(reinterpret_cast<uint32_t*>(ll_out + (size_t)v * args.ll_pitch + u), lo);
   } else {
     const DwtBandOut blo = args.band[comp][p ? 2 : 0];  // LL (last level) or LH
-    lift_wave<REV>(x, [&](int i, T val) {
-      if (i & 1) {
-        if constexpr (REV) hi[(i - 5) >> 1] = (uint32_t)val;
-        else hi[(i - 5) >> 1] = (uint32_t)quantize(__fmul_rn(val, kK), bhi.step);
-      } else {
-        if constexpr (REV) lo[(i - 4) >> 1] = (uint32_t)val;
-        else lo[(i - 4) >> 1] = (uint32_t)quantize(__fmul_rn(val, kInvK), blo.step);
-      }
-    });
+    if constexpr (!REV) quantize_run(lo, blo.step);
     if (lo_ok) store_run(slot_at(args.coef, blo, v, u, cbs, cbhs), lo);
   }
+  if constexpr (!REV) quantize_run(hi, bhi.step);
   if (hi_ok) store_run(slot_at(args.coef, bhi, v, u, cbs, cbhs), hi);
 }
 
