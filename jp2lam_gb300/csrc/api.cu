@@ -1000,7 +1000,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   pa.hull_slope = dptr<double>(c->hulls);
   pa.hull_n = dptr<uint8_t>(c->hulln);
   pa.keep = dptr<BlockKeep>(c->keep);
-  launch_pcrd(pa, c->stream);
+  launch_pcrd(pa, c->num_sms, c->stream);
   record(c, 4);
   // ---- compaction ----
   launch_compact(ta.blocks, pa.keep, nb, ta.out, dptr<uint8_t>(c->body), dptr<uint32_t>(c->offsets),

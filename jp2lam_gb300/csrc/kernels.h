@@ -144,7 +144,7 @@ struct PcrdArgs {
   BlockKeep* keep;
 };
 
-void launch_pcrd(const PcrdArgs& a, cudaStream_t st);
+void launch_pcrd(const PcrdArgs& a, int num_sms, cudaStream_t st);
 
 // ------------------------------------------------------ device Tier-2 --
 struct T2Node {  // tag-tree node: minimum zero bit-planes, first included leaf (or ~0)

@@ -44,6 +44,28 @@ __device__ __forceinline__ uint32_t cum_len(const PassRec* pr, uint32_t n, uint3
   return total >= prev ? total : prev;
 }
 
+// What a pass takes off the distortion:
+// estimate_pass_distortion_delta_pass_kind_aware with visibility 1.0.
+__device__ __forceinline__ double pass_delta(const PassRec& r, const BandParam& bp, const CompParam& cp, double block_w) {
+  int bpl = r.bitplane < 30 ? r.bitplane : 30;
+  double plane = __dmul_rn((double)(1ull << bpl), bp.quant_step);
+  double energy = __dmul_rn(plane, plane);
+  double contrib;
+  if (r.kind == 0) contrib = __dmul_rn((double)r.ns, energy);
+  else if (r.kind == 1) contrib = __dmul_rn(__dmul_rn((double)r.sig_before, energy), 0.25);
+  else contrib = __dmul_rn(__dmul_rn((double)r.ns, energy), 0.85);
+  double raw = __dmul_rn(__dmul_rn(__dmul_rn(bp.subband_weight, bp.band_bias), block_w), contrib);
+  // apply_contrast_masking_to_delta(raw, 1.0, ..): the blended weight is
+  // exactly 1.0 for visibility 1.0, so the delta is raw (or 0).
+  return __dmul_rn(raw <= 0.0 ? 0.0 : raw, cp.comp_weight);
+}
+
+// class_distortion_weight (src/profile.rs:141-154)
+__device__ __forceinline__ double block_weight(const BlockOut& o, const BandParam& bp) {
+  double cw_base = o.cls == 0 ? 2.5 : (o.cls == 1 ? 1.5 : 1.0);
+  return bp.is_ll ? __dmul_rn(cw_base, 1.1) : cw_base;
+}
+
 __global__ void pcrd_hull_kernel(PcrdArgs a) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= a.nblocks) return;
@@ -61,9 +83,7 @@ __global__ void pcrd_hull_kernel(PcrdArgs a) {
   }
   const BandParam bp = a.bands[d.band_param];
   const PassRec* pr = a.passes + d.pass_off;
-  // class_distortion_weight (src/profile.rs:141-154)
-  double cw_base = o.cls == 0 ? 2.5 : (o.cls == 1 ? 1.5 : 1.0);
-  double block_w = bp.is_ll ? __dmul_rn(cw_base, 1.1) : cw_base;
+  const double block_w = block_weight(o, bp);
 
   // The hull as a stack of points (bytes hb, distortion hd, pass count hp)
   // with hs[k] the slope from point k-1 to point k, computed once when
@@ -81,20 +101,7 @@ __global__ void pcrd_hull_kernel(PcrdArgs a) {
   double cum_d = 0.0;
   for (uint32_t i = 0; i < n; ++i) {
     const PassRec r = pr[i];
-    // estimate_pass_distortion_delta_pass_kind_aware with visibility 1.0
-    int bpl = r.bitplane < 30 ? r.bitplane : 30;
-    double plane = __dmul_rn((double)(1ull << bpl), bp.quant_step);
-    double energy = __dmul_rn(plane, plane);
-    double contrib;
-    if (r.kind == 0) contrib = __dmul_rn((double)r.ns, energy);
-    else if (r.kind == 1) contrib = __dmul_rn(__dmul_rn((double)r.sig_before, energy), 0.25);
-    else contrib = __dmul_rn(__dmul_rn((double)r.ns, energy), 0.85);
-    double raw = __dmul_rn(__dmul_rn(__dmul_rn(bp.subband_weight, bp.band_bias), block_w), contrib);
-    // apply_contrast_masking_to_delta(raw, 1.0, ..): the blended weight is
-    // exactly 1.0 for visibility 1.0, so the delta is raw (or 0).
-    double delta = raw <= 0.0 ? 0.0 : raw;
-    delta = __dmul_rn(delta, cp.comp_weight);
-    cum_d = __dadd_rn(cum_d, delta);
+    cum_d = __dadd_rn(cum_d, pass_delta(r, bp, cp, block_w));
     uint32_t cum = cum_len(pr, n, i, o.payload_len) + 2u;  // HEADER_OVERHEAD_BYTES
     // push, after popping the top while the slope does not strictly
     // decrease (the slope into the new point >= the slope into the top)
@@ -120,6 +127,73 @@ __global__ void pcrd_hull_kernel(PcrdArgs a) {
     if (isfinite(s) && s > mx) mx = s;
   }
   a.hull_n[b] = (uint8_t)(hn - 1);
+  if (mx > 0.0) atomicMax(a.comp_max_slope + d.comp_key, (unsigned long long)__double_as_longlong(mx));
+}
+
+// pcrd_hull_kernel with a warp per block, for waves of few blocks: f64
+// arithmetic is slow to answer here, and a lane alone waits for some forty such
+// operations per pass. Lanes take the passes' distortions and the slopes
+// between neighbouring points side by side; the running sum, in pass order, and
+// the pruning stay with one lane (a pushed point's slope is from the point
+// before it, which is always the top, so only a pop needs a division of its
+// own).
+__global__ void __launch_bounds__(32) pcrd_hull_warp_kernel(PcrdArgs a) {
+  __shared__ double dist[kMaxPts], slope[kMaxPts], hs[kMaxPts];
+  __shared__ uint32_t bytes[kMaxPts];
+  __shared__ uint8_t hp[kMaxPts];
+  const uint32_t b = blockIdx.x, lane = threadIdx.x;
+  const BlockDesc d = a.blocks[b];
+  const BlockOut o = a.res[b];
+  const CompParam cp = a.comps[d.comp_key];
+  const uint32_t n = o.npasses;
+  if (n + 1 > (uint32_t)kMaxPts || cp.lossless || n == 0) {
+    if (lane == 0) a.hull_n[b] = n + 1 > (uint32_t)kMaxPts ? kHullTooLong : 0;
+    return;
+  }
+  const BandParam bp = a.bands[d.band_param];
+  const PassRec* pr = a.passes + d.pass_off;
+  const double block_w = block_weight(o, bp);
+  for (uint32_t i = lane; i < n; i += 32) {
+    dist[i + 1] = pass_delta(pr[i], bp, cp, block_w);
+    bytes[i + 1] = cum_len(pr, n, i, o.payload_len) + 2u;  // HEADER_OVERHEAD_BYTES
+  }
+  __syncwarp();
+  if (lane == 0) {
+    double sum = 0.0;
+    dist[0] = 0.0;
+    bytes[0] = 0;
+    for (uint32_t i = 1; i <= n; ++i) dist[i] = sum = __dadd_rn(sum, dist[i]);
+  }
+  __syncwarp();
+  for (uint32_t i = lane; i < n; i += 32) slope[i + 1] = rd_slope(bytes[i], dist[i], bytes[i + 1], dist[i + 1]);
+  __syncwarp();
+  int hn = 1;
+  if (lane == 0) {
+    double ts = 0.0;
+    hp[0] = 0;
+    hs[0] = 0.0;
+    for (uint32_t i = 1; i <= n; ++i) {
+      double sn = slope[i];
+      while (hn >= 2 && sn >= ts) {
+        --hn;
+        const uint32_t t = hp[hn - 1];
+        ts = hs[hn - 1];
+        sn = rd_slope(bytes[t], dist[t], bytes[i], dist[i]);
+      }
+      hp[hn] = (uint8_t)i;
+      hs[hn] = ts = sn;
+      ++hn;
+    }
+  }
+  hn = __shfl_sync(0xffffffffu, hn, 0);
+  double mx = 0.0;
+  for (int i = 1 + (int)lane; i < hn; i += 32) {
+    const double s = hs[i];
+    a.hull_passes[d.pass_off + i - 1] = hp[i];
+    a.hull_slope[d.pass_off + i - 1] = s;
+    if (isfinite(s) && s > mx) mx = s;
+  }
+  if (lane == 0) a.hull_n[b] = (uint8_t)(hn - 1);
   if (mx > 0.0) atomicMax(a.comp_max_slope + d.comp_key, (unsigned long long)__double_as_longlong(mx));
 }
 
@@ -191,7 +265,10 @@ __global__ void scan_partial_kernel(const uint32_t* in, uint32_t stride, uint32_
   __syncthreads();
   const uint32_t excl = x - v + (wid > 0 ? warp_tot[wid - 1] : 0u);
   if (i < n) out[i] = excl;
-  if (threadIdx.x == kScanT - 1) sums[blockIdx.x] = excl + v;
+  if (threadIdx.x == kScanT - 1) {
+    sums[blockIdx.x] = excl + v;
+    if (gridDim.x == 1) out[n] = excl + v;
+  }
 }
 
 __global__ void scan_sums_kernel(uint32_t* sums, uint32_t nparts, uint32_t* out, uint32_t n) {
@@ -230,14 +307,18 @@ __global__ void copy_bodies_kernel(const BlockDesc* blocks, const BlockKeep* kee
 
 }  // namespace
 
-void launch_pcrd(const PcrdArgs& a, cudaStream_t st) {
+void launch_pcrd(const PcrdArgs& a, int num_sms, cudaStream_t st) {
   if (a.nblocks == 0) return;
   cudaMemsetAsync(a.comp_max_slope, 0, sizeof(unsigned long long) * a.ncomp_keys, st);
   // one warp per CTA: a page's blocks spread over all SMs, whose few f64
   // units bound the hull's divisions
   const int t = 32;
   const uint32_t g = (a.nblocks + t - 1) / t;
-  pcrd_hull_kernel<<<g, t, 0, st>>>(a);
+  // up to 16 blocks per SM a warp each: a 256x256 page 13.7 us (a lane each:
+  // 42.6), 2,107 blocks 17.5; above that the few f64 units an SM has are kept
+  // busier by full warps (151,704 blocks: 91 us)
+  if (a.nblocks <= 16u * (uint32_t)num_sms) pcrd_hull_warp_kernel<<<a.nblocks, 32, 0, st>>>(a);
+  else pcrd_hull_kernel<<<g, t, 0, st>>>(a);
   pcrd_select_kernel<<<g, t, 0, st>>>(a);
 }
 
@@ -249,8 +330,9 @@ void launch_scan_u32(const uint32_t* in, uint32_t stride, uint32_t n, uint32_t* 
   }
   const uint32_t parts = (n + kScanT - 1) / kScanT;
   scan_partial_kernel<<<parts, kScanT, 0, st>>>(in, stride, n, out, scratch);
+  if (parts == 1) return;  // one launch for a small page
   scan_sums_kernel<<<1, 32, 0, st>>>(scratch, parts, out, n);
-  if (parts > 1) scan_add_kernel<<<parts, kScanT, 0, st>>>(out, n, scratch);
+  scan_add_kernel<<<parts, kScanT, 0, st>>>(out, n, scratch);
 }
 
 void launch_compact(const BlockDesc* blocks, const BlockKeep* keep, uint32_t nblocks,

@@ -133,3 +133,15 @@ def test_split_wave(eng, orc, kind, q):
     data = eng.encode(img.ravel(), w, h, 1, q, 0)
     assert eng.counters()[0] > 8 * 152
     assert data == orc.encode(img.ravel(), w, h, 1, q, 0)
+
+
+@pytest.mark.parametrize("q", [20, 50, 95, 99])
+@pytest.mark.parametrize("kind", ["noise", "sparse", "ramp"])
+@pytest.mark.parametrize("w,h,c", [(64, 64, 1), (2200, 1800, 3)])
+def test_hulls_by_warps_and_by_lanes(eng, orc, kind, w, h, c, q):
+    # rate-distortion curves of few and of many passes, in a wave of one block
+    # and in one whose blocks are too many for a warp each
+    px = np.repeat(_content(kind, w, h).reshape(h, w, 1), c, axis=2).ravel()
+    data = eng.encode(px, w, h, c, q, 0)
+    assert (eng.counters()[0] > 16 * 152) == (w > 64)
+    assert data == orc.encode(px, w, h, c, q, 0)
