@@ -1551,18 +1551,18 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   }
   first[maxl + 1] = (uint32_t)jobs.size();
   std::vector<PixJob> pix;
-  uint64_t total_px = 0;
+  uint32_t pix_blocks = 0;
   for (size_t i : ids) {
     const DecodePage& p = pg[i];
     PixJob j{};
     j.planes = (p.L.levels > 0 ? tmp : planes) + p.plane_base;
     j.px = dpx + p.px_base;
     j.npx = p.npx;
-    j.pix_base = total_px;
+    j.block_base = pix_blocks;
     j.ncomp = (uint32_t)p.L.ncomp;
-    j.mct = p.L.mct ? 1u : 0u;
+    j.mct = p.L.mct && p.L.ncomp == 3 ? 1u : 0u;
     j.reversible = p.L.reversible ? 1u : 0u;
-    total_px += p.npx;
+    pix_blocks += (uint32_t)((p.npx + kPixBlock - 1) / kPixBlock);
     pix.push_back(j);
   }
   const size_t blk_bytes = (blk.size() * sizeof(DecBlock) + 255) & ~size_t(255);
@@ -1587,7 +1587,7 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   launch_t1_decode(dblk, (uint32_t)blk.size(), dptr<uint8_t>(c->t2out), reinterpret_cast<unsigned long long*>(tmp),
                    planes, reinterpret_cast<uint32_t*>(dpx), c->stream);
   for (int l = 1; l <= maxl; ++l) launch_idwt_level(djobs + first[l], first[l + 1] - first[l], tiles[l], c->stream);
-  launch_dec_pixels(dpix, (uint32_t)pix.size(), total_px, c->stream);
+  launch_dec_pixels(dpix, (uint32_t)pix.size(), pix_blocks, c->stream);
   if (!cuda_ok(c, cudaGetLastError(), "decode kernels")) return JP2G_DECODE_FAILED;
   if (ids.size() >= 8) {
     // many files: one read-back into pinned memory, then the host threads

@@ -248,9 +248,11 @@ void idwt_jobs(void* plane, void* out, void* other, const std::pair<int, int>* l
 struct PixJob {
   const int32_t* planes;  // ncomp planes of npx samples (int32 or f32 bits)
   uint8_t* px;
-  uint64_t npx, pix_base;  // pix_base: the page's first global sample index
-  uint32_t ncomp, mct, reversible, pad;
+  uint64_t npx;
+  uint32_t block_base;  // the page's first CTA of the launch
+  uint32_t ncomp, mct, reversible;  // mct: 3 components
 };
+constexpr uint32_t kPixBlock = 1024;  // samples per CTA
 // Bit-planes that a block's passes reach: its top one in one pass, then three each.
 JP2G_HD uint32_t dec_planes(uint32_t npasses) { return npasses ? (npasses + 4) / 3 : 0; }
 // 64-bit words of a block's masks.
@@ -261,7 +263,7 @@ void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* d
                       int32_t* planes, uint32_t* scratch, cudaStream_t st);
 // One inverse-DWT level for njobs jobs (recon.cu).
 void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_tiles, cudaStream_t st);
-void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint64_t total_px, cudaStream_t st);
+void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint32_t nblocks, cudaStream_t st);
 bool upload_decode_tables(const uint8_t* zc, const uint8_t* sc, const uint8_t* spb, const uint32_t* mq);
 
 // Where a code-block's samples sit in its component's plane (Mallat

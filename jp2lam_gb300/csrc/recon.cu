@@ -295,46 +295,75 @@ __global__ void recon_ssim_kernel(ReconArgs r) {
 }
 
 // ------------------------------------------------------------- decoding --
-__device__ __forceinline__ uint8_t clamp_int(int32_t v) { return (uint8_t)min(max(v + 128, 0), 255); }
-__device__ __forceinline__ uint8_t clamp_round(float v) {
-  return (uint8_t)(int)fminf(fmaxf(roundf(__fadd_rn(v, 128.0f)), 0.0f), 255.0f);
+__device__ __forceinline__ uint32_t clamp_int(int32_t v) { return (uint32_t)min(max(v + 128, 0), 255); }
+__device__ __forceinline__ uint32_t clamp_round(float v) {
+  return (uint32_t)(int)fminf(fmaxf(roundf(__fadd_rn(v, 128.0f)), 0.0f), 255.0f);
 }
 
 // Inverse RCT (src/simd/scalar.rs:216-228) or ICT (scalar.rs:201-214), the
-// level shift and clamp (finalize, scalar.rs:230-242) of one sample of one
-// page, written interleaved.
-__global__ void dec_pixels_kernel(const PixJob* jobs, uint32_t njobs, uint64_t total) {
-  const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
+// level shift and clamp (finalize, scalar.rs:230-242) of sample i of a page of n,
+// as bytes from bit 0 on.
+__device__ __forceinline__ uint32_t pixel_of(const PixJob& jb, int32_t s0, int32_t s1, int32_t s2) {
+  if (jb.reversible) {
+    if (jb.mct) {
+      const int32_t gg = s0 - ((s1 + s2) >> 2);
+      return clamp_int(s2 + gg) | clamp_int(gg) << 8 | clamp_int(s1 + gg) << 16;
+    }
+    return clamp_int(s0) | clamp_int(s1) << 8 | clamp_int(s2) << 16;
+  }
+  const float yy = __int_as_float(s0), cb = __int_as_float(s1), cr = __int_as_float(s2);
+  if (jb.mct)
+    return clamp_round(__fadd_rn(yy, __fmul_rn(1.402f, cr))) |
+           clamp_round(__fadd_rn(__fadd_rn(yy, -__fmul_rn(0.34413f, cb)), -__fmul_rn(0.71414f, cr))) << 8 |
+           clamp_round(__fadd_rn(yy, __fmul_rn(1.772f, cb))) << 16;
+  return clamp_round(yy) | clamp_round(cb) << 8 | clamp_round(cr) << 16;
+}
+
+// A page's samples, written interleaved: a CTA takes kPixBlock of them, a
+// thread four in a row by 16-byte loads and 4-byte stores where the planes and
+// the output are aligned for them, else every 256th. Bound by memory: 12 sRGB
+// 2550x3300 pages 0.22 ms; a thread per sample, by byte stores, took 0.49.
+__global__ void __launch_bounds__(256) dec_pixels_kernel(const PixJob* jobs, uint32_t njobs) {
   uint32_t lo = 0, hi = njobs;
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (jobs[mid].pix_base <= g) lo = mid;
+    if (jobs[mid].block_base <= blockIdx.x) lo = mid;
     else hi = mid;
   }
-  const PixJob& jb = jobs[lo];
-  const size_t n = jb.npx, i = g - jb.pix_base;
-  uint8_t* out = jb.px + (size_t)jb.ncomp * i;
-  if (jb.reversible) {
-    const int32_t* q = jb.planes;
-    if (jb.ncomp == 3 && jb.mct) {
-      const int32_t yy = q[i], db = q[n + i], dr = q[2 * n + i];
-      const int32_t gg = yy - ((db + dr) >> 2);
-      out[0] = clamp_int(dr + gg);
-      out[1] = clamp_int(gg);
-      out[2] = clamp_int(db + gg);
+  const PixJob jb = jobs[lo];
+  const size_t n = jb.npx, first = (size_t)(blockIdx.x - jb.block_base) * kPixBlock;
+  const int32_t* q = jb.planes;
+  const bool aligned = n % 4 == 0 && reinterpret_cast<size_t>(q) % 16 == 0 && reinterpret_cast<size_t>(jb.px) % 4 == 0;
+  if (aligned) {
+    const size_t i = first + 4 * threadIdx.x;
+    if (i >= n) return;
+    const int4 z = make_int4(0, 0, 0, 0);
+    const int4 s0 = *reinterpret_cast<const int4*>(q + i);
+    const int4 s1 = jb.ncomp == 3 ? *reinterpret_cast<const int4*>(q + n + i) : z;
+    const int4 s2 = jb.ncomp == 3 ? *reinterpret_cast<const int4*>(q + 2 * n + i) : z;
+    const uint32_t p0 = pixel_of(jb, s0.x, s1.x, s2.x), p1 = pixel_of(jb, s0.y, s1.y, s2.y);
+    const uint32_t p2 = pixel_of(jb, s0.z, s1.z, s2.z), p3 = pixel_of(jb, s0.w, s1.w, s2.w);
+    uint32_t* out = reinterpret_cast<uint32_t*>(jb.px + jb.ncomp * i);
+    if (jb.ncomp == 3) {
+      out[0] = p0 | p1 << 24;
+      out[1] = p1 >> 8 | p2 << 16;
+      out[2] = p2 >> 16 | p3 << 8;
     } else {
-      for (uint32_t c = 0; c < jb.ncomp; ++c) out[c] = clamp_int(q[c * n + i]);
+      out[0] = (p0 & 0xffu) | (p1 & 0xffu) << 8 | (p2 & 0xffu) << 16 | p3 << 24;
     }
-  } else {
-    const float* f = reinterpret_cast<const float*>(jb.planes);
-    if (jb.ncomp == 3 && jb.mct) {
-      const float yy = f[i], cb = f[n + i], cr = f[2 * n + i];
-      out[0] = clamp_round(__fadd_rn(yy, __fmul_rn(1.402f, cr)));
-      out[1] = clamp_round(__fadd_rn(__fadd_rn(yy, -__fmul_rn(0.34413f, cb)), -__fmul_rn(0.71414f, cr)));
-      out[2] = clamp_round(__fadd_rn(yy, __fmul_rn(1.772f, cb)));
-    } else {
-      for (uint32_t c = 0; c < jb.ncomp; ++c) out[c] = clamp_round(f[c * n + i]);
+    return;
+  }
+  #pragma unroll
+  for (uint32_t k = 0; k < kPixBlock; k += 256) {
+    const size_t i = first + k + threadIdx.x;
+    if (i >= n) return;
+    const bool three = jb.ncomp == 3;
+    const uint32_t p = pixel_of(jb, q[i], three ? q[n + i] : 0, three ? q[2 * n + i] : 0);
+    uint8_t* out = jb.px + jb.ncomp * i;
+    out[0] = (uint8_t)p;
+    if (three) {
+      out[1] = (uint8_t)(p >> 8);
+      out[2] = (uint8_t)(p >> 16);
     }
   }
 }
@@ -378,9 +407,9 @@ void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_tiles
   idwt_kernel<<<total_tiles, kIdwtThreads, 0, st>>>(jobs, njobs);
 }
 
-void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint64_t total_px, cudaStream_t st) {
-  if (njobs == 0 || total_px == 0) return;
-  dec_pixels_kernel<<<(unsigned)((total_px + 255) / 256), 256, 0, st>>>(jobs, njobs, total_px);
+void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint32_t nblocks, cudaStream_t st) {
+  if (njobs == 0 || nblocks == 0) return;
+  dec_pixels_kernel<<<nblocks, 256, 0, st>>>(jobs, njobs);
 }
 
 void launch_recon(ReconArgs r, const std::pair<int, int>* ladder, int levels, cudaStream_t st) {
