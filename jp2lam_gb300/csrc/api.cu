@@ -116,8 +116,8 @@ struct jp2g_ctx {
   std::mutex errmu;
   std::mutex mu;    // device pools and stream: one wave (or encode) at a time
   // device pools
-  DevBuf px, px2, ll0, coef, payload, passes, res, keep, blocks, bands, comps, maxslope, hullp,
-      hulls, hulln, offsets, scratch, body, nplanes, planebase, items, itemrec, planes, signs, sym, stats,
+  DevBuf px, px2, ll0, coef, payload, passes, res, keep, blocks, bands, comps, maxslope, hulln,
+      offsets, scratch, body, nplanes, planebase, items, itemrec, planes, signs, sym, stats,
       dwtargs, dwtbases, mqorder, mqscratch, recon, reconblk, t2pk, t2bd, t2pg, t2tmpl, t2tree, t2raw, t2hdr,
       t2hdrlen, t2pktoff, t2pagelen, t2pageoff, t2nchunks, t2chunkbase, t2out;
   // pinned host staging
@@ -829,14 +829,12 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
       !reserve(c, c->bands, bands.size() * sizeof(BandParam)) ||
       !reserve(c, c->comps, comps.size() * sizeof(CompParam)) ||
       !reserve(c, c->maxslope, std::max<size_t>(comps.size(), 8) * (sizeof(unsigned long long) + 4 * sizeof(uint32_t))) ||
-      !reserve(c, c->hullp, std::max<size_t>(nb, 1) * pcap * sizeof(uint16_t)) ||
-      !reserve(c, c->hulls, std::max<size_t>(nb, 1) * pcap * sizeof(double)) ||
       !reserve(c, c->hulln, std::max<size_t>(nb, 1)) ||
       !reserve(c, c->offsets, (size_t)(nb + 1) * 4) ||
       !reserve(c, c->scratch, ((size_t)nb / 1024 + 2) * 4) ||
       !reserve(c, c->nplanes, std::max<size_t>(nb, 1) * 4) ||
       !reserve(c, c->planebase, (size_t)(nb + 1) * 4) ||
-      !reserve(c, c->body, std::max<size_t>(nb, 1) * cap) ||
+      !reserve(c, c->body, std::max<size_t>(nb, 1) * std::max<size_t>(cap, pcap * (sizeof(double) + sizeof(uint16_t)))) ||
       !reserve(c, c->stats, 64) || !reserve_host(c, c->hcount, 64))
     return kEncodeFailed;
 
@@ -897,7 +895,10 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   ta.res = dptr<BlockOut>(c->res);
   ta.nplanes = dptr<uint32_t>(c->nplanes);
   ta.plane_base = dptr<uint32_t>(c->planebase);
-  ta.sym_slot = (uint32_t)(((slot * 5 / 2 + 15) & ~size_t(15)) + 48);  // each pass padded to 16 symbols
+  // A sample gives at most two symbols, a cleanup run's four at most ten; a run
+  // that finds one is not next to another, so an item has at most 2 1/4 symbols a
+  // sample, and its three passes' padding to 16 fits what is left of 2 1/2.
+  ta.sym_slot = (uint32_t)((slot * 5 / 2 + 15) & ~size_t(15));
   ta.sym_count = dptr<unsigned long long>(c->stats);
   ta.bands = dptr<BandParam>(c->bands);
   ta.comps = dptr<CompParam>(c->comps);
@@ -996,8 +997,9 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   pa.comps = dptr<CompParam>(c->comps);
   pa.comp_max_slope = dptr<unsigned long long>(c->maxslope);
   pa.ncomp_keys = (uint32_t)comps.size();
-  pa.hull_passes = dptr<uint16_t>(c->hullp);
-  pa.hull_slope = dptr<double>(c->hulls);
+  // the hulls lie where compaction writes the retained bytes afterwards
+  pa.hull_slope = dptr<double>(c->body);
+  pa.hull_passes = reinterpret_cast<uint16_t*>(pa.hull_slope + (size_t)nb * pcap);
   pa.hull_n = dptr<uint8_t>(c->hulln);
   pa.keep = dptr<BlockKeep>(c->keep);
   launch_pcrd(pa, c->num_sms, c->stream);
@@ -1062,7 +1064,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
 void release_pools(jp2g_ctx* c) {
   cudaStreamSynchronize(c->stream);
   DevBuf* bufs[] = {&c->px, &c->px2, &c->ll0, &c->coef, &c->payload, &c->passes, &c->res, &c->keep,
-                    &c->blocks, &c->bands, &c->comps, &c->maxslope, &c->hullp, &c->hulls, &c->hulln,
+                    &c->blocks, &c->bands, &c->comps, &c->maxslope, &c->hulln,
                     &c->offsets, &c->scratch, &c->body, &c->nplanes, &c->planebase, &c->items,
                     &c->itemrec, &c->planes, &c->signs, &c->sym, &c->stats, &c->dwtargs, &c->dwtbases,
                     &c->mqorder, &c->mqscratch, &c->recon, &c->reconblk, &c->t2pk, &c->t2bd, &c->t2pg,
@@ -1281,7 +1283,7 @@ void jp2g_destroy(jp2g_ctx* c) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   DevBuf* bufs[] = {&c->px, &c->px2, &c->ll0, &c->coef, &c->payload, &c->passes, &c->res, &c->keep,
-                    &c->blocks, &c->bands, &c->comps, &c->maxslope, &c->hullp, &c->hulls, &c->hulln,
+                    &c->blocks, &c->bands, &c->comps, &c->maxslope, &c->hulln,
                     &c->offsets, &c->scratch, &c->body, &c->nplanes, &c->planebase, &c->items,
                     &c->itemrec, &c->planes, &c->signs, &c->sym, &c->stats, &c->dwtargs, &c->dwtbases,
                     &c->mqorder, &c->mqscratch, &c->recon, &c->reconblk, &c->t2pk, &c->t2bd, &c->t2pg,
@@ -1479,7 +1481,7 @@ size_t half_plane_bytes(const DecodePage& p) {
 uint64_t decode_device_bytes(const DecodePage& p, size_t nbytes) {
   // bytes, planes, tmp planes or masks, samples, code-blocks, jobs
   uint64_t masks = 0;
-  for (const DecBlock& b : p.L.blocks) masks += 8ull * dec_mask_words(b.npasses);
+  for (const DecBlock& b : p.L.blocks) masks += 8ull * dec_mask_words(b.w, b.npasses);
   return nbytes + p.npx * p.L.ncomp * 4 + std::max<uint64_t>(p.npx, half_plane_bytes(p)) * p.L.ncomp +
          std::max<uint64_t>(p.npx * p.L.ncomp * 4, masks) + p.L.blocks.size() * sizeof(DecBlock) +
          (uint64_t)(p.L.levels * p.L.ncomp + 1) * sizeof(IdwtJob) + sizeof(PixJob) + 1024;
@@ -1511,7 +1513,7 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
       b.plane_off += pg[i].plane_base;
       b.data_off += (uint32_t)pg[i].data_base;
       b.mask_off = mask_words;
-      mask_words += dec_mask_words(b.npasses);
+      mask_words += dec_mask_words(b.w, b.npasses);
       blk.push_back(b);
     }
   // the blocks' masks lie where the inverse DWT's scratch planes come later

@@ -199,7 +199,7 @@ void launch_t2(const T2Args& a, uint32_t* scan_scratch, int num_sms, cudaStream_
 // One code-block of a codestream being decoded.
 struct DecBlock {
   uint64_t plane_off;           // its first sample in the planes buffer (elements)
-  uint64_t mask_off;            // its masks (64-bit words): 64 columns per decoded bit-plane, then its signs
+  uint64_t mask_off;            // its masks (64-bit words): its columns per decoded bit-plane, then its signs
   uint32_t data_off, data_len;  // its segment in the input bytes
   uint32_t stride;              // its plane's row pitch (the image width)
   uint16_t w, h;
@@ -255,8 +255,8 @@ struct PixJob {
 constexpr uint32_t kPixBlock = 1024;  // samples per CTA
 // Bit-planes that a block's passes reach: its top one in one pass, then three each.
 JP2G_HD uint32_t dec_planes(uint32_t npasses) { return npasses ? (npasses + 4) / 3 : 0; }
-// 64-bit words of a block's masks.
-JP2G_HD uint32_t dec_mask_words(uint32_t npasses) { return npasses ? 64 * (dec_planes(npasses) + 1) : 0; }
+// 64-bit words of a block's masks, one per column and bit-plane and one for the signs.
+JP2G_HD uint32_t dec_mask_words(uint32_t w, uint32_t npasses) { return npasses ? w * (dec_planes(npasses) + 1) : 0; }
 // Tier-1 decoding of every code-block into coefficients (t1dec.cu). masks: the
 // blocks' masks; scratch: nblocks + 2048 words.
 void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, unsigned long long* masks,

@@ -10,6 +10,9 @@
 //
 // 1. t1_analyze_kernel (warp per block): max magnitude, non-zero count ->
 //    magnitude bit-planes, zero bit-planes, block class.
+//    t1_planes_kernel (warp per block): column masks per bit-plane, and from
+//    their counts which bit-planes to model and how many symbols to expect;
+//    t1_split_kernel: the blocks with the most, to be modelled and coded first.
 // 2. t1_model_kernel (warp per (block, bit-plane)): the significance state
 //    at the start of bit-plane p is known in closed form (|q| >> (p+1) != 0),
 //    and so is the refinement history (|q| >> (p+2) != 0), so every
@@ -22,7 +25,8 @@
 //    columns (one lane per column), into a per-bit-plane symbol slot.
 // 3. t1_mq_kernel (lane per block): runs the MQ coder over a block's symbol
 //    streams, top bit-plane first, recording numbytes() after every pass
-//    and writing the byte stream to the block's payload slot.
+//    and writing the byte stream to the block's payload slot, until rate
+//    control can choose none of the passes to come (Stop).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -668,10 +672,11 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a,
 // - Each pass's symbols are padded to whole 16-symbol chunks with symbols that
 //   change nothing (t1_model_kernel), so a pass ends between two chunks.
 //
-// Measured (2550x3300 gray q85 page; batch of 24 sRGB q75 pages): MQ stage 3.04
-// and 5.2 ms (403 G symbols/s); 4.38 and 11.1 ms with an integer coder, split
-// over producer/consumer warp pairs on the page, branching at its byte output
-// in the batch. A lone chain takes 90 cycles per symbol; 106 when predicates
+// Measured with every pass coded (2550x3300 gray q85 page; batch of 24 sRGB q75
+// pages): 3.04 and 5.2 ms; 4.38 and 11.1 ms with an integer coder split over two
+// warps on the page and branching at its byte output in the batch. Now that
+// blocks stop early the page's takes 1.6 ms. A lone chain takes 90 cycles per
+// symbol (32 lanes and 16 warps per SM: 490 G symbols/s); 106 when predicates
 // chose between A and Qe, and a renormalised context's state was read only then.
 //
 // Context entry, in shared memory: x = Qe / 2^15 as a float, its sign bit the

@@ -385,15 +385,15 @@ __global__ void __launch_bounds__(kDecWarps * 32) t1_decode_kernel(const DecBloc
     dec.run_pass(pass);
     --left;
     if (pass == 2 || left == 0) {  // the bit-plane's masks
-      out[lane] = dec.col[0].ones;
-      out[lane + 32] = dec.col[1].ones;
+      if ((int)lane < d.w) out[lane] = dec.col[0].ones;
+      if ((int)lane + 32 < d.w) out[lane + 32] = dec.col[1].ones;
       dec.col[0].ones = dec.col[1].ones = 0;
-      out += 64;
+      out += d.w;
     }
     pass = pass == 2 ? 0 : pass + 1;
   }
-  out[lane] = dec.col[0].sgn;
-  out[lane + 32] = dec.col[1].sgn;
+  if ((int)lane < d.w) out[lane] = dec.col[0].sgn;
+  if ((int)lane + 32 < d.w) out[lane + 32] = dec.col[1].sgn;
 }
 
 // Coefficients of every code-block from its masks, a warp per block: a lane
@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(128) t1_coefficients_kernel(const DecBlock* bl
       #pragma unroll
       for (int k = 0; k < 32; ++k) {
         const int j = top - k;  // bit-plane k is the block's plane j
-        t[k] = j >= 0 && j < np ? mw[(64 * j + x) * 2 + half] : 0u;
+        t[k] = j >= 0 && j < np ? mw[(d.w * j + x) * 2 + half] : 0u;
       }
-      const uint32_t sg = np > 0 ? mw[(64 * np + x) * 2 + half] : 0u;
+      const uint32_t sg = np > 0 ? mw[(d.w * np + x) * 2 + half] : 0u;
       transpose32(t);
       #pragma unroll
       for (int i = 0; i < 32; ++i) {
