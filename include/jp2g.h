@@ -106,7 +106,7 @@ int jp2g_decode(jp2g_ctx* ctx, const uint8_t* bytes, size_t n, int flags, uint8_
 
 /* jp2g_decode over n files at once (bytes[i], lens[i]): the files share
  * device launches (one Tier-1 decoding launch over all their code-blocks,
- * one inverse-DWT launch pair per level, one for the samples), in rounds
+ * one inverse-DWT launch per level, one for the samples), in rounds
  * that fit the device memory budget. Per file: outs[i]/out_lens[i] (free
  * with jp2g_free), ws/hs/ncomps and status[i]; one file's failure does not
  * fail the others. Returns JP2G_OK or the first failing file's status (its
