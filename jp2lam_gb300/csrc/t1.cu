@@ -867,7 +867,8 @@ __device__ __forceinline__ void mq_chunk16(Mq& m, MqSmem& sm, uint32_t lane, con
 // lambda, or a half, a quarter or an eighth as large: lambda is then at least
 // that share of lambda_raw, and the block, measured with it, may stop unless a
 // later pass could still raise the largest slope. A block that has not been
-// stopped gives its largest slope as before.
+// stopped gives its largest slope as before. A block's last pass shows no
+// slope: it takes the termination's bytes too, which are not in its count yet.
 //
 // The sums are f32: `slack` bounds their rounding against the f64 curve (a
 // term is within 1e-6 of its value, and each of at most 124 passes adds two
@@ -992,6 +993,7 @@ __device__ __forceinline__ void mq_code_block(const T1Args& a, uint32_t b, MqSme
     else
       *pr = PassRec{pos, 0u, r.sig_before, 1, bp, 0};
     ++pr;
+    if (k == 2 && j + 1 == mbp) return;  // the last pass: its bytes are known only after termination
     stop.pass(pos, k == 2 ? 0.85f * (float)r.ns_cl : (k == 0 ? (float)r.ns_sp : 0.25f * (float)r.sig_before), bp);
   };
   // the first pass of item j that has symbols
