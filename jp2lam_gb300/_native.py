@@ -74,14 +74,12 @@ class Request(ctypes.Structure):
                 ("ncomp", ctypes.c_uint32), ("interleaved", ctypes.c_int32), ("on_device", ctypes.c_int32),
                 ("quality", ctypes.c_int32), ("format", ctypes.c_int32)]
 
-# jp2g_result_alloc, and the bytes objects whose memory it hands out
+# jp2g_result_alloc, and the bytes objects whose memory it hands out (prototypes
+# of their own: ctypes.pythonapi's functions are shared by the whole process)
 _ResultAlloc = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_size_t)
-_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.restype = ctypes.py_object
-_new_bytes.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
-_bytes_at = ctypes.pythonapi.PyBytes_AsString
-_bytes_at.restype = ctypes.c_void_p
-_bytes_at.argtypes = [ctypes.py_object]
+_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
+_bytes_at = ctypes.PYFUNCTYPE(ctypes.c_void_p, ctypes.py_object)(("PyBytes_AsString", ctypes.pythonapi))
 
 _lib = None
 _lock = threading.Lock()
