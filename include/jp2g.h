@@ -84,6 +84,24 @@ int jp2g_encode_with_psnr(jp2g_ctx* ctx, const uint8_t* px, uint32_t w, uint32_t
 typedef uint8_t* (*jp2g_result_alloc)(void* user, uint32_t index, size_t bytes);
 int jp2g_set_result_alloc(jp2g_ctx* ctx, jp2g_result_alloc alloc, void* user);
 
+/* A jp2g_result_alloc, its user a jp2g_py_results, whose memory is that of new
+ * Python bytes objects, made by the interpreter's own functions. It runs no
+ * Python code, so that no signal handler of the host program runs, or raises,
+ * inside an encode call; without memory it returns NULL. objects: n slots, null
+ * at first, that receive references owned by the caller; an object that a
+ * later call for the same index replaces is released. */
+typedef struct jp2g_py_results {
+  int (*gil_ensure)(void);                          /* PyGILState_Ensure */
+  void (*gil_release)(int);                         /* PyGILState_Release */
+  void* (*new_bytes)(const char* bytes, ptrdiff_t); /* PyBytes_FromStringAndSize */
+  char* (*bytes_at)(void* object);                  /* PyBytes_AsString */
+  void (*clear_error)(void);                        /* PyErr_Clear */
+  void (*decref)(void* object);                     /* Py_DecRef */
+  void** objects;
+  uint32_t n;
+} jp2g_py_results;
+uint8_t* jp2g_py_result_alloc(void* user, uint32_t index, size_t bytes);
+
 /* Decodes a J2K or JP2 file as decode_jp2 does (src/decode/mod.rs:56-61):
  * single tile, one quality layer, LRCP, one precinct per resolution, 8-bit
  * gray or 3-component, 64x64 or smaller code-blocks — the codestreams this

@@ -54,7 +54,7 @@ EXPORTS = [
     "jp2g_encode_batch", "jp2g_submit", "jp2g_poll", "jp2g_set_option", "jp2g_get_option",
     "jp2g_autotune", "jp2g_debug_assemble", "jp2g_debug_plan", "jp2g_cancel", "jp2g_debug_context_labels",
     "jp2g_debug_coefficients_f32", "jp2g_encode_with_psnr", "jp2g_debug_assemble_device", "jp2g_decode",
-    "jp2g_decode_batch", "jp2g_set_result_alloc",
+    "jp2g_decode_batch", "jp2g_set_result_alloc", "jp2g_py_result_alloc",
 ]
 
 PENDING = 6
@@ -74,12 +74,47 @@ class Request(ctypes.Structure):
                 ("ncomp", ctypes.c_uint32), ("interleaved", ctypes.c_int32), ("on_device", ctypes.c_int32),
                 ("quality", ctypes.c_int32), ("format", ctypes.c_int32)]
 
-# jp2g_result_alloc, and the bytes objects whose memory it hands out (prototypes
-# of their own: ctypes.pythonapi's functions are shared by the whole process)
+# jp2g_result_alloc
 _ResultAlloc = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_size_t)
-_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(
-    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
-_bytes_at = ctypes.PYFUNCTYPE(ctypes.c_void_p, ctypes.py_object)(("PyBytes_AsString", ctypes.pythonapi))
+
+
+class _PyResults(ctypes.Structure):
+    """jp2g_py_results"""
+    _fields_ = [("api", ctypes.c_void_p * 6), ("objects", ctypes.POINTER(ctypes.c_void_p)),
+                ("n", ctypes.c_uint32)]
+
+
+_PY_API = (ctypes.c_void_p * 6)(*[ctypes.cast(getattr(ctypes.pythonapi, f), ctypes.c_void_p).value for f in (
+    "PyGILState_Ensure", "PyGILState_Release", "PyBytes_FromStringAndSize", "PyBytes_AsString", "PyErr_Clear",
+    "Py_DecRef")])
+# a prototype of its own: ctypes.pythonapi's functions are shared by the whole process
+_decref = ctypes.PYFUNCTYPE(None, ctypes.c_void_p)(("Py_DecRef", ctypes.pythonapi))
+
+
+class _Results:
+    """The codestreams of one encode call, which the library writes straight
+    into new bytes objects while the object is entered."""
+
+    def __init__(self, engine: "Engine", n: int):
+        self._engine = engine
+        self._objects = (ctypes.c_void_p * max(n, 1))()
+        self._results = _PyResults(_PY_API, self._objects, n)
+
+    def __enter__(self):
+        lib = self._engine.lib
+        lib.jp2g_set_result_alloc(self._engine.handle, lib.jp2g_py_result_alloc, ctypes.byref(self._results))
+        return self
+
+    def __exit__(self, *_):
+        self._engine.lib.jp2g_set_result_alloc(self._engine.handle, None, None)
+
+    def __getitem__(self, i: int) -> bytes:
+        return ctypes.cast(self._objects[i], ctypes.py_object).value
+
+    def __del__(self):
+        for p in self._objects:
+            if p:
+                _decref(p)
 
 _lib = None
 _lock = threading.Lock()
@@ -104,7 +139,9 @@ def load_library(path: str = LIB_PATH):
                                            ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint8, ctypes.c_int,
                                            ctypes.POINTER(_u8p), ctypes.POINTER(ctypes.c_size_t)]
         lib.jp2g_free.argtypes = [_u8p]
-        lib.jp2g_set_result_alloc.argtypes = [ctypes.c_void_p, _ResultAlloc, ctypes.c_void_p]
+        lib.jp2g_set_result_alloc.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+        lib.jp2g_py_result_alloc.argtypes = [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_size_t]
+        lib.jp2g_py_result_alloc.restype = ctypes.c_void_p
         lib.jp2g_last_error.argtypes = [ctypes.c_void_p]
         lib.jp2g_last_error.restype = ctypes.c_char_p
         lib.jp2g_stream.argtypes = [ctypes.c_void_p]
@@ -173,16 +210,6 @@ class Engine:
             _raise(rc, self.lib.jp2g_last_error(None).decode())
         self.handle = h
         self._lock = threading.Lock()
-        # codestreams are written straight into new bytes objects; filled by
-        # the library during a call (under _lock), by index
-        results = self._results = {}
-
-        def alloc(_, index, n):
-            results[index] = data = _new_bytes(None, n)
-            return _bytes_at(data)
-
-        self._alloc = _ResultAlloc(alloc)
-        self.lib.jp2g_set_result_alloc(h, self._alloc, None)
         self._inflight = {}  # ticket -> pixel buffer kept alive until polled
         self._inflight_lock = threading.Lock()
 
@@ -197,12 +224,6 @@ class Engine:
         except Exception:
             pass
 
-    def _take(self, rc: int) -> bytes:
-        """The codestream of a single-page call; called under _lock."""
-        data = self._results.pop(0, None)
-        self._check(rc)
-        return data
-
     def _check(self, rc: int):
         if rc != 0:
             _raise(rc, self.lib.jp2g_last_error(self.handle).decode())
@@ -215,10 +236,11 @@ class Engine:
             raise InvalidInput("pixel buffer length does not match the image dimensions")
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock:
+        with self._lock, _Results(self, 1) as results:
             rc = self.lib.jp2g_encode(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                       int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n))
-            return self._take(rc)
+            self._check(rc)
+        return results[0]
 
     def encode_with_psnr(self, px, w: int, h: int, ncomp: int, quality: int, fmt: int,
                          interleaved: bool = True):
@@ -231,11 +253,12 @@ class Engine:
         out = _u8p()
         n = ctypes.c_size_t()
         psnr, ssim = ctypes.c_double(), ctypes.c_double()
-        with self._lock:
+        with self._lock, _Results(self, 1) as results:
             rc = self.lib.jp2g_encode_with_psnr(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                                 int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n),
                                                 ctypes.byref(psnr), ctypes.byref(ssim))
-            return self._take(rc), psnr.value, ssim.value
+            self._check(rc)
+        return results[0], psnr.value, ssim.value
 
     @staticmethod
     def _decode_flags(rct_chroma_extra_bitplane, accept_empty_segments):
@@ -298,10 +321,11 @@ class Engine:
     def encode_device(self, dev_ptr: int, w: int, h: int, ncomp: int, quality: int, fmt: int) -> bytes:
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock:
+        with self._lock, _Results(self, 1) as results:
             rc = self.lib.jp2g_encode_device(self.handle, ctypes.c_void_p(dev_ptr), w, h, ncomp, quality,
                                              fmt, ctypes.byref(out), ctypes.byref(n))
-            return self._take(rc)
+            self._check(rc)
+        return results[0]
 
     @staticmethod
     def _request(page, keep):
@@ -333,11 +357,9 @@ class Engine:
         outs = (_u8p * max(n, 1))()
         lens = (ctypes.c_size_t * max(n, 1))()
         status = (ctypes.c_int * max(n, 1))()
-        with self._lock:
+        with self._lock, _Results(self, n) as files:
             rc = self.lib.jp2g_encode_batch(self.handle, reqs, n, outs, lens, status)
             msg = self.lib.jp2g_last_error(self.handle).decode() if rc != 0 else ""
-            files = dict(self._results)
-            self._results.clear()
         result = []
         for i in range(n):
             if status[i] == 0:
