@@ -78,11 +78,17 @@ int jp2g_encode_with_psnr(jp2g_ctx* ctx, const uint8_t* px, uint32_t w, uint32_t
  * and jp2g_encode_batch (index: the request's) ask alloc for the codestream's
  * bytes once its length is known, write into what it returns and return that
  * pointer, which is not for jp2g_free. alloc runs on the calling thread, may be
- * called more than once for an index (the last one counts) and may return
- * NULL (JP2G_ENCODE_FAILED). A null alloc: malloc again. Served requests
+ * called more than once for an index (the last one counts), must not call
+ * into the context (which is locked) and may return NULL
+ * (JP2G_ENCODE_FAILED). A null alloc: malloc again. Served requests
  * (jp2g_submit) always use malloc. */
 typedef uint8_t* (*jp2g_result_alloc)(void* user, uint32_t index, size_t bytes);
 int jp2g_set_result_alloc(jp2g_ctx* ctx, jp2g_result_alloc alloc, void* user);
+
+/* The same for the encode calls that the calling thread makes, on any context,
+ * in place of the context's own allocator; a null alloc ends it. Other threads'
+ * calls are not affected. */
+void jp2g_set_thread_result_alloc(jp2g_result_alloc alloc, void* user);
 
 /* A jp2g_result_alloc, its user a jp2g_py_results, whose memory is that of new
  * Python bytes objects, made by the interpreter's own functions. It runs no

@@ -54,7 +54,7 @@ EXPORTS = [
     "jp2g_encode_batch", "jp2g_submit", "jp2g_poll", "jp2g_set_option", "jp2g_get_option",
     "jp2g_autotune", "jp2g_debug_assemble", "jp2g_debug_plan", "jp2g_cancel", "jp2g_debug_context_labels",
     "jp2g_debug_coefficients_f32", "jp2g_encode_with_psnr", "jp2g_debug_assemble_device", "jp2g_decode",
-    "jp2g_decode_batch", "jp2g_set_result_alloc", "jp2g_py_result_alloc",
+    "jp2g_decode_batch", "jp2g_set_result_alloc", "jp2g_py_result_alloc", "jp2g_set_thread_result_alloc",
 ]
 
 PENDING = 6
@@ -93,20 +93,21 @@ _decref = ctypes.PYFUNCTYPE(None, ctypes.c_void_p)(("Py_DecRef", ctypes.pythonap
 
 class _Results:
     """The codestreams of one encode call, which the library writes straight
-    into new bytes objects while the object is entered."""
+    into new bytes objects. While it is entered, that is where the thread's
+    encode calls put them; calls on the C ABI by other threads, or outside of
+    it, return memory for jp2g_free."""
 
-    def __init__(self, engine: "Engine", n: int):
-        self._engine = engine
+    def __init__(self, lib, n: int):
+        self._lib = lib
         self._objects = (ctypes.c_void_p * max(n, 1))()
         self._results = _PyResults(_PY_API, self._objects, n)
 
     def __enter__(self):
-        lib = self._engine.lib
-        lib.jp2g_set_result_alloc(self._engine.handle, lib.jp2g_py_result_alloc, ctypes.byref(self._results))
+        self._lib.jp2g_set_thread_result_alloc(self._lib.jp2g_py_result_alloc, ctypes.byref(self._results))
         return self
 
     def __exit__(self, *_):
-        self._engine.lib.jp2g_set_result_alloc(self._engine.handle, None, None)
+        self._lib.jp2g_set_thread_result_alloc(None, None)
 
     def __getitem__(self, i: int) -> bytes:
         return ctypes.cast(self._objects[i], ctypes.py_object).value
@@ -140,6 +141,8 @@ def load_library(path: str = LIB_PATH):
                                            ctypes.POINTER(_u8p), ctypes.POINTER(ctypes.c_size_t)]
         lib.jp2g_free.argtypes = [_u8p]
         lib.jp2g_set_result_alloc.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+        lib.jp2g_set_thread_result_alloc.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+        lib.jp2g_set_thread_result_alloc.restype = None
         lib.jp2g_py_result_alloc.argtypes = [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_size_t]
         lib.jp2g_py_result_alloc.restype = ctypes.c_void_p
         lib.jp2g_last_error.argtypes = [ctypes.c_void_p]
@@ -236,7 +239,7 @@ class Engine:
             raise InvalidInput("pixel buffer length does not match the image dimensions")
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock, _Results(self, 1) as results:
+        with self._lock, _Results(self.lib, 1) as results:
             rc = self.lib.jp2g_encode(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                       int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n))
             self._check(rc)
@@ -253,7 +256,7 @@ class Engine:
         out = _u8p()
         n = ctypes.c_size_t()
         psnr, ssim = ctypes.c_double(), ctypes.c_double()
-        with self._lock, _Results(self, 1) as results:
+        with self._lock, _Results(self.lib, 1) as results:
             rc = self.lib.jp2g_encode_with_psnr(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                                 int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n),
                                                 ctypes.byref(psnr), ctypes.byref(ssim))
@@ -321,7 +324,7 @@ class Engine:
     def encode_device(self, dev_ptr: int, w: int, h: int, ncomp: int, quality: int, fmt: int) -> bytes:
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock, _Results(self, 1) as results:
+        with self._lock, _Results(self.lib, 1) as results:
             rc = self.lib.jp2g_encode_device(self.handle, ctypes.c_void_p(dev_ptr), w, h, ncomp, quality,
                                              fmt, ctypes.byref(out), ctypes.byref(n))
             self._check(rc)
@@ -357,7 +360,7 @@ class Engine:
         outs = (_u8p * max(n, 1))()
         lens = (ctypes.c_size_t * max(n, 1))()
         status = (ctypes.c_int * max(n, 1))()
-        with self._lock, _Results(self, n) as files:
+        with self._lock, _Results(self.lib, n) as files:
             rc = self.lib.jp2g_encode_batch(self.handle, reqs, n, outs, lens, status)
             msg = self.lib.jp2g_last_error(self.handle).decode() if rc != 0 else ""
         result = []

@@ -59,14 +59,15 @@ struct HostBuf {
 enum Stage { kH2D = 0, kDWT, kT1, kPCRD, kCompact, kD2H, kHost, kTotal, kNumStages };
 enum SubEvent { kEvAnalyzeEnd = kNumStages + 1, kEvModelEnd, kEvT2End, kNumEvents };
 
-// One page of a wave: its request, its plan and, after the device phase,
-// the page-local retained blocks and bytes that Tier-2 needs.
-// jp2g_set_result_alloc
+// jp2g_set_result_alloc, jp2g_set_thread_result_alloc
 struct ResultAlloc {
   jp2g_result_alloc fn = nullptr;
   void* user = nullptr;
 };
+thread_local ResultAlloc t_result_alloc;
 
+// One page of a wave: its request, its plan and, after the device phase,
+// the page-local retained blocks and bytes that Tier-2 needs.
 struct PageJob {
   const uint8_t* host_px = nullptr;
   const uint8_t* dev_px = nullptr;
@@ -171,6 +172,9 @@ struct jp2g_ctx {
 };
 
 namespace {
+
+// The allocator of the calling thread's encode calls.
+ResultAlloc result_alloc(const jp2g_ctx* c) { return t_result_alloc.fn ? t_result_alloc : c->result_alloc; }
 
 void set_msg(jp2g_ctx* c, const std::string& m) {
   std::lock_guard<std::mutex> lk(c->errmu);
@@ -1347,7 +1351,7 @@ int jp2g_encode(jp2g_ctx* c, const uint8_t* px, uint32_t w, uint32_t h, uint32_t
   if (!px) return set_err(c, JP2G_INVALID_INPUT, "pixel pointer is null");
   cudaSetDevice(c->device);
   PageJob j;
-  j.alloc = c->result_alloc;
+  j.alloc = result_alloc(c);
   j.host_px = px;
   j.w = w;
   j.h = h;
@@ -1367,7 +1371,7 @@ int jp2g_encode_device(jp2g_ctx* c, const uint8_t* d_px, uint32_t w, uint32_t h,
   if (!d_px) return set_err(c, JP2G_INVALID_INPUT, "pixel pointer is null");
   cudaSetDevice(c->device);
   PageJob j;
-  j.alloc = c->result_alloc;
+  j.alloc = result_alloc(c);
   j.dev_px = d_px;
   j.w = w;
   j.h = h;
@@ -1449,7 +1453,7 @@ int jp2g_encode_with_psnr(jp2g_ctx* c, const uint8_t* px, uint32_t w, uint32_t h
   if (!px) return set_err(c, JP2G_INVALID_INPUT, "pixel pointer is null");
   cudaSetDevice(c->device);
   PageJob j;
-  j.alloc = c->result_alloc;
+  j.alloc = result_alloc(c);
   j.host_px = px;
   j.w = w;
   j.h = h;
@@ -1767,7 +1771,7 @@ static int encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8
   std::vector<PageJob*> ptrs(n);
   for (uint32_t i = 0; i < n; ++i) {
     job_from_request(reqs[i], &jobs[i]);
-    if (!own_results) jobs[i].alloc = c->result_alloc;
+    if (!own_results) jobs[i].alloc = result_alloc(c);
     jobs[i].index = i;
     ptrs[i] = &jobs[i];
     outs[i] = nullptr;
@@ -2299,6 +2303,8 @@ int jp2g_set_result_alloc(jp2g_ctx* c, jp2g_result_alloc alloc, void* user) {
   c->result_alloc = {alloc, user};
   return JP2G_OK;
 }
+
+void jp2g_set_thread_result_alloc(jp2g_result_alloc alloc, void* user) { t_result_alloc = {alloc, user}; }
 
 const char* jp2g_last_error(jp2g_ctx* c) { return c ? c->err.c_str() : g_create_error.c_str(); }
 

@@ -2,6 +2,7 @@
 import ctypes
 import signal
 import sys
+import threading
 
 import numpy as np
 import pytest
@@ -16,18 +17,10 @@ def test_importing_leaves_pythonapi_prototypes_alone():
         assert f.restype is ctypes.c_int and f.argtypes is None
 
 
-class _NoEngine:
-    """As much of an Engine as _Results needs without a GPU."""
-    handle = None
-
-    def __init__(self):
-        self.lib = _native.load_library()
-
-
 def test_result_alloc_without_memory_returns_null():
-    eng = _NoEngine()
-    results = _native._Results(eng, 2)
-    alloc = lambda i, n: eng.lib.jp2g_py_result_alloc(ctypes.byref(results._results), i, n)  # noqa: E731
+    lib = _native.load_library()
+    results = _native._Results(lib, 2)
+    alloc = lambda i, n: lib.jp2g_py_result_alloc(ctypes.byref(results._results), i, n)  # noqa: E731
     for n in (1 << 62, 1 << 63, (1 << 64) - 1):
         assert alloc(0, n) is None
     assert alloc(2, 10) is None  # not an index of the call
@@ -38,9 +31,9 @@ def test_result_alloc_without_memory_returns_null():
 
 
 def test_result_objects_are_released_once():
-    eng = _NoEngine()
-    results = _native._Results(eng, 1)
-    alloc = lambda n: eng.lib.jp2g_py_result_alloc(ctypes.byref(results._results), 0, n)  # noqa: E731
+    lib = _native.load_library()
+    results = _native._Results(lib, 1)
+    alloc = lambda n: lib.jp2g_py_result_alloc(ctypes.byref(results._results), 0, n)  # noqa: E731
     alloc(1000)
     first = results[0]
     mine = sys.getrefcount(first) - 1  # without the slot's
@@ -76,4 +69,75 @@ def test_signal_handler_that_raises_during_an_encode():
     finally:
         signal.setitimer(signal.ITIMER_REAL, 0)
         signal.signal(signal.SIGALRM, before)
+        eng.close()
+
+
+def _raw_encode(eng, px, w, h, c, q):
+    """jp2g_encode on an engine's context and jp2g_free, as a C caller has them."""
+    out, n = _native._u8p(), ctypes.c_size_t()
+    rc = eng.lib.jp2g_encode(eng.handle, px.ctypes.data_as(ctypes.c_void_p), w, h, c, 1, q, 0, ctypes.byref(out),
+                             ctypes.byref(n))
+    assert rc == 0
+    data = ctypes.string_at(out, n.value)
+    eng.lib.jp2g_free(out)
+    return data
+
+
+@pytest.mark.gpu
+def test_raw_calls_on_an_engines_context_own_their_results(orc):
+    w, h = 200, 150
+    px = np.random.default_rng(2).integers(0, 256, w * h, dtype=np.uint8)
+    want = orc.encode(px, w, h, 1, 80, 0)
+    eng = jl.Engine(0)
+    try:
+        assert eng.encode(px, w, h, 1, 80, 0) == want
+        assert _raw_encode(eng, px, w, h, 1, 80) == want
+        raw = []
+
+        def other():
+            for _ in range(100):
+                raw.append(_raw_encode(eng, px, w, h, 1, 80))
+
+        t = threading.Thread(target=other)
+        t.start()
+        while t.is_alive():
+            page = {"px": px, "w": w, "h": h, "ncomp": 1, "quality": 80, "fmt": 0}
+            assert eng.encode_batch([page, page]) == [want, want]
+        t.join()
+        assert raw == [want] * 100
+    finally:
+        eng.close()
+
+
+@pytest.mark.gpu
+def test_result_alloc_of_a_context(orc):
+    # a context's allocator: asked by the encode calls of any thread but the
+    # engine's own and those with one of theirs; null ends it
+    w, h = 120, 90
+    px = np.random.default_rng(3).integers(0, 256, w * h, dtype=np.uint8)
+    want = orc.encode(px, w, h, 1, 60, 0)
+    eng = jl.Engine(0)
+    memory = np.zeros(1 << 20, np.uint8)
+
+    @_native._ResultAlloc
+    def alloc(user, index, n):
+        return memory.ctypes.data if index == 0 and n <= memory.size else None
+
+    def raw():
+        out, n = _native._u8p(), ctypes.c_size_t()
+        rc = eng.lib.jp2g_encode(eng.handle, px.ctypes.data_as(ctypes.c_void_p), w, h, 1, 1, 60, 0,
+                                 ctypes.byref(out), ctypes.byref(n))
+        assert rc == 0
+        return ctypes.cast(out, ctypes.c_void_p).value, n.value
+
+    try:
+        assert eng.lib.jp2g_set_result_alloc(eng.handle, alloc, None) == 0
+        at, n = raw()
+        assert at == memory.ctypes.data and memory[:n].tobytes() == want
+        memory[:n] = 0
+        assert eng.encode(px, w, h, 1, 60, 0) == want
+        assert not memory[:n].any()
+        assert eng.lib.jp2g_set_result_alloc(eng.handle, None, None) == 0
+        assert _raw_encode(eng, px, w, h, 1, 60) == want
+    finally:
         eng.close()
