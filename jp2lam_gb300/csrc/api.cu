@@ -725,8 +725,7 @@ int run_tier2(jp2g_ctx* c, const std::vector<PageJob*>& live, const BlockKeep* d
   a.nchunks = dptr<uint32_t>(c->t2nchunks);
   a.chunk_base = dptr<uint32_t>(c->t2chunkbase);
   a.out = dptr<uint8_t>(c->t2out);
-  launch_t2(a, dptr<uint32_t>(c->scratch), c->num_sms, c->stream);
-  c->counters[5] += 6 + (npg > 1024 ? 1 : 0) + (npk > 1024 ? 1 : 0);
+  c->counters[5] += launch_t2(a, dptr<uint32_t>(c->scratch), c->num_sms, c->stream);
   record(c, kEvT2End);
   const uint32_t* hoff = reinterpret_cast<const uint32_t*>(c->hpageoff.p);
   if (!cuda_ok(c, cudaMemcpyAsync(c->hpageoff.p, a.page_off, (npg + 1) * 4, cudaMemcpyDeviceToHost, c->stream),
@@ -912,7 +911,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
       (ta.settled && !cuda_ok(c, cudaMemsetAsync(ta.settled, 0, comps.size() * 16, c->stream), "memset")))
     return kEncodeFailed;
   launch_t1_analyze(ta, c->stream);
-  launch_scan_u32(ta.nplanes, 1, nb, ta.plane_base, dptr<uint32_t>(c->scratch), c->stream);
+  c->counters[5] += launch_scan_u32(ta.nplanes, 1, nb, ta.plane_base, dptr<uint32_t>(c->scratch), c->stream);
   // The number of (block, bit-plane) items sizes the symbol buffer. Up to two
   // blocks per SM, and without a memory budget, the most there can be serves as
   // well (some 40 MB), and the device need not wait for the host to read the
@@ -996,7 +995,9 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
     launch_t1_model(ta, c->num_sms, kT1Again, c->stream);
     launch_t1_mq(ta, c->num_sms, bpw, kT1Again, c->stream);
   }
-  c->counters[5] += 8 + (nb > 1024 ? 1 : 0) + (split ? 6 : 0) + (ta.foresee ? 3 : 0);
+  // analysis, masks, modelling, order and coding; the split with another part's; the second round
+  const uint64_t models = ta.nitems ? 1 + (split ? 1 : 0) + (ta.foresee ? 1 : 0) : 0;
+  c->counters[5] += 6 + (split ? 5 : 0) + (ta.foresee ? 2 : 0) + models;
   record(c, 3);
   // ---- PCRD ----
   PcrdArgs pa{};
@@ -1016,9 +1017,8 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   launch_pcrd(pa, c->num_sms, c->stream);
   record(c, 4);
   // ---- compaction ----
-  launch_compact(ta.blocks, pa.keep, nb, ta.out, dptr<uint8_t>(c->body), dptr<uint32_t>(c->offsets),
-                 dptr<uint32_t>(c->scratch), c->stream);
-  c->counters[5] += 3 + (nb > 1024 ? 1 : 0);  // 2 PCRD, scan + copy kernels
+  c->counters[5] += 2 + launch_compact(ta.blocks, pa.keep, nb, ta.out, dptr<uint8_t>(c->body),
+                                       dptr<uint32_t>(c->offsets), dptr<uint32_t>(c->scratch), c->stream);
   record(c, 5);
   // ---- read back the per-block results ----
   if (!reserve_host(c, c->hkeep, std::max<size_t>(nb, 1) * sizeof(BlockKeep)) ||

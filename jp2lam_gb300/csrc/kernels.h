@@ -125,9 +125,10 @@ void launch_mq_order(const T1Args& a, T1Part part, uint32_t* order, uint32_t* ke
 
 // Exclusive prefix sum of n uint32 values read with a stride of `stride`
 // words: out[i] = sum of in[0..i), out[n] = total. `scratch` holds
-// ceil(n/1024)+1 words.
-void launch_scan_u32(const uint32_t* in, uint32_t stride, uint32_t n, uint32_t* out,
-                     uint32_t* scratch, cudaStream_t st);
+// ceil(n/1024)+1 words. Returns its kernel launches, as launch_compact and
+// launch_t2 do.
+int launch_scan_u32(const uint32_t* in, uint32_t stride, uint32_t n, uint32_t* out,
+                    uint32_t* scratch, cudaStream_t st);
 
 struct PcrdArgs {
   const BlockDesc* blocks;
@@ -193,7 +194,7 @@ struct T2Args {
 // Packet headers, page layout (page_off[npages] = total bytes) and the
 // finished codestreams in `out`. scan_scratch: ceil(max(npages,
 // npackets)/1024)+1 words.
-void launch_t2(const T2Args& a, uint32_t* scan_scratch, int num_sms, cudaStream_t st);
+int launch_t2(const T2Args& a, uint32_t* scan_scratch, int num_sms, cudaStream_t st);
 
 // ------------------------------------------------------------- decoding --
 // One code-block of a codestream being decoded.
@@ -303,8 +304,8 @@ void launch_recon(ReconArgs r, const std::pair<int, int>* ladder, int levels, cu
 // Packs the retained payload bytes of every block, in work-list order, into
 // `dst`; offsets[b] receives the byte offset of block b and offsets[n] the
 // total. `scratch` holds ceil(n/1024)+1 uint32.
-void launch_compact(const BlockDesc* blocks, const BlockKeep* keep, uint32_t nblocks,
-                    const uint8_t* src, uint8_t* dst, uint32_t* offsets, uint32_t* scratch,
-                    cudaStream_t st);
+int launch_compact(const BlockDesc* blocks, const BlockKeep* keep, uint32_t nblocks,
+                   const uint8_t* src, uint8_t* dst, uint32_t* offsets, uint32_t* scratch,
+                   cudaStream_t st);
 
 }  // namespace jp2g

@@ -322,28 +322,30 @@ void launch_pcrd(const PcrdArgs& a, int num_sms, cudaStream_t st) {
   pcrd_select_kernel<<<g, t, 0, st>>>(a);
 }
 
-void launch_scan_u32(const uint32_t* in, uint32_t stride, uint32_t n, uint32_t* out,
-                     uint32_t* scratch, cudaStream_t st) {
+int launch_scan_u32(const uint32_t* in, uint32_t stride, uint32_t n, uint32_t* out,
+                    uint32_t* scratch, cudaStream_t st) {
   if (n == 0) {
     cudaMemsetAsync(out, 0, sizeof(uint32_t), st);
-    return;
+    return 0;
   }
   const uint32_t parts = (n + kScanT - 1) / kScanT;
   scan_partial_kernel<<<parts, kScanT, 0, st>>>(in, stride, n, out, scratch);
-  if (parts == 1) return;  // one launch for a small page
+  if (parts == 1) return 1;  // one launch for a small page
   scan_sums_kernel<<<1, 32, 0, st>>>(scratch, parts, out, n);
   scan_add_kernel<<<parts, kScanT, 0, st>>>(out, n, scratch);
+  return 3;
 }
 
-void launch_compact(const BlockDesc* blocks, const BlockKeep* keep, uint32_t nblocks,
-                    const uint8_t* src, uint8_t* dst, uint32_t* offsets, uint32_t* scratch,
-                    cudaStream_t st) {
+int launch_compact(const BlockDesc* blocks, const BlockKeep* keep, uint32_t nblocks,
+                   const uint8_t* src, uint8_t* dst, uint32_t* offsets, uint32_t* scratch,
+                   cudaStream_t st) {
   static_assert(sizeof(BlockKeep) == 12, "body_len is read as every third word");
-  launch_scan_u32(reinterpret_cast<const uint32_t*>(keep) + 1, 3, nblocks, offsets, scratch, st);
-  if (nblocks == 0) return;
+  const int scan = launch_scan_u32(reinterpret_cast<const uint32_t*>(keep) + 1, 3, nblocks, offsets, scratch, st);
+  if (nblocks == 0) return scan;
   const uint32_t threads = 256;
   const uint32_t grid = (uint32_t)(((uint64_t)nblocks * 32 + threads - 1) / threads);
   copy_bodies_kernel<<<grid, threads, 0, st>>>(blocks, keep, nblocks, src, dst, offsets);
+  return scan + 1;
 }
 
 }  // namespace jp2g

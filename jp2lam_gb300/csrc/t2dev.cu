@@ -320,14 +320,16 @@ __global__ void __launch_bounds__(128) t2_pages_kernel(T2Args a) {
 
 }  // namespace
 
-void launch_t2(const T2Args& a, uint32_t* scan_scratch, int num_sms, cudaStream_t st) {
-  if (a.npackets == 0) return;
+int launch_t2(const T2Args& a, uint32_t* scan_scratch, int num_sms, cudaStream_t st) {
+  if (a.npackets == 0) return 0;
   t2_header_kernel<<<a.npackets, kT2Threads, 0, st>>>(a);
   t2_layout_kernel<<<(a.npages + 127) / 128, 128, 0, st>>>(a);
-  launch_scan_u32(a.page_len, 1, a.npages, a.page_off, scan_scratch, st);
-  launch_scan_u32(a.nchunks, 1, a.npackets, a.chunk_base, scan_scratch, st);
+  int launches = 4;
+  launches += launch_scan_u32(a.page_len, 1, a.npages, a.page_off, scan_scratch, st);
+  launches += launch_scan_u32(a.nchunks, 1, a.npackets, a.chunk_base, scan_scratch, st);
   t2_copy_kernel<<<(unsigned)num_sms * 8, kT2Threads, 0, st>>>(a);
   t2_pages_kernel<<<(a.npages + 3) / 4, 128, 0, st>>>(a);
+  return launches;
 }
 
 }  // namespace jp2g
