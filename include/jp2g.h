@@ -266,7 +266,11 @@ void* jp2g_stream(jp2g_ctx* ctx);
  * [5] read-back of the codestreams into the callers' buffers, [6] host
  * time after it, [7] total, the tier-1 split [8] analysis and bit-plane
  * masks, [9] context modelling, [10] MQ coding, and [11] device Tier-2
- * (packet headers and assembly, between [4] and [5]). Returns the count. */
+ * (packet headers and assembly, between [4] and [5]). A wave of more than
+ * eight code-blocks per SM is coded in two parts, the first one's MQ coding
+ * beside the second one's modelling: [9] ends when both are modelled, [10]
+ * begins with the first one's coding, and [8] + [9] + [10] is more than [2].
+ * Returns the count. */
 int jp2g_set_timing(jp2g_ctx* ctx, int enabled);
 int jp2g_stage_times(jp2g_ctx* ctx, float* ms, int n);
 

@@ -57,7 +57,7 @@ struct HostBuf {
 };
 
 enum Stage { kH2D = 0, kDWT, kT1, kPCRD, kCompact, kD2H, kHost, kTotal, kNumStages };
-enum SubEvent { kEvAnalyzeEnd = kNumStages + 1, kEvModelEnd, kEvT2End, kNumEvents };
+enum SubEvent { kEvAnalyzeEnd = kNumStages + 1, kEvModelEnd, kEvMqBegin, kEvT2End, kNumEvents };
 
 // jp2g_set_result_alloc, jp2g_set_thread_result_alloc
 struct ResultAlloc {
@@ -234,9 +234,10 @@ T* dptr(DevBuf& b) {
   return reinterpret_cast<T*>(b.p);
 }
 
-void record(jp2g_ctx* c, int i) {
-  if (c->timing) cudaEventRecord(c->ev[i], c->stream);
+void record_on(jp2g_ctx* c, int i, cudaStream_t st) {
+  if (c->timing) cudaEventRecord(c->ev[i], st);
 }
+void record(jp2g_ctx* c, int i) { record_on(c, i, c->stream); }
 
 // Per-block payload capacity and pass-record capacity for a plan.
 uint32_t slot_cap(const PagePlan& p) { return (uint32_t)(p.cbw * p.cbh * 4 + 1024); }
@@ -976,12 +977,14 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
     if (!cuda_ok(c, cudaEventRecord(c->ev_mq[0], c->stream), "part modelled") ||
         !cuda_ok(c, cudaStreamWaitEvent(c->mq_stream, c->ev_mq[0], 0), "wait for a part"))
       return kEncodeFailed;
+    record_on(c, kEvMqBegin, c->mq_stream);
     launch_mq_order(ta, kT1Part0, order, key, scratch + kOrderScratch, c->mq_stream);
     launch_t1_mq(ta, c->num_sms, bpw, kT1Part0, c->mq_stream);
   }
   const T1Part rest = split ? kT1Part1 : kT1All;
   launch_t1_model(ta, c->num_sms, rest, c->stream);
   record(c, kEvModelEnd);
+  if (!split) record(c, kEvMqBegin);
   launch_mq_order(ta, rest, order, key, scratch, c->stream);
   launch_t1_mq(ta, c->num_sms, bpw, rest, c->stream);
   if (split && (!cuda_ok(c, cudaEventRecord(c->ev_mq[1], c->mq_stream), "part coded") ||
@@ -1133,6 +1136,14 @@ float stage_span(jp2g_ctx* c, int s) {
   return ms;
 }
 
+// The tier-1 split: analysis (+ masks, item list), modelling, MQ coding. A
+// split wave's first part is coded beside the modelling of the other.
+void tier1_split(jp2g_ctx* c, float ms[3]) {
+  cudaEventElapsedTime(&ms[0], c->ev[2], c->ev[kEvAnalyzeEnd]);
+  cudaEventElapsedTime(&ms[1], c->ev[kEvAnalyzeEnd], c->ev[kEvModelEnd]);
+  cudaEventElapsedTime(&ms[2], c->ev[kEvMqBegin], c->ev[3]);
+}
+
 // Adds the device stages of the wave just run (events 0..6) to stage_ms.
 void add_wave_stage_times(jp2g_ctx* c) {
   if (!c->timing) return;
@@ -1143,11 +1154,9 @@ void add_wave_stage_times(jp2g_ctx* c) {
   c->stage_ms[kNumStages + 3] += ms;
   cudaEventElapsedTime(&ms, c->ev[0], c->ev[6]);
   c->stage_ms[kTotal] += ms;
-  const int sub[3][2] = {{2, kEvAnalyzeEnd}, {kEvAnalyzeEnd, kEvModelEnd}, {kEvModelEnd, 3}};
-  for (int k = 0; k < 3; ++k) {
-    cudaEventElapsedTime(&ms, c->ev[sub[k][0]], c->ev[sub[k][1]]);
-    c->stage_ms[kNumStages + k] += ms;
-  }
+  float split[3] = {};
+  tier1_split(c, split);
+  for (int k = 0; k < 3; ++k) c->stage_ms[kNumStages + k] += split[k];
 }
 
 // Reads the stage events of the last wave into stage_ms.
@@ -1157,10 +1166,7 @@ void read_stage_times(jp2g_ctx* c) {
   for (int s = 0; s < kTotal; ++s) c->stage_ms[s] = stage_span(c, s);
   cudaEventElapsedTime(&c->stage_ms[kTotal], c->ev[0], c->ev[8]);
   cudaEventElapsedTime(&c->stage_ms[kNumStages + 3], c->ev[kCompact + 1], c->ev[kEvT2End]);
-  // tier-1 split: analysis (+item list), modelling, MQ coding
-  cudaEventElapsedTime(&c->stage_ms[kNumStages + 0], c->ev[2], c->ev[kEvAnalyzeEnd]);
-  cudaEventElapsedTime(&c->stage_ms[kNumStages + 1], c->ev[kEvAnalyzeEnd], c->ev[kEvModelEnd]);
-  cudaEventElapsedTime(&c->stage_ms[kNumStages + 2], c->ev[kEvModelEnd], c->ev[3]);
+  tier1_split(c, &c->stage_ms[kNumStages]);
 }
 
 // One page through the whole pipeline (jp2g_encode and the debug entry

@@ -57,3 +57,23 @@ def test_kernel_launches_of_a_large_wave(eng):
     names = _kernels(lambda: eng.encode_batch(pages))
     assert eng.counters()[0] > 48 * 152
     assert len(names) == eng.counters()[5], names
+
+
+@pytest.mark.parametrize("w,h,split", [(1000, 900, False), (3000, 3300, True)])
+def test_stage_times_of_modelling_and_coding(eng, w, h, split):
+    # a split wave's first part (here the noise) is coded while the second is
+    # modelled (the much fainter rest of the page)
+    rng = np.random.default_rng(w)
+    px = rng.integers(100, 156, (h, w), dtype=np.uint8)
+    px[:, : w // 4] = rng.integers(0, 256, (h, w // 4))
+    eng.set_timing(True)
+    try:
+        eng.encode(px, w, h, 1, 85, 0)
+        eng.encode(px, w, h, 1, 85, 0)
+        t = eng.stage_times()
+    finally:
+        eng.set_timing(False)
+    assert (eng.counters()[0] > 8 * 152) == split
+    beside = t["t1_analyze"] + t["t1_model"] + t["t1_mq"] - t["tier1"]
+    assert beside > 0.02 * t["tier1"] if split else abs(beside) < 0.01 * t["tier1"]
+    assert t["t1_mq"] < t["tier1"]
