@@ -279,7 +279,13 @@ int jp2g_stage_times(jp2g_ctx* ctx, float* ms, int n);
  * coded as far as rate control can choose its passes) before rate
  * control, [4] bytes retained, [5] kernel launches, [6] coefficient
  * bit-planes (sum over blocks of coefficients x magnitude bit-planes),
- * [7] MQ symbols coded. */
+ * [7] MQ symbols coded, [8] bit-planes modelled (of [6]'s, those of blocks
+ * with something to code), and of the second round that large waves take for
+ * blocks with more bit-planes to code than were modelled at first: [9] blocks
+ * that came to the end of those, [10] blocks of them that were coded on.
+ * A block's coding stops when another block's slope allows it, so [2], [3], [7],
+ * [8], [9] and [10] may differ a little from one encode of a page to the next;
+ * the codestream does not. */
 int jp2g_counters(jp2g_ctx* ctx, uint64_t* out, int n);
 
 /* Inspection entry points for parity tests. */

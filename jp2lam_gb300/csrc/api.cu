@@ -58,6 +58,7 @@ struct HostBuf {
 
 enum Stage { kH2D = 0, kDWT, kT1, kPCRD, kCompact, kD2H, kHost, kTotal, kNumStages };
 enum SubEvent { kEvAnalyzeEnd = kNumStages + 1, kEvModelEnd, kEvMqBegin, kEvT2End, kNumEvents };
+constexpr int kNumCounters = 11;  // jp2g_counters
 
 // jp2g_set_result_alloc, jp2g_set_thread_result_alloc
 struct ResultAlloc {
@@ -136,7 +137,7 @@ struct jp2g_ctx {
   cudaEvent_t ev_up[2] = {};
   uint8_t* wave_px = nullptr;  // the current wave's device pixels
   float stage_ms[kNumStages + 4] = {};
-  uint64_t counters[8] = {};
+  uint64_t counters[kNumCounters] = {};
   // default wave: 240,000 code-blocks (the autotuner's choice on sRGB and
   // uneven batches: fewer waves, fewer MQ tails); 160,000 under a budget
   int64_t opt[JP2G_NUM_OPTS] = {240000, 0, 0, 0, 0, 0, 0};
@@ -839,7 +840,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
       !reserve(c, c->nplanes, std::max<size_t>(nb, 1) * 4) ||
       !reserve(c, c->planebase, (size_t)(nb + 1) * 4) ||
       !reserve(c, c->body, std::max<size_t>(nb, 1) * std::max<size_t>(cap, pcap * (sizeof(double) + sizeof(uint16_t)))) ||
-      !reserve(c, c->stats, 64) || !reserve_host(c, c->hcount, 64))
+      !reserve(c, c->stats, 64) || !reserve_host(c, c->hcount, 128))
     return kEncodeFailed;
 
   record(c, 0);
@@ -1032,7 +1033,7 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
                                   cudaMemcpyDeviceToHost, c->stream), "D2H keep") ||
       !cuda_ok(c, cudaMemcpyAsync(c->hres.p, c->res.p, nb * sizeof(BlockOut),
                                   cudaMemcpyDeviceToHost, c->stream), "D2H results") ||
-      !cuda_ok(c, cudaMemcpyAsync(hcount + 2, c->stats.p, 8, cudaMemcpyDeviceToHost, c->stream),
+      !cuda_ok(c, cudaMemcpyAsync(hcount + 16, c->stats.p, 64, cudaMemcpyDeviceToHost, c->stream),
                "D2H statistics") ||
       !cuda_ok(c, cudaMemcpyAsync(hcount + 4, dptr<uint32_t>(c->offsets) + nb, 4, cudaMemcpyDeviceToHost,
                                   c->stream), "D2H retained bytes") ||
@@ -1067,7 +1068,11 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
     c->counters[6] += (uint64_t)hr[i].mbp * blocks[i].w * blocks[i].h;
   }
   c->counters[4] = total;
-  c->counters[7] = *reinterpret_cast<const uint64_t*>(hcount + 2);
+  c->counters[7] = *reinterpret_cast<const uint64_t*>(hcount + 16);
+  const uint32_t* count = hcount + 16 + 4;  // T1Count
+  c->counters[8] = (uint64_t)count[kCountItems] + count[kCountItems + 1] + count[kCountAgainItems];
+  c->counters[9] = count[kCountUnfinished];
+  c->counters[10] = count[kCountAgainBlocks];
   if (dbg && dbg->res) dbg->res->assign(hr, hr + nb);
   if (dbg && dbg->keep) dbg->keep->assign(hk, hk + nb);
   return kOk;
@@ -1119,11 +1124,11 @@ int run_wave_within_budget(jp2g_ctx* c, PageJob* const* jobs, size_t n, const Pr
   }
   c->budget_wave_blocks = std::max<uint64_t>(1, blocks / 2);
   const size_t h = n / 2;
-  uint64_t counters[8];
+  uint64_t counters[kNumCounters];
   if ((rc = run_wave_within_budget(c, jobs, h, pre))) return rc;
   std::memcpy(counters, c->counters, sizeof counters);
   if ((rc = run_wave_within_budget(c, jobs + h, n - h, pre))) return rc;
-  for (int k = 0; k < 8; ++k) c->counters[k] += counters[k];
+  for (int k = 0; k < kNumCounters; ++k) c->counters[k] += counters[k];
   return kOk;
 }
 
@@ -1784,7 +1789,7 @@ static int encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8
     out_lens[i] = 0;
   }
   int rc = JP2G_OK;
-  uint64_t counters[8] = {};
+  uint64_t counters[kNumCounters] = {};
   std::memset(c->stage_ms, 0, sizeof c->stage_ms);
   const auto t0 = std::chrono::steady_clock::now();
   // Host pixels of wave k+1 are staged (on a helper thread, into the other
@@ -1860,7 +1865,7 @@ static int encode_batch(jp2g_ctx* c, const jp2g_request* reqs, uint32_t n, uint8
     if (stager.joinable()) stager.join();
     staged = next_staged;
     uploaded = next_uploaded;
-    for (int k = 0; k < 8; ++k) counters[k] += c->counters[k];
+    for (int k = 0; k < kNumCounters; ++k) counters[k] += c->counters[k];
     if (rc != JP2G_OK) break;
     add_wave_stage_times(c);
   }
@@ -2331,7 +2336,7 @@ int jp2g_stage_times(jp2g_ctx* c, float* ms, int n) {
 
 int jp2g_counters(jp2g_ctx* c, uint64_t* out, int n) {
   if (!c || !out) return 0;
-  int k = std::min(n, 8);
+  int k = std::min(n, kNumCounters);
   for (int i = 0; i < k; ++i) out[i] = c->counters[i];
   return k;
 }

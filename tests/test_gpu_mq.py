@@ -2,6 +2,8 @@
 end at every symbol count, carry through bytes of 0xFF, shift by many bits at
 once or hardly at all, in every packing of blocks to a warp's lanes, against
 the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -145,3 +147,66 @@ def test_hulls_by_warps_and_by_lanes(eng, orc, kind, w, h, c, q):
     data = eng.encode(px, w, h, c, q, 0)
     assert (eng.counters()[0] > 16 * 152) == (w > 64)
     assert data == orc.encode(px, w, h, c, q, 0)
+
+
+def _round_counters(eng):
+    """Bit-planes modelled, blocks left unfinished by the first round, blocks
+    coded on in the second."""
+    c = (ctypes.c_uint64 * 11)()
+    assert eng.lib.jp2g_counters(eng.handle, c, 11) == 11
+    return list(c[8:])
+
+
+def _misleading(w, h, seed):
+    """Content whose bit counts make coding look dearer than it is: every block
+    regular (signs and bits that the contexts foresee), so that many more
+    bit-planes are worth their bytes than a forecast from counts expects."""
+    y, x = np.mgrid[0:h, 0:w]
+    period = 2 + seed % 3
+    px = 128 + (((x // period + y // period) & 1) * 2 - 1) * (20 + 7 * (seed % 5)) + ((x ^ y) & 3)
+    return px.astype(np.uint8)
+
+
+@pytest.mark.parametrize("q", [20, 60, 90])
+def test_second_round_is_taken(eng, orc, q):
+    # 32x32 and 64x64 blocks; some blocks of the wave are left unfinished by the
+    # first round, and some of these are coded on by the second
+    pages = []
+    for i in range(40):
+        w, h = (1024 + 3 * i, 900 + i) if q < 30 else (2048 + 3 * i, 1500 + i)
+        px = _misleading(w, h, i) if i % 2 else _stop_content(("outlier", "texture")[i // 2 % 2], w, h, 1)
+        pages.append({"px": px, "w": w, "h": h, "ncomp": 1, "quality": q, "fmt": 0})
+    outs = eng.encode_batch(pages)
+    assert eng.counters()[0] > 48 * 152
+    modelled, unfinished, again = _round_counters(eng)
+    assert modelled > 0
+    assert unfinished >= again > 0
+    for i in range(0, 40, 3):
+        p = pages[i]
+        assert outs[i] == orc.encode(p["px"], p["w"], p["h"], 1, q, 0, threads=8), i
+
+
+@pytest.mark.parametrize("bpw", [1, 3, 31, 32])
+@pytest.mark.parametrize("large", [False, True])
+def test_packings_of_split_and_large_waves(eng, orc, bpw, large):
+    # a packing of the caller's choice where the wave is coded in two parts, and
+    # where there is a second round
+    rng = np.random.default_rng(bpw)
+    pages = []
+    for i in range(12 if large else 4):
+        w, h = (1800 + 5 * i, 1500 + i) if large else (1600, 1300 + i)
+        px = _misleading(w, h, i)
+        px[: h // 3] = rng.integers(0, 256, (h // 3, w))
+        pages.append({"px": px, "w": w, "h": h, "ncomp": 1, "quality": 70, "fmt": 0})
+    if large:
+        pages = pages + pages[:1] * 2
+    eng.set_option(_native.OPT_MQ_BLOCKS_PER_WARP, bpw)
+    try:
+        outs = eng.encode_batch(pages)
+    finally:
+        eng.set_option(_native.OPT_MQ_BLOCKS_PER_WARP, 0)
+    blocks = eng.counters()[0]
+    assert blocks > 48 * 152 if large else 8 * 152 < blocks <= 48 * 152
+    assert (_round_counters(eng)[2] > 0) == large
+    for p, out in list(zip(pages, outs))[::3]:
+        assert out == orc.encode(p["px"], p["w"], p["h"], 1, 70, 0, threads=8)
