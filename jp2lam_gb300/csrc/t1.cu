@@ -1110,7 +1110,9 @@ __global__ void __launch_bounds__(kMqWarps * 32, 3) t1_mq_kernel(T1Args a, T1Par
     const uint32_t slot = (blockIdx.x * kMqWarps + wid) * (uint32_t)bpw + (uint32_t)lane;
     mq_code_block<0>(a, lane < bpw && slot < n ? a.mq_order[first + slot] : kNoBlock, sm);
   } else {  // the blocks that t1_recheck_kernel listed, over a fixed grid
-    const uint32_t per_cta = kMqWarps * (uint32_t)bpw, count = a.counts[kCountAgainBlocks];
+    const uint32_t count = a.counts[kCountAgainBlocks];
+    if (bpw == 0) bpw = mq_blocks_auto(count, warps);
+    const uint32_t per_cta = kMqWarps * (uint32_t)bpw;
     for (uint32_t first = blockIdx.x * per_cta; first < count; first += gridDim.x * per_cta) {
       const uint32_t slot = first + (uint32_t)(wid * bpw + lane);
       mq_code_block<1>(a, lane < bpw && slot < count ? a.again[slot] : kNoBlock, sm);
@@ -1195,12 +1197,14 @@ void launch_t1_split(const T1Args& a, cudaStream_t st) {
   t1_split_kernel<<<(a.nblocks + 255) / 256, 256, 0, st>>>(a);
 }
 
-// CTAs loop over the items. Few are left for the second round; a split wave's
-// are short, as the coding of an earlier part waits for their places.
+// CTAs loop over the items. A split wave's are short, as the coding of an
+// earlier part waits for their places. The second round's items are few on most
+// pages (39 blocks' of 24 sRGB ones) and many where the content is regular, so
+// it has as many CTAs as the SMs hold at once.
 void launch_t1_model(const T1Args& a, int num_sms, T1Part part, cudaStream_t st) {
   if (a.nitems == 0) return;
   uint32_t need = (a.nitems + kModelWarps - 1) / kModelWarps;
-  uint32_t cap = (uint32_t)num_sms * (part == kT1Again ? 2 : part == kT1All ? 6 * 4 : 6 * 24);
+  uint32_t cap = (uint32_t)num_sms * (part == kT1Again ? 5 : part == kT1All ? 6 * 4 : 6 * 24);
   t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a, part);
 }
 
@@ -1213,8 +1217,8 @@ void launch_t1_mq(const T1Args& a, int num_sms, int bpw, T1Part part, cudaStream
   const uint32_t sms = (uint32_t)num_sms;
   if (bpw < 1 || bpw > 32) bpw = 0;
   const uint32_t most = (uint32_t)mq_blocks_per_warp(a, num_sms, bpw);
-  if (part == kT1Again) {  // few
-    t1_mq_kernel<1><<<sms, kMqWarps * 32, 0, st>>>(a, part, (int)std::min(most, 4u), 0u);
+  if (part == kT1Again) {  // four CTAs fit an SM; the first ones take a short list
+    t1_mq_kernel<1><<<sms * 4, kMqWarps * 32, 0, st>>>(a, part, bpw, sms * 4u);
     return;
   }
   // a part of the wave's blocks takes a CTA on each SM, or as many blocks per warp as the whole wave

@@ -210,3 +210,13 @@ def test_packings_of_split_and_large_waves(eng, orc, bpw, large):
     assert (_round_counters(eng)[2] > 0) == large
     for p, out in list(zip(pages, outs))[::3]:
         assert out == orc.encode(p["px"], p["w"], p["h"], 1, 70, 0, threads=8)
+
+
+def test_second_round_of_most_blocks(eng, orc):
+    # more blocks in the second round than its warps have lanes: each CTA codes several lists
+    w, h = 1700, 2200
+    y, x = np.mgrid[0:h, 0:w]
+    px = ((((x // 2 + y // 2) & 1) * 60 + 100) + ((x ^ y) & 3)).astype(np.uint8)
+    outs = eng.encode_batch([{"px": px, "w": w, "h": h, "ncomp": 1, "quality": 20, "fmt": 0}] * 32)
+    assert _round_counters(eng)[2] > 152 * 4 * 4 * 32
+    assert set(outs) == {orc.encode(px, w, h, 1, 20, 0, threads=8)}
