@@ -87,7 +87,8 @@ class _PyResults(ctypes.Structure):
 _PY_API = (ctypes.c_void_p * 6)(*[ctypes.cast(getattr(ctypes.pythonapi, f), ctypes.c_void_p).value for f in (
     "PyGILState_Ensure", "PyGILState_Release", "PyBytes_FromStringAndSize", "PyBytes_AsString", "PyErr_Clear",
     "Py_DecRef")])
-# a prototype of its own: ctypes.pythonapi's functions are shared by the whole process
+# prototypes of their own: ctypes.pythonapi's functions are shared by the whole process
+_new_ref = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p)(("Py_NewRef", ctypes.pythonapi))
 _decref = ctypes.PYFUNCTYPE(None, ctypes.c_void_p)(("Py_DecRef", ctypes.pythonapi))
 
 
@@ -101,16 +102,23 @@ class _Results:
         self._lib = lib
         self._objects = (ctypes.c_void_p * max(n, 1))()
         self._results = _PyResults(_PY_API, self._objects, n)
+        self._alloc = ctypes.cast(lib.jp2g_py_result_alloc, ctypes.c_void_p).value
+        self._user = ctypes.addressof(self._results)
 
     def __enter__(self):
-        self._lib.jp2g_set_thread_result_alloc(self._lib.jp2g_py_result_alloc, ctypes.byref(self._results))
+        self._lib.jp2g_set_thread_result_alloc(self._alloc, self._user)
         return self
 
     def __exit__(self, *_):
         self._lib.jp2g_set_thread_result_alloc(None, None)
 
-    def __getitem__(self, i: int) -> bytes:
-        return ctypes.cast(self._objects[i], ctypes.py_object).value
+    def take(self, i: int) -> bytes:
+        """The codestream of index i, which leaves the object."""
+        p = self._objects[i]
+        data = _new_ref(p)
+        self._objects[i] = None
+        _decref(p)
+        return data
 
     def __del__(self):
         for p in self._objects:
@@ -213,6 +221,7 @@ class Engine:
             _raise(rc, self.lib.jp2g_last_error(None).decode())
         self.handle = h
         self._lock = threading.Lock()
+        self._result = _Results(self.lib, 1)  # of the single-page calls, under _lock
         self._inflight = {}  # ticket -> pixel buffer kept alive until polled
         self._inflight_lock = threading.Lock()
 
@@ -239,11 +248,11 @@ class Engine:
             raise InvalidInput("pixel buffer length does not match the image dimensions")
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock, _Results(self.lib, 1) as results:
+        with self._lock, self._result as result:
             rc = self.lib.jp2g_encode(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                       int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n))
             self._check(rc)
-        return results[0]
+            return result.take(0)
 
     def encode_with_psnr(self, px, w: int, h: int, ncomp: int, quality: int, fmt: int,
                          interleaved: bool = True):
@@ -256,12 +265,12 @@ class Engine:
         out = _u8p()
         n = ctypes.c_size_t()
         psnr, ssim = ctypes.c_double(), ctypes.c_double()
-        with self._lock, _Results(self.lib, 1) as results:
+        with self._lock, self._result as result:
             rc = self.lib.jp2g_encode_with_psnr(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                                 int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n),
                                                 ctypes.byref(psnr), ctypes.byref(ssim))
             self._check(rc)
-        return results[0], psnr.value, ssim.value
+            return result.take(0), psnr.value, ssim.value
 
     @staticmethod
     def _decode_flags(rct_chroma_extra_bitplane, accept_empty_segments):
@@ -324,11 +333,11 @@ class Engine:
     def encode_device(self, dev_ptr: int, w: int, h: int, ncomp: int, quality: int, fmt: int) -> bytes:
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock, _Results(self.lib, 1) as results:
+        with self._lock, self._result as result:
             rc = self.lib.jp2g_encode_device(self.handle, ctypes.c_void_p(dev_ptr), w, h, ncomp, quality,
                                              fmt, ctypes.byref(out), ctypes.byref(n))
             self._check(rc)
-        return results[0]
+            return result.take(0)
 
     @staticmethod
     def _request(page, keep):
@@ -366,7 +375,7 @@ class Engine:
         result = []
         for i in range(n):
             if status[i] == 0:
-                result.append(files[i])
+                result.append(files.take(i))
             else:
                 result.append(_BY_CODE.get(status[i], Jp2LamError)(msg or f"page {i} failed"))
         return result

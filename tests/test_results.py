@@ -26,23 +26,28 @@ def test_result_alloc_without_memory_returns_null():
     assert alloc(2, 10) is None  # not an index of the call
     at = alloc(1, 5)
     ctypes.memmove(at, b"hello", 5)
-    assert results[1] == b"hello"
-    assert alloc(1, 0) and results[1] == b""
+    assert results.take(1) == b"hello"
+    assert alloc(1, 0) and results.take(1) == b""
 
 
 def test_result_objects_are_released_once():
     lib = _native.load_library()
     results = _native._Results(lib, 1)
-    alloc = lambda n: lib.jp2g_py_result_alloc(ctypes.byref(results._results), 0, n)  # noqa: E731
-    alloc(1000)
-    first = results[0]
-    mine = sys.getrefcount(first) - 1  # without the slot's
-    alloc(2000)
-    assert sys.getrefcount(first) == mine
-    second = results[0]
-    with_slot = sys.getrefcount(second)
+
+    def new(n):  # an object in the slot, and this reference to it
+        lib.jp2g_py_result_alloc(ctypes.byref(results._results), 0, n)
+        return _native._new_ref(results._objects[0])
+
+    first = new(1000)
+    refs = sys.getrefcount(first)
+    second = new(2000)  # replaces it
+    assert sys.getrefcount(first) == refs - 1
+    assert sys.getrefcount(second) == refs
+    taken = results.take(0)
+    assert taken is second and sys.getrefcount(second) == refs  # the slot's is now `taken`'s
+    third = new(3000)
     del results
-    assert sys.getrefcount(second) == with_slot - 1
+    assert sys.getrefcount(second) == refs and sys.getrefcount(third) == refs - 1
 
 
 @pytest.mark.gpu
