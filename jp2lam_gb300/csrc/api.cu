@@ -1529,9 +1529,14 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   // device job tables: blocks, then per-level inverse-DWT jobs, then pixel jobs
   std::vector<DecBlock> blk;
   blk.reserve(nblk);
-  uint64_t mask_words = 0;
+  uint64_t mask_words = 0, coded = 0;
+  uint32_t longest = 0;
   for (size_t i : ids)
     for (DecBlock b : pg[i].L.blocks) {
+      if (b.npasses) {
+        coded += b.data_len;
+        longest = std::max(longest, b.data_len);
+      }
       b.plane_off += pg[i].plane_base;
       b.data_off += (uint32_t)pg[i].data_base;
       b.mask_off = mask_words;
@@ -1608,8 +1613,14 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
       !cuda_ok(c, cudaMemcpyAsync(dpix, pix.data(), pix.size() * sizeof(PixJob), cudaMemcpyHostToDevice, c->stream),
                "H2D pages"))
     return JP2G_DECODE_FAILED;
+  // The longest segment's chain sets the time up to six times its bytes per SM;
+  // above that all segments' instructions do. Latency's form against the other's,
+  // ms: 2550x3300 gray q85, 1 file (1 x its bytes per SM) 5.07 and 5.74, 4 (5 x)
+  // 7.95 and 8.27, 6 (7 x) 10.0 and 9.88, 8 (10 x) 11.4 and 9.94; 1700x2200
+  // lossless, 4 (10 x) 10.6 and 8.56; 12 sRGB q75 (13 x) 20.4 and 17.2.
+  const bool many = coded > 6ull * (uint64_t)c->num_sms * longest;
   launch_t1_decode(dblk, (uint32_t)blk.size(), dptr<uint8_t>(c->t2out), reinterpret_cast<unsigned long long*>(tmp),
-                   planes, reinterpret_cast<uint32_t*>(dpx), c->stream);
+                   planes, reinterpret_cast<uint32_t*>(dpx), many, c->stream);
   for (int l = 1; l <= maxl; ++l) launch_idwt_level(djobs + first[l], first[l + 1] - first[l], tiles[l], c->stream);
   launch_dec_pixels(dpix, (uint32_t)pix.size(), pix_blocks, c->stream);
   if (!cuda_ok(c, cudaGetLastError(), "decode kernels")) return JP2G_DECODE_FAILED;

@@ -259,9 +259,10 @@ JP2G_HD uint32_t dec_planes(uint32_t npasses) { return npasses ? (npasses + 4) /
 // 64-bit words of a block's masks, one per column and bit-plane and one for the signs.
 JP2G_HD uint32_t dec_mask_words(uint32_t w, uint32_t npasses) { return npasses ? w * (dec_planes(npasses) + 1) : 0; }
 // Tier-1 decoding of every code-block into coefficients (t1dec.cu). masks: the
-// blocks' masks; scratch: nblocks + 2048 words.
+// blocks' masks; scratch: nblocks + 2048 words. many: there are chains enough
+// for their instructions, not their latency, to set the time.
 void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, unsigned long long* masks,
-                      int32_t* planes, uint32_t* scratch, cudaStream_t st);
+                      int32_t* planes, uint32_t* scratch, bool many, cudaStream_t st);
 // One inverse-DWT level for njobs jobs (recon.cu).
 void launch_idwt_level(const IdwtJob* jobs, uint32_t njobs, uint32_t total_tiles, cudaStream_t st);
 void launch_dec_pixels(const PixJob* jobs, uint32_t njobs, uint32_t nblocks, cudaStream_t st);

@@ -109,6 +109,7 @@ __device__ __forceinline__ uint32_t six_rows(unsigned long long v, int k) {
 }
 __device__ __forceinline__ uint32_t four_rows(unsigned long long v, int k) { return (uint32_t)(v >> (4 * k)) & 0xfu; }
 
+template <bool kMany>
 struct BlockDecoder {
   const DecShared& sh;
   const uint8_t* zc;
@@ -163,8 +164,41 @@ struct BlockDecoder {
   // masks (a predicate takes longer to reach its users than a sign bit), and
   // the bytes that a shift has run out of are read at the next symbol, while
   // its context is on its way.
+  // In batches, where other warps fill a chain's waits, the shortest code
+  // decides instead (kMany): a decision without renormalisation ends early, and
+  // the rest is predicated. A lone chain takes 13 % longer that way; 12
+  // 1275x1650 files of 2x2 checks at quality 20, whose samples nearly all become
+  // significant in one pass, 4.56 ms (6.6 in the other form, 4.78 with two
+  // blocks to a warp, a lane each).
   __device__ __forceinline__ bool decode(uint32_t cx) {
     const uint32_t e = __shfl_sync(kAll, word, (int)cx);
+    if (kMany) {
+      const uint32_t qe = e & 0x7fff8000u, d = a - qe, t = c - qe;
+      if ((int)((d << 1) & ~t) < 0) {  // an MPS, A still 0x8000 or more
+        a = d;
+        c = t;
+        return (e & 1u) != 0;
+      }
+      const bool low = (int)t < 0, lps = low != (d < qe);
+      const uint32_t v = low ? qe : d;
+      if (!low) c = t;
+      if (lane == cx) {
+        word = lps ? lps_next : mps_next;
+        const uint2 n = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(sh.next) + (word & 0x3f8u));
+        mps_next = n.x;
+        lps_next = n.y;
+      }
+      int k = __clz((int)v) - 1;
+      a = v << k;
+      while (k > ct) {
+        c = (c << ct) & 0x7fffffffu;
+        k -= ct;
+        bytein();
+      }
+      c = (c << k) & 0x7fffffffu;
+      ct -= k;
+      return ((e & 1u) != 0) != lps;
+    }
     if (ct < 0) {
       c = shift_from;
       ct += shift;
@@ -367,6 +401,7 @@ struct BlockDecoder {
 // Seven CTAs fit an SM with or without the bound; with it the compiler keeps
 // everything in 72 registers (without, it spills 8 bytes on the chain): a gray
 // 2550x3300 file 5.36 -> 5.08 ms, a 512x512 lossless one 4.56 -> 4.34.
+template <bool kMany>
 __global__ void __launch_bounds__(kDecWarps * 32, 7) t1_decode_kernel(const DecBlock* blocks, const uint32_t* order,
                                                                       uint32_t nblocks, const uint8_t* data,
                                                                       unsigned long long* masks) {
@@ -378,7 +413,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, 7) t1_decode_kernel(const DecB
   if (slot >= nblocks) return;
   const DecBlock d = blocks[order[slot]];
   if (d.npasses == 0) return;
-  BlockDecoder dec{sh, sh.zc[d.orient & 3], lists[threadIdx.x >> 5], lane, d.w, d.h};
+  BlockDecoder<kMany> dec{sh, sh.zc[d.orient & 3], lists[threadIdx.x >> 5], lane, d.w, d.h};
   dec.start(data + d.data_off, d.data_len);
   unsigned long long* out = masks + d.mask_off;
   // cleanup of the top bit-plane, then significance, refinement and cleanup
@@ -470,7 +505,7 @@ bool upload_decode_tables(const uint8_t* zc, const uint8_t* sc, const uint8_t* s
 }
 
 void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* data, unsigned long long* masks,
-                      int32_t* planes, uint32_t* scratch, cudaStream_t st) {
+                      int32_t* planes, uint32_t* scratch, bool many, cudaStream_t st) {
   if (nblocks == 0) return;
   uint32_t* hist = scratch;
   uint32_t* cursor = scratch + kDecBuckets;
@@ -480,7 +515,9 @@ void launch_t1_decode(const DecBlock* blocks, uint32_t nblocks, const uint8_t* d
   dec_hist_kernel<<<g, 256, 0, st>>>(blocks, nblocks, hist);
   launch_scan_u32(hist, 1, kDecBuckets - 1, cursor, order, st);  // `order` is filled after the scan
   dec_scatter_kernel<<<g, 256, 0, st>>>(blocks, nblocks, cursor, order);
-  t1_decode_kernel<<<(nblocks + kDecWarps - 1) / kDecWarps, kDecWarps * 32, 0, st>>>(blocks, order, nblocks, data, masks);
+  const uint32_t ctas = (nblocks + kDecWarps - 1) / kDecWarps;
+  if (many) t1_decode_kernel<true><<<ctas, kDecWarps * 32, 0, st>>>(blocks, order, nblocks, data, masks);
+  else t1_decode_kernel<false><<<ctas, kDecWarps * 32, 0, st>>>(blocks, order, nblocks, data, masks);
   t1_coefficients_kernel<<<(nblocks + 3) / 4, 128, 0, st>>>(blocks, nblocks, masks, planes);
 }
 

@@ -234,3 +234,26 @@ def test_inverse_transform_at_the_edges_of_tiles(eng, orc, w, h, q):
     assert np.array_equal(eng.decode(data, **flags)[0], want)
     pair = eng.decode_batch([data, data], **flags)
     assert all(np.array_equal(np.asarray(p[0]), want) for p in pair)
+
+
+@pytest.mark.parametrize("q", [100, 80, 20])
+def test_batch_of_many_chains(eng, orc, q):
+    # so many segments that their instructions, not the longest one's latency, set
+    # the time: the decoder's other form, at the edges of stripes and halves, on
+    # regular and on noisy content
+    files, lens = [], []
+    for i, (w, h) in enumerate([(31, 4), (32, 5), (33, 3), (63, 64), (65, 66), (96, 1), (2, 130), (161, 97), (64, 64)]):
+        rng = np.random.default_rng(q + i)
+        y, x = np.mgrid[0:h, 0:w]
+        regular = ((((x // 2 + y // 2) & 1) * 60 + 100) + ((x ^ y) & 3)).astype(np.uint8)
+        for px in (regular, np.full((h, w), 200, np.uint8), rng.integers(0, 256, (h, w), dtype=np.uint8)):
+            files.append(orc.encode(px, w, h, 1, q, i % 2))
+            lens.append(orc.block_summary(px, w, h, 1, q)[:, 8])
+    lens = np.concatenate(lens)
+    copies = 1 + int(7 * 152 * lens.max() // lens.sum())
+    assert copies * lens.sum() > 6 * 152 * lens.max()
+    got = eng.decode_batch(files * copies, accept_empty_segments=True)
+    for k, f in enumerate(files):
+        want = orc.decode(f, accept_empty_segments=True)[3]
+        for g in got[k::len(files)]:
+            assert np.array_equal(np.asarray(g[0]), want), k
