@@ -916,8 +916,9 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   c->counters[5] += launch_scan_u32(ta.nplanes, 1, nb, ta.plane_base, dptr<uint32_t>(c->scratch), c->stream);
   // The number of (block, bit-plane) items sizes the symbol buffer. Up to two
   // blocks per SM, and without a memory budget, the most there can be serves as
-  // well (some 40 MB), and the device need not wait for the host to read the
-  // number: a 256x256 page takes 2 % less, a 517x389 sRGB one 2.5 %.
+  // well (20 bit-planes a block at least: up to 69 MB on 152 SMs), and the device
+  // need not wait for the host to read the number: a 256x256 page takes 2 % less,
+  // a 517x389 sRGB one 2.5 %.
   if (nb <= (uint32_t)c->num_sms * 2u && c->budget == 0) {
     ta.nitems = nb * ((pcap + 2) / 3);
   } else {
@@ -934,16 +935,16 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   // small wave these are the chains that the call waits for (three quarters of
   // the longest and more); a large one's coding takes long after them too, and
   // more of it goes first. With eight blocks per SM or fewer, modelling is too
-  // short to gain anything (48 pages of 256x256: 2.08 ms whole, 2.11 split). Modelling and coding, ms, with 3/4, 1/2 and 5/12 in
-  // part 0 and without the split: 2550x3300 sRGB page 1.92, 2.01, 2.07 and 2.30;
-  // 5100x6600 sRGB lossless 3.45, 3.24, 3.40 and 3.81; 24 sRGB pages -, 5.93,
-  // 5.53 and 7.1.
+  // short to gain anything (48 pages of 256x256: 2.08 ms whole, 2.11 split).
+  // Modelling and coding, ms, with 3/4, 1/2 and 5/12 in part 0 and without the
+  // split: 2550x3300 sRGB page 1.92, 2.01, 2.07 and 2.30; 5100x6600 sRGB
+  // lossless 3.45, 3.24, 3.40 and 3.81; 24 sRGB pages -, 5.93, 5.53 and 7.1.
   const bool split = nb > (uint32_t)c->num_sms * 8u;
   if (!reserve(c, c->items, std::max<size_t>(ta.nitems, 1) * 4 * (split ? 2 : 1)) ||
       !reserve(c, c->itemrec, std::max<size_t>(ta.nitems, 1) * sizeof(ItemRec)) ||
       !reserve(c, c->planes, std::max<size_t>(ta.nitems, 1) * 1024) ||
       !reserve(c, c->signs, std::max<size_t>(nb, 1) * 512) ||
-      !reserve(c, c->sym, std::max<size_t>(ta.nitems, 1) * ta.sym_slot + 64))  // the MQ reader runs 48 B ahead
+      !reserve(c, c->sym, std::max<size_t>(ta.nitems, 1) * ta.sym_slot + 64))  // the MQ reader runs 16 B ahead
     return kEncodeFailed;
   ta.items = dptr<uint32_t>(c->items);
   ta.item_rec = dptr<ItemRec>(c->itemrec);
@@ -966,8 +967,10 @@ int run_wave(jp2g_ctx* c, PageJob* const* jobs, size_t njobs, WaveDebug* dbg,
   uint32_t* const scratch = dptr<uint32_t>(c->mqscratch);
   uint32_t* const key = scratch + (split ? 2 : 1) * kOrderScratch;
   ta.mq_order = order;
-  ta.unfinished = split ? key + nb : key;  // not split: the order has been made
-  if (split) ta.weight = key + 2 * (size_t)nb;
+  if (split) {  // (only split waves are large enough for a second round)
+    ta.unfinished = key + nb;
+    ta.weight = key + 2 * (size_t)nb;
+  }
   ta.share = large ? 5 : 9;
   const int bpw = (int)c->opt[JP2G_OPT_MQ_BLOCKS_PER_WARP];
   launch_t1_planes(ta, c->stream);
@@ -1481,8 +1484,8 @@ int jp2g_encode_with_psnr(jp2g_ctx* c, const uint8_t* px, uint32_t w, uint32_t h
 // decode_jp2 (src/decode/mod.rs:56-61) on the device, for many files at
 // once: the host parses each file's boxes, headers and packet headers
 // (decode.cpp, on host threads); a round of files then shares one Tier-1
-// decoding launch over all their code-blocks, one inverse-DWT launch pair
-// per level over all their components, and one launch for the samples
+// decoding launch over all their code-blocks, one inverse-DWT launch per
+// level over all their components, and one launch for the samples
 // (t1dec.cu, recon.cu). Rounds are sized by device memory (the context's
 // budget, else 24 GiB); a round whose pools cannot grow is split.
 namespace {

@@ -115,8 +115,6 @@ void launch_t1_model(const T1Args& a, int num_sms, T1Part part, cudaStream_t st)
 void launch_t1_mq(const T1Args& a, int num_sms, int bpw, T1Part part, cudaStream_t st);
 // Between the rounds: which unfinished blocks are coded on.
 void launch_t1_recheck(const T1Args& a, int num_sms, cudaStream_t st);
-// Code-blocks per warp that launch_t1_mq uses for `bpw` (0 = automatic).
-int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw);
 // Orders the blocks of a part (or all) by their MQ symbol count, largest
 // first (counting sort on 1024 buckets), into order[], one part behind the
 // other. key: nblocks words; scratch: kOrderScratch words.

@@ -31,8 +31,6 @@
 
 #include <algorithm>
 
-#include <cstring>
-
 #include "jp2g_internal.h"
 #include "kernels.h"
 #include "t1_logic.h"
@@ -48,18 +46,14 @@ constexpr uint32_t kPadSymbol = kCtxNone;  // pads symbol streams to whole chunk
 // A symbol is a byte: context | decision << 7.
 constexpr uint32_t kOne = 0x80u;
 constexpr uint32_t kMqCtx = 20;
-constexpr int kModelWarps = 4;  // 7 KB of shared memory each: 6 CTAs per SM
+constexpr int kModelWarps = 4;  // 7 KB of shared memory each; registers allow 5 CTAs per SM
 constexpr int kMqWarps = 4;
 
-struct Tables {
-  uint8_t zc[4 * 512];
-  uint8_t sc[256];
-  uint8_t spb[256];
-  uint32_t mq[94];  // qe | nmps << 16 | nlps << 24
-};
-
-// Built on the host from the standard's rules, copied in by upload_t1_tables.
-__constant__ Tables c_tables;
+// The MQ states, qe | nmps << 16 | nlps << 24: built on the host from the
+// standard's rules, copied in by upload_t1_tables. (The context rules are logic
+// operations, t1_logic.h.)
+constexpr uint32_t kStates = 94;
+__constant__ uint32_t c_mq[kStates];
 
 // ---------------------------------------------------------------- analyze --
 // A warp per block, 16 bytes a lane, eight loads in flight. Bound by memory in
@@ -683,7 +677,6 @@ __global__ void __launch_bounds__(kModelWarps * 32, 5) t1_model_kernel(T1Args a,
 // MPS; y = shared address of the state's successors in the table | MPS << 3. The
 // table holds per state (state, MPS pair) its successors' entries: after an MPS
 // renormalisation, then after an LPS.
-constexpr uint32_t kStates = 94;
 struct __align__(16) MqTable {
   uint2 next[kStates][2];
 };
@@ -692,7 +685,7 @@ struct __align__(16) MqTable {
 constexpr uint32_t kNoState = kStates;
 __device__ __forceinline__ uint2 mq_entry(uint32_t state, uint32_t table) {
   if (state == kNoState) return make_uint2(0u, table);
-  const uint32_t qe = c_tables.mq[state] & 0xffffu, mps = state & 1u;
+  const uint32_t qe = c_mq[state] & 0xffffu, mps = state & 1u;
   return make_uint2(__float_as_uint((float)qe * (1.0f / 32768.0f)) | mps << 31, (table + state * 16u) | mps << 3);
 }
 __device__ __forceinline__ uint32_t mq_state(uint2 e, uint32_t table) { return (e.y - table) >> 4; }
@@ -702,7 +695,7 @@ __device__ __forceinline__ uint32_t mq_table_at(const MqTable& t) {
 __device__ __forceinline__ void load_mq_table(MqTable& t) {
   const uint32_t at = mq_table_at(t);
   for (uint32_t i = threadIdx.x; i < kStates; i += blockDim.x) {
-    const uint32_t v = c_tables.mq[i];  // qe | nmps << 16 | nlps << 24
+    const uint32_t v = c_mq[i];
     t.next[i][0] = mq_entry((v >> 16) & 0xffu, at);
     t.next[i][1] = mq_entry(v >> 24, at);
   }
@@ -1170,15 +1163,7 @@ void context_labels_from_logic(uint8_t* zc, uint8_t* sc, uint8_t* spb) {
   }
 }
 
-bool upload_t1_tables(const uint8_t* zc, const uint8_t* sc, const uint8_t* spb,
-                      const uint32_t* mq) {
-  Tables t;
-  memcpy(t.zc, zc, sizeof t.zc);
-  memcpy(t.sc, sc, sizeof t.sc);
-  memcpy(t.spb, spb, sizeof t.spb);
-  memcpy(t.mq, mq, sizeof t.mq);
-  return cudaMemcpyToSymbol(c_tables, &t, sizeof t) == cudaSuccess;
-}
+bool upload_t1_tables(const uint32_t* mq) { return cudaMemcpyToSymbol(c_mq, mq, sizeof c_mq) == cudaSuccess; }
 
 void launch_t1_analyze(const T1Args& a, cudaStream_t st) {
   if (a.nblocks == 0) return;
@@ -1208,15 +1193,11 @@ void launch_t1_model(const T1Args& a, int num_sms, T1Part part, cudaStream_t st)
   t1_model_kernel<<<need < cap ? need : cap, kModelWarps * 32, 0, st>>>(a, part);
 }
 
-int mq_blocks_per_warp(const T1Args& a, int num_sms, int bpw) {
-  return bpw >= 1 && bpw <= 32 ? bpw : mq_blocks_auto(a.nblocks, (uint32_t)num_sms * 4u);
-}
-
 void launch_t1_mq(const T1Args& a, int num_sms, int bpw, T1Part part, cudaStream_t st) {
   if (a.nblocks == 0) return;
   const uint32_t sms = (uint32_t)num_sms;
   if (bpw < 1 || bpw > 32) bpw = 0;
-  const uint32_t most = (uint32_t)mq_blocks_per_warp(a, num_sms, bpw);
+  const uint32_t most = (uint32_t)(bpw ? bpw : mq_blocks_auto(a.nblocks, sms * 4u));
   if (part == kT1Again) {  // four CTAs fit an SM; the first ones take a short list
     t1_mq_kernel<1><<<sms * 4, kMqWarps * 32, 0, st>>>(a, part, bpw, sms * 4u);
     return;
