@@ -660,19 +660,17 @@ def main():
     st_mean = {k: float(np.mean([s[k] for s in dev_st])) for k in keys}
     peaks = _peaks()
     hbm = float(peaks.get("hbm_gbs", 6800.0))
-    # Algorithmic bytes per launch (one page per step), over the launch's
-    # CUDA-event time on the engine's stream:
+    # Algorithmic bytes per page (one page per step), over the stage's
+    # CUDA-event time:
     #  DWT + colour + quantisation: 5 B per component-sample (1 B pixel read,
     #    4 B int32 coefficient written), all levels together;
-    #  Tier-1 modelling: 4 B per coefficient per modelled bit-plane read
-    #    (counter 6) + 1 B per MQ symbol written (counter 7);
-    #  MQ coding: 1 B per symbol read + the payload bytes written (counter 3).
+    #  MQ coding: 1 B per symbol coded (counter 7) + the payload bytes written
+    #    (counter 3), both parts of a split wave, from the first one's start
+    #    (part of it beside the modelling of the second).
     dwt_bytes = 5.0 * W * H * NCOMP
-    model_bytes = 4.0 * counters[6] + counters[7]
     mq_bytes = float(counters[7] + counters[3])
     kernels = {
         "dwt": ("dwt_batch_kernel (all levels)", dwt_bytes, st_mean["dwt"]),
-        "t1_model": ("t1_model_kernel", model_bytes, st_mean["t1_model"]),
         "t1_mq": ("t1_mq_kernel", mq_bytes, st_mean["t1_mq"]),
     }
     def gbs(k):
@@ -714,9 +712,6 @@ def main():
             "roofline_dwt": {"bound": "hbm", "achieved": dwt_gbs, "peak": hbm, "unit": "GB/s",
                              "frac": dwt_gbs / hbm if dwt_gbs else None,
                              "algorithmic_bytes_per_launch_set": dwt_bytes},
-            "roofline_model": {"bound": "hbm", "achieved": gbs("t1_model"), "peak": hbm, "unit": "GB/s",
-                               "frac": gbs("t1_model") / hbm if gbs("t1_model") else None,
-                               "algorithmic_bytes_per_launch": model_bytes},
             "gpu_launches": int(counters[5]) * args.steps,
             "clocks": clocks.summary(),
             "output_bytes": int(np.mean(dev_sizes))}
@@ -747,7 +742,6 @@ def main():
         # stdout carries each leg's headline figures last, so they stay in
         # view at the end of the output.
         print("bench detail: " + json.dumps(dict(line, **detail)), file=sys.stderr, flush=True)
-        line.pop("roofline_model", None)
         line.pop("stages_ms", None)
         line.update(_compact_legs(detail))
         print(json.dumps(line), flush=True)

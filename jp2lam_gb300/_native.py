@@ -109,8 +109,10 @@ class _Results:
         self._lib.jp2g_set_thread_result_alloc(self._alloc, self._user)
         return self
 
-    def __exit__(self, *_):
+    def __exit__(self, exc, *_):
         self._lib.jp2g_set_thread_result_alloc(None, None)
+        if exc is not None:
+            self.clear()
 
     def take(self, i: int) -> bytes:
         """The codestream of index i, which leaves the object."""
@@ -120,10 +122,13 @@ class _Results:
         _decref(p)
         return data
 
-    def __del__(self):
-        for p in self._objects:
+    def clear(self):
+        for i, p in enumerate(self._objects):
             if p:
+                self._objects[i] = None
                 _decref(p)
+
+    __del__ = clear
 
 _lib = None
 _lock = threading.Lock()
@@ -221,7 +226,7 @@ class Engine:
             _raise(rc, self.lib.jp2g_last_error(None).decode())
         self.handle = h
         self._lock = threading.Lock()
-        self._result = _Results(self.lib, 1)  # of the single-page calls, under _lock
+        self._results = _Results(self.lib, 64)  # of the calls of up to 64 pages, under _lock
         self._inflight = {}  # ticket -> pixel buffer kept alive until polled
         self._inflight_lock = threading.Lock()
 
@@ -248,11 +253,11 @@ class Engine:
             raise InvalidInput("pixel buffer length does not match the image dimensions")
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock, self._result as result:
+        with self._lock, self._results as results:
             rc = self.lib.jp2g_encode(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                       int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n))
             self._check(rc)
-            return result.take(0)
+            return results.take(0)
 
     def encode_with_psnr(self, px, w: int, h: int, ncomp: int, quality: int, fmt: int,
                          interleaved: bool = True):
@@ -265,12 +270,12 @@ class Engine:
         out = _u8p()
         n = ctypes.c_size_t()
         psnr, ssim = ctypes.c_double(), ctypes.c_double()
-        with self._lock, self._result as result:
+        with self._lock, self._results as results:
             rc = self.lib.jp2g_encode_with_psnr(self.handle, buf.ctypes.data_as(ctypes.c_void_p), w, h, ncomp,
                                                 int(interleaved), quality, fmt, ctypes.byref(out), ctypes.byref(n),
                                                 ctypes.byref(psnr), ctypes.byref(ssim))
             self._check(rc)
-            return result.take(0), psnr.value, ssim.value
+            return results.take(0), psnr.value, ssim.value
 
     @staticmethod
     def _decode_flags(rct_chroma_extra_bitplane, accept_empty_segments):
@@ -333,11 +338,11 @@ class Engine:
     def encode_device(self, dev_ptr: int, w: int, h: int, ncomp: int, quality: int, fmt: int) -> bytes:
         out = _u8p()
         n = ctypes.c_size_t()
-        with self._lock, self._result as result:
+        with self._lock, self._results as results:
             rc = self.lib.jp2g_encode_device(self.handle, ctypes.c_void_p(dev_ptr), w, h, ncomp, quality,
                                              fmt, ctypes.byref(out), ctypes.byref(n))
             self._check(rc)
-            return result.take(0)
+            return results.take(0)
 
     @staticmethod
     def _request(page, keep):
@@ -369,15 +374,13 @@ class Engine:
         outs = (_u8p * max(n, 1))()
         lens = (ctypes.c_size_t * max(n, 1))()
         status = (ctypes.c_int * max(n, 1))()
-        with self._lock, _Results(self.lib, n) as files:
+        with self._lock, (self._results if n <= 64 else _Results(self.lib, n)) as results:
             rc = self.lib.jp2g_encode_batch(self.handle, reqs, n, outs, lens, status)
             msg = self.lib.jp2g_last_error(self.handle).decode() if rc != 0 else ""
-        result = []
-        for i in range(n):
-            if status[i] == 0:
-                result.append(files.take(i))
-            else:
-                result.append(_BY_CODE.get(status[i], Jp2LamError)(msg or f"page {i} failed"))
+            result = [results.take(i) if status[i] == 0 else
+                      _BY_CODE.get(status[i], Jp2LamError)(msg or f"page {i} failed") for i in range(n)]
+            if rc != 0:
+                results.clear()
         return result
 
     def submit(self, page) -> int:

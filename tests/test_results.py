@@ -46,8 +46,12 @@ def test_result_objects_are_released_once():
     taken = results.take(0)
     assert taken is second and sys.getrefcount(second) == refs  # the slot's is now `taken`'s
     third = new(3000)
+    with pytest.raises(KeyError), results:
+        raise KeyError  # a call that fails leaves nothing behind
+    assert sys.getrefcount(third) == refs - 1 and results._objects[0] is None
+    fourth = new(4000)
     del results
-    assert sys.getrefcount(second) == refs and sys.getrefcount(third) == refs - 1
+    assert sys.getrefcount(second) == refs and sys.getrefcount(fourth) == refs - 1
 
 
 @pytest.mark.gpu
