@@ -1503,10 +1503,13 @@ size_t half_plane_bytes(const DecodePage& p) {
   return p.L.levels > 0 ? (size_t)((p.L.width + 1) / 2) * ((p.L.height + 1) / 2) * 4 : 0;
 }
 
-uint64_t decode_device_bytes(const DecodePage& p, size_t nbytes) {
-  // bytes, planes, tmp planes or masks, samples, code-blocks, jobs
+uint64_t decode_device_bytes(const DecodePage& p, size_t nbytes, bool budget) {
+  // bytes, planes, tmp planes or masks (of a block at least, see decode_round), samples, code-blocks, jobs
   uint64_t masks = 0;
-  for (const DecBlock& b : p.L.blocks) masks += 8ull * dec_mask_words(b.w, b.npasses);
+  for (const DecBlock& b : p.L.blocks) {
+    const uint64_t m = 8ull * dec_mask_words(b.w, b.npasses);
+    masks = budget ? std::max(masks, m) : masks + m;
+  }
   return nbytes + p.npx * p.L.ncomp * 4 + std::max<uint64_t>(p.npx, half_plane_bytes(p)) * p.L.ncomp +
          std::max<uint64_t>(p.npx * p.L.ncomp * 4, masks) + p.L.blocks.size() * sizeof(DecBlock) +
          (uint64_t)(p.L.levels * p.L.ncomp + 1) * sizeof(IdwtJob) + sizeof(PixJob) + 1024;
@@ -1532,7 +1535,14 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   // device job tables: blocks, then per-level inverse-DWT jobs, then pixel jobs
   std::vector<DecBlock> blk;
   blk.reserve(nblk);
-  uint64_t mask_words = 0, coded = 0;
+  // The blocks' masks lie where the inverse DWT's scratch planes come later. Those
+  // of blocks a few rows high take more than their samples do (8 bytes a column
+  // and bit-plane); under a memory budget Tier-1 then runs in parts whose masks
+  // fit.
+  const size_t planes_bytes = ((size_t)nplane * 4 + 15) & ~size_t(15);
+  const uint64_t part_words = c->budget ? planes_bytes / 8 : ~0ull;
+  std::vector<size_t> parts{0};  // first blocks
+  uint64_t mask_words = 0, at = 0, coded = 0;
   uint32_t longest = 0;
   for (size_t i : ids)
     for (DecBlock b : pg[i].L.blocks) {
@@ -1542,12 +1552,17 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
       }
       b.plane_off += pg[i].plane_base;
       b.data_off += (uint32_t)pg[i].data_base;
-      b.mask_off = mask_words;
-      mask_words += dec_mask_words(b.w, b.npasses);
+      const uint32_t words = dec_mask_words(b.w, b.npasses);
+      if (at > 0 && at + words > part_words) {
+        parts.push_back(blk.size());
+        at = 0;
+      }
+      b.mask_off = at;
+      at += words;
+      mask_words = std::max(mask_words, at);
       blk.push_back(b);
     }
-  // the blocks' masks lie where the inverse DWT's scratch planes come later
-  const size_t planes_bytes = ((size_t)nplane * 4 + 15) & ~size_t(15);
+  parts.push_back(blk.size());
   const size_t tmp_bytes = std::max<size_t>(planes_bytes, mask_words * 8);
   // and the blocks' order, and then every other level's samples, where the pixels do
   size_t half_bytes = 0;
@@ -1622,8 +1637,10 @@ int decode_round(jp2g_ctx* c, std::vector<DecodePage>& pg, const std::vector<siz
   // 7.95 and 8.27, 6 (7 x) 10.0 and 9.88, 8 (10 x) 11.4 and 9.94; 1700x2200
   // lossless, 4 (10 x) 10.6 and 8.56; 12 sRGB q75 (13 x) 20.4 and 17.2.
   const bool many = coded > 6ull * (uint64_t)c->num_sms * longest;
-  launch_t1_decode(dblk, (uint32_t)blk.size(), dptr<uint8_t>(c->t2out), reinterpret_cast<unsigned long long*>(tmp),
-                   planes, reinterpret_cast<uint32_t*>(dpx), many, c->stream);
+  for (size_t k = 0; k + 1 < parts.size(); ++k)
+    launch_t1_decode(dblk + parts[k], (uint32_t)(parts[k + 1] - parts[k]), dptr<uint8_t>(c->t2out),
+                     reinterpret_cast<unsigned long long*>(tmp), planes, reinterpret_cast<uint32_t*>(dpx), many,
+                     c->stream);
   for (int l = 1; l <= maxl; ++l) launch_idwt_level(djobs + first[l], first[l + 1] - first[l], tiles[l], c->stream);
   launch_dec_pixels(dpix, (uint32_t)pix.size(), pix_blocks, c->stream);
   if (!cuda_ok(c, cudaGetLastError(), "decode kernels")) return JP2G_DECODE_FAILED;
@@ -1692,7 +1709,7 @@ int decode_rounds(jp2g_ctx* c, std::vector<DecodePage>& pg, std::vector<size_t> 
     std::vector<size_t> round;
     uint64_t used = 0;
     while (k < ids.size()) {
-      const uint64_t b = decode_device_bytes(pg[ids[k]], lens[ids[k]]);
+      const uint64_t b = decode_device_bytes(pg[ids[k]], lens[ids[k]], c->budget != 0);
       if (!round.empty() && used + b > cap) break;
       used += b;
       round.push_back(ids[k++]);

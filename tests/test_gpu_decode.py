@@ -257,3 +257,20 @@ def test_batch_of_many_chains(eng, orc, q):
         want = orc.decode(f, accept_empty_segments=True)[3]
         for g in got[k::len(files)]:
             assert np.array_equal(np.asarray(g[0]), want), k
+
+
+@pytest.mark.parametrize("w,h,budget", [(20000, 1, 400_000), (1, 3000, 60_000), (4000, 3, 200_000), (3000, 12, 600_000)])
+@pytest.mark.parametrize("q", [100, 60])
+def test_strips_decode_within_the_memory_of_their_samples(orc, w, h, budget, q):
+    # blocks of a few rows, whose bit-planes' masks are larger than their samples
+    px = np.random.default_rng(w + h).integers(0, 256, w * h, dtype=np.uint8)
+    data = orc.encode(px, w, h, 1, q, 0)
+    want = orc.decode(data, accept_empty_segments=True)[3]
+    e = jl.Engine(0, budget)
+    try:
+        got, _, _, _ = e.decode(data, accept_empty_segments=True)
+        assert np.array_equal(np.asarray(got), want)
+        for g in e.decode_batch([data] * 5, accept_empty_segments=True):
+            assert np.array_equal(np.asarray(g[0]), want)
+    finally:
+        e.close()
