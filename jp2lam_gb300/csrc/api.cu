@@ -1477,6 +1477,11 @@ int jp2g_encode_with_psnr(jp2g_ctx* c, const uint8_t* px, uint32_t w, uint32_t h
   j.format = format;
   int rc = encode_one(c, &j, nullptr);
   if (rc == JP2G_OK) rc = page_metrics(c, j, psnr_db, ssim);
+  if (rc != JP2G_OK && c->budget_hit) {  // pools of earlier waves crowd the budget: once more from empty ones
+    release_pools(c);
+    rc = encode_one(c, &j, nullptr);
+    if (rc == JP2G_OK) rc = page_metrics(c, j, psnr_db, ssim);
+  }
   return finish_output(c, rc, j, out, out_len);
 }
 
@@ -1716,6 +1721,11 @@ int decode_rounds(jp2g_ctx* c, std::vector<DecodePage>& pg, std::vector<size_t> 
     }
     c->budget_hit = false;
     int rc = decode_round(c, pg, round, bytes, lens, outs, out_lens);
+    if (rc != JP2G_OK && c->budget_hit) {  // pools of earlier calls crowd the budget
+      release_pools(c);
+      c->budget_hit = false;
+      rc = decode_round(c, pg, round, bytes, lens, outs, out_lens);
+    }
     if (rc != JP2G_OK && c->budget_hit && round.size() > 1) {
       release_pools(c);
       const size_t half = round.size() / 2;
